@@ -91,9 +91,9 @@ def build_torch(verbose: bool = False, force: bool = False) -> str:
 def build_oracle_ref(verbose: bool = False, ref: str | None = None) -> str | None:
     """Compile the reference's software FP8 cast and its fused CUDA kernels into oracle/_ref, from the
     reference checkout named by `ref` or the environment variable GPUK_REFERENCE_DIR (skipped where none is given
-    or present: the built files travel with the tree)."""
+    or its sources are not there: the built files travel with the tree)."""
     ref = ref or os.environ.get("GPUK_REFERENCE_DIR")
-    if not ref or not os.path.isdir(ref):
+    if not ref or not os.path.isfile(os.path.join(ref, "src", "common", "float8.h")):
         return None
     for sub in ("ref_fp8", "ref_kernels"):
         mk = os.path.join(ROOT, "oracle", sub)
