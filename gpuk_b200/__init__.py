@@ -30,6 +30,19 @@ from . import cabi  # noqa: E402  (loads libgpuk_core.so first; libgpuk_b200.so 
 torch.ops.load_library(filename)
 _ops = torch.ops.gpuk
 
+
+def _load_native():
+    """The CPython functions that live in the same library (csrc/native.cpp)."""
+    import importlib.machinery
+    import importlib.util
+    loader = importlib.machinery.ExtensionFileLoader("gpuk_b200._native", filename)
+    module = importlib.util.module_from_spec(importlib.util.spec_from_loader("gpuk_b200._native", loader))
+    loader.exec_module(module)
+    return module
+
+
+_native = _load_native()
+
 init_ar_fusion = _ops.init_ar_fusion
 destroy_ar_fusion = _ops.destroy_ar_fusion
 get_ar_fusion_barrier_handle = _ops.get_ar_fusion_barrier_handle

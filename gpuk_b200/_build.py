@@ -26,7 +26,7 @@ NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
     "-Xcompiler", "-fPIC",
 ]
-CORE_SOURCES = ["core.cu", "launch_bf16.cu", "launch_f16.cu", "launch_f32.cu", "noalloc.cu", "fp8_linear.cu"]
+CORE_SOURCES = ["core.cu", "launch_bf16.cu", "launch_f16.cu", "launch_f32.cu", "noalloc.cu", "fp8_linear.cu", "decoder_ops.cu"]
 HEADERS = ["common.cuh", "epilogue.cuh", "kernels.cuh", "launch.cuh", "launch_impl.cuh",
            os.path.join(ROOT, "include", "gpuk_b200.h")]
 
@@ -70,21 +70,25 @@ def build_torch(verbose: bool = False, force: bool = False) -> str:
     import torch
     from torch.utils import cpp_extension as ce
 
-    src = os.path.join(CSRC, "torch_ops.cpp")
-    deps = [src, os.path.join(ROOT, "include", "gpuk_b200.h"), CORE_LIB]
+    srcs = [os.path.join(CSRC, "torch_ops.cpp"), os.path.join(CSRC, "native.cpp")]
+    deps = srcs + [os.path.join(ROOT, "include", "gpuk_b200.h"), CORE_LIB]
     if not force and _newer(TORCH_LIB, deps):
         return TORCH_LIB
-    inc = []
+    import sysconfig
+    inc = ["-I", sysconfig.get_path("include")]
     for p in ce.include_paths(device_type="cuda") if "device_type" in ce.include_paths.__code__.co_varnames else ce.include_paths(cuda=True):
         inc += ["-I", p]
     torch_lib = os.path.join(os.path.dirname(torch.__file__), "lib")
     abi = int(torch._C._GLIBCXX_USE_CXX11_ABI)
-    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={abi}",
-           "-DTORCH_EXTENSION_NAME=gpuk_b200", "-I", os.path.join(ROOT, "include")] + inc + [
-           src, "-o", TORCH_LIB, "-L", HERE, "-lgpuk_core", "-Wl,-rpath,$ORIGIN",
-           "-L", torch_lib, "-ltorch", "-ltorch_cpu", "-lc10", "-ltorch_cuda", "-lc10_cuda",
-           f"-Wl,-rpath,{torch_lib}"]
-    _run(cmd, verbose)
+    os.makedirs(OBJ, exist_ok=True)
+    objs = [os.path.join(OBJ, os.path.basename(s)[:-4] + ".o") for s in srcs]
+    compile_one = ["g++", "-O2", "-std=c++17", "-fPIC", f"-D_GLIBCXX_USE_CXX11_ABI={abi}",
+                   "-DTORCH_EXTENSION_NAME=gpuk_b200", "-I", os.path.join(ROOT, "include")] + inc + ["-c"]
+    with ThreadPoolExecutor(max_workers=len(srcs)) as ex:
+        list(ex.map(lambda so: _run(compile_one + [so[0], "-o", so[1]], verbose), zip(srcs, objs)))
+    _run(["g++", "-shared"] + objs + ["-o", TORCH_LIB, "-L", HERE, "-lgpuk_core", "-Wl,-rpath,$ORIGIN",
+          "-L", torch_lib, "-ltorch", "-ltorch_cpu", "-lc10", "-ltorch_cuda", "-lc10_cuda", "-ltorch_python",
+          f"-Wl,-rpath,{torch_lib}"], verbose)
     return TORCH_LIB
 
 

@@ -1,0 +1,140 @@
+// The elementwise steps of a decoder layer between its projections, one launch each:
+//
+//   rope_append_kernel   rotary embedding of q and k and the write of k and v into the KV cache, straight from the
+//                        q|k|v projection's output.  As PyTorch operators: slicing, four multiplications, two additions
+//                        and a concatenation each for q and k, two casts, two indexed stores.
+//   silu_mul_kernel      silu(w1 x) * (w3 x) from the joint w1|w3 output.
+//
+// Both are bound by their bytes for long prompts and by launch latency for a decode step, so what counts is one pass and
+// one launch.  Rounding points are those of the operator chains: fp32 products and sums each rounded (no fused
+// multiply-add), one rounding to bf16; silu rounded to bf16 before the multiplication.
+#include <cuda_bf16.h>
+#include <cuda_runtime.h>
+
+#include <cstdint>
+
+#include "../../include/gpuk_b200.h"
+#include "launch.cuh"
+
+namespace gpuk {
+namespace {
+
+using bf16 = __nv_bfloat16;
+constexpr int kRopeVec = 16;      // elements of a head one thread takes: eight (even, odd) pairs, two 16-byte loads
+constexpr int kThreads = 256;
+
+struct RopeParams {
+    const bf16 *qkv;         // [batch * t, (heads + 2 * kv_heads) * head_dim]
+    const float *cos, *sin;  // [table_rows, head_dim / 2]
+    const int64_t *pos;      // [t]
+    bf16 *q_out;             // [batch * t, heads * head_dim]
+    bf16 *k_cache, *v_cache; // [batch, kv_heads, max_seq, head_dim]
+    int64_t total;           // threads with work
+    int t, heads, kv_heads, head_dim, table_rows, max_seq;
+};
+
+// Thread -> (row, head, part of the head), the part fastest: a warp reads one contiguous run of the row.
+__global__ void __launch_bounds__(kThreads) rope_append_kernel(const __grid_constant__ RopeParams p) {
+    grid_dependency_sync();
+    const int64_t idx = static_cast<int64_t>(blockIdx.x) * kThreads + threadIdx.x;
+    if (idx >= p.total) return;
+    const int parts = p.head_dim / kRopeVec, all = p.heads + 2 * p.kv_heads;
+    const int part = static_cast<int>(idx % parts);
+    const int64_t rest = idx / parts;
+    const int head = static_cast<int>(rest % all);
+    const int64_t row = rest / all;
+    const int b = static_cast<int>(row / p.t);
+    const uint4 *src = reinterpret_cast<const uint4 *>(p.qkv + (row * all + head) * p.head_dim + part * kRopeVec);
+    const uint4 in0 = ld_stream(src), in1 = ld_stream(src + 1);
+    const int64_t raw = p.pos[row % p.t];
+    // a negative position counts from the end of what it indexes, as in an indexed tensor
+    const int64_t at = raw < 0 ? raw + p.max_seq : raw, angle = raw < 0 ? raw + p.table_rows : raw;
+    const bool in_cache = at >= 0 && at < p.max_seq;      // the caller checks; nothing is written past the cache in any case
+    const int kv = head - p.heads;
+    if (kv >= p.kv_heads) {      // v: as it is
+        if (!in_cache) return;
+        uint4 *dst = reinterpret_cast<uint4 *>(p.v_cache + ((static_cast<int64_t>(b) * p.kv_heads + kv - p.kv_heads) * p.max_seq + at) * p.head_dim + part * kRopeVec);
+        dst[0] = in0;
+        dst[1] = in1;
+        return;
+    }
+    if (kv >= 0 && !in_cache) return;
+    if (angle < 0 || angle >= p.table_rows) return;
+    const int half = p.head_dim / 2, first = part * (kRopeVec / 2);
+    float c[8], s[8];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const float4 cv = __ldg(reinterpret_cast<const float4 *>(p.cos + angle * half + first) + i);
+        const float4 sv = __ldg(reinterpret_cast<const float4 *>(p.sin + angle * half + first) + i);
+        c[4 * i] = cv.x, c[4 * i + 1] = cv.y, c[4 * i + 2] = cv.z, c[4 * i + 3] = cv.w;
+        s[4 * i] = sv.x, s[4 * i + 1] = sv.y, s[4 * i + 2] = sv.z, s[4 * i + 3] = sv.w;
+    }
+    const uint32_t w[8] = {in0.x, in0.y, in0.z, in0.w, in1.x, in1.y, in1.z, in1.w};
+    float lo[8], hi[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const float x1 = __uint_as_float(w[i] << 16), x2 = __uint_as_float(w[i] & 0xffff0000u);
+        lo[i] = __fsub_rn(__fmul_rn(x1, c[i]), __fmul_rn(x2, s[i]));
+        hi[i] = __fadd_rn(__fmul_rn(x2, c[i]), __fmul_rn(x1, s[i]));
+    }
+    bf16 *dst = kv < 0 ? p.q_out + (row * p.heads + head) * p.head_dim
+                       : p.k_cache + ((static_cast<int64_t>(b) * p.kv_heads + kv) * p.max_seq + at) * p.head_dim;
+    *reinterpret_cast<uint4 *>(dst + first) = Elem<bf16>::pack(lo);
+    *reinterpret_cast<uint4 *>(dst + half + first) = Elem<bf16>::pack(hi);
+}
+
+// in [rows, 2 * f]: w1's channels, then w3's.  One thread per 16-byte vector of the output.
+__global__ void __launch_bounds__(kThreads) silu_mul_kernel(const uint4 *in, uint4 *out, int64_t vecs, int row_vecs) {
+    grid_dependency_sync();
+    const int64_t idx = static_cast<int64_t>(blockIdx.x) * kThreads + threadIdx.x;
+    if (idx >= vecs) return;
+    const int64_t row = idx / row_vecs, v = idx - row * row_vecs;
+    const uint4 *src = in + row * 2 * row_vecs + v;
+    const uint4 a = ld_stream(src), b = ld_stream(src + row_vecs);
+    float f[8];
+    Elem<bf16>::unpack(a, f);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) f[i] = f[i] / (1.0f + expf(-f[i]));
+    out[idx] = Elem<bf16>::mul(Elem<bf16>::pack(f), b);
+}
+
+bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
+
+}  // namespace
+}  // namespace gpuk
+
+using namespace gpuk;
+
+extern "C" int gpuk_rope_append(const void *qkv, const float *cos, const float *sin, const int64_t *pos, void *q_out, void *k_cache, void *v_cache,
+                                int batch, int t, int heads, int kv_heads, int head_dim, int table_rows, int max_seq, void *stream) {
+    if (batch < 0 || t < 0 || heads <= 0 || kv_heads <= 0 || table_rows <= 0 || max_seq <= 0)
+        return set_last_error(GPUK_ERR_INVALID_ARGUMENT, "rope_append: bad sizes");
+    if (head_dim <= 0 || head_dim % kRopeVec) return set_last_error(GPUK_ERR_UNSUPPORTED, "rope_append: head_dim %d is not a multiple of %d", head_dim, kRopeVec);
+    if (batch == 0 || t == 0) return GPUK_OK;
+    if (!qkv || !cos || !sin || !pos || !q_out || !k_cache || !v_cache) return set_last_error(GPUK_ERR_INVALID_ARGUMENT, "rope_append: null pointer");
+    if (!aligned16(qkv) || !aligned16(cos) || !aligned16(sin) || !aligned16(q_out) || !aligned16(k_cache) || !aligned16(v_cache))
+        return set_last_error(GPUK_ERR_INVALID_ARGUMENT, "rope_append: pointers must be 16-byte aligned");
+    RopeParams p = {static_cast<const bf16 *>(qkv), cos, sin, pos, static_cast<bf16 *>(q_out), static_cast<bf16 *>(k_cache), static_cast<bf16 *>(v_cache),
+                    static_cast<int64_t>(batch) * t * (heads + 2 * kv_heads) * (head_dim / kRopeVec), t, heads, kv_heads, head_dim, table_rows, max_seq};
+    const int64_t grid = (p.total + kThreads - 1) / kThreads;
+    if (grid > 0x7fffffffll) return set_last_error(GPUK_ERR_UNSUPPORTED, "rope_append: too many rows");
+    void *args[] = {&p};
+    cudaError_t e = launch_kernel(reinterpret_cast<const void *>(&rope_append_kernel), static_cast<int>(grid), kThreads, 1, false, args, static_cast<cudaStream_t>(stream));
+    if (e != cudaSuccess) return set_last_error(GPUK_ERR_CUDA, "rope_append: launch failed: %s", cudaGetErrorString(e));
+    return GPUK_OK;
+}
+
+extern "C" int gpuk_silu_mul(const void *in, void *out, int64_t rows, int f, void *stream) {
+    if (rows < 0 || f <= 0) return set_last_error(GPUK_ERR_INVALID_ARGUMENT, "silu_mul: bad sizes");
+    if (f % 8) return set_last_error(GPUK_ERR_UNSUPPORTED, "silu_mul: %d channels are not a multiple of 8", f);
+    if (rows == 0) return GPUK_OK;
+    if (!in || !out || !aligned16(in) || !aligned16(out)) return set_last_error(GPUK_ERR_INVALID_ARGUMENT, "silu_mul: pointers must be 16-byte aligned and not null");
+    int row_vecs = f / 8;
+    int64_t vecs = rows * row_vecs;
+    const int64_t grid = (vecs + kThreads - 1) / kThreads;
+    if (grid > 0x7fffffffll) return set_last_error(GPUK_ERR_UNSUPPORTED, "silu_mul: too many rows");
+    void *args[] = {&in, &out, &vecs, &row_vecs};
+    cudaError_t e = launch_kernel(reinterpret_cast<const void *>(&silu_mul_kernel), static_cast<int>(grid), kThreads, 1, false, args, static_cast<cudaStream_t>(stream));
+    if (e != cudaSuccess) return set_last_error(GPUK_ERR_CUDA, "silu_mul: launch failed: %s", cudaGetErrorString(e));
+    return GPUK_OK;
+}

@@ -151,6 +151,8 @@ class TPDecoder:
         freqs = torch.outer(torch.arange(a.max_seq_len * 2, dtype=torch.float32), inv)
         self.cos, self.sin = freqs.cos().to(self.device), freqs.sin().to(self.device)
         self._zeros = {}
+        # the elementwise steps between the projections as this library's kernels (csrc/decoder_ops.cu)
+        self.own_elementwise = fused and self.device.type == "cuda" and a.dtype == torch.bfloat16 and hd % 16 == 0 and a.ffn_dim // w % 8 == 0
 
     # ------------------------------------------------------------------------------------
     def fill_kv_cache(self, upto: int, seed: int = 7) -> None:
@@ -215,25 +217,39 @@ class TPDecoder:
         b, t = tokens.shape
         hd = a.head_dim
         h = F.embedding(tokens, self.tok_embeddings).view(b * t, a.dim)
-        cos, sin = self.cos[input_pos], self.sin[input_pos]
         last = int(input_pos[-1]) + 1 if cache_len is None else cache_len
+        own = self.own_elementwise
+        if own:
+            from gpuk_b200 import _native
+            if last > a.max_seq_len:
+                raise RuntimeError(f"position {last - 1} is beyond the KV cache ({a.max_seq_len} positions)")
+            pos = input_pos.to(device=self.device, dtype=torch.int64).contiguous()
+        else:
+            cos, sin = self.cos[input_pos], self.sin[input_pos]
         mask = None
         if t > 1:
             mask = (torch.arange(last, device=self.device)[None, :] <= input_pos[:, None])[None, None]
         normed, scale = self._norm_only(h, self.layers[0]["attention_norm"])
         for li, layer in enumerate(self.layers):
-            qkv = layer["wqkv"](normed, scale).view(b, t, self.h_local + 2 * self.kv_local, hd)
-            q, k, v = qkv.split([self.h_local, self.kv_local, self.kv_local], dim=2)
-            q, k = self._rope(q, cos, sin), self._rope(k, cos, sin)
-            layer["k_cache"][:b, :, input_pos] = k.transpose(1, 2)
-            layer["v_cache"][:b, :, input_pos] = v.transpose(1, 2)
+            qkv = layer["wqkv"](normed, scale)
+            if own:
+                q = _native.rope_append(qkv, self.cos, self.sin, pos, layer["k_cache"], layer["v_cache"], self.h_local).view(b, t, self.h_local, hd)
+            else:
+                q, k, v = qkv.view(b, t, self.h_local + 2 * self.kv_local, hd).split([self.h_local, self.kv_local, self.kv_local], dim=2)
+                q, k = self._rope(q, cos, sin), self._rope(k, cos, sin)
+                layer["k_cache"][:b, :, input_pos] = k.transpose(1, 2)
+                layer["v_cache"][:b, :, input_pos] = v.transpose(1, 2)
             att = F.scaled_dot_product_attention(q.transpose(1, 2), layer["k_cache"][:b, :, :last], layer["v_cache"][:b, :, :last],
                                                  attn_mask=mask, enable_gqa=True)
             partial = layer["wo"](att.transpose(1, 2).reshape(b * t, self.h_local * hd))
             h, normed, scale = self._reduce_add_norm(partial, h, layer["ffn_norm"])
             g13 = layer["w13"](normed, scale)
-            f1, f3 = g13.split(a.ffn_dim // self.world, dim=-1)
-            partial = layer["w2"](F.silu(f1) * f3)
+            if own:
+                act = _native.silu_mul(g13)
+            else:
+                f1, f3 = g13.split(a.ffn_dim // self.world, dim=-1)
+                act = F.silu(f1) * f3
+            partial = layer["w2"](act)
             nxt = self.layers[li + 1]["attention_norm"] if li + 1 < a.n_layers else self.norm
             h, normed, scale = self._reduce_add_norm(partial, h, nxt)
         return self.output(normed, scale).view(b, t, -1)

@@ -357,6 +357,22 @@ int gpuk_fp8_pack_weight(const void *w_fp8, void *packed, int n, int k, void *st
 int gpuk_fp8_linear_status(void);
 
 /*
+ * The elementwise steps of a decoder layer in bf16, one launch each (the reference runs them as chains of PyTorch
+ * operators, model/transformer_model.py:504-519).
+ *
+ * gpuk_rope_append: qkv [batch * t, (heads + 2 * kv_heads) * head_dim] as the q|k|v projection wrote it; pos [t] int64
+ * positions on the device; cos, sin [table_rows, head_dim / 2] fp32.  Interleaved pairs in, halves out.  Writes the rotated
+ * queries to q_out [batch * t, heads * head_dim] and the rotated keys and the values to positions pos of the caches
+ * [batch, kv_heads, max_seq, head_dim].  A negative position counts from the end; one outside a table or cache is not
+ * written.  head_dim a multiple of 16, pointers 16-byte aligned.
+ *
+ * gpuk_silu_mul: out [rows, f] = silu(in[:, :f]) * in[:, f:], in [rows, 2 * f]; f a multiple of 8.
+ */
+int gpuk_rope_append(const void *qkv, const float *cos, const float *sin, const int64_t *pos, void *q_out, void *k_cache, void *v_cache,
+                     int batch, int t, int heads, int kv_heads, int head_dim, int table_rows, int max_seq, void *stream);
+int gpuk_silu_mul(const void *in, void *out, int64_t rows, int f, void *stream);
+
+/*
  * No counterpart in the reference.  Same job as gpuk_emulated_allreduce_rms (fused op only)
  * for callers that must not allocate device memory -- a health probe or test harness inside a
  * process whose own arena already owns the GPU's memory, where a library-side cudaMalloc may
