@@ -975,7 +975,7 @@ def run_fp8_linear(tokens=32, iters=200, k_split=0):
                      "torch_scaled_mm_frac_of_hbm_peak": nbytes / lib * 1e-3 / peak,
                      "max_bf16_steps_from_scaled_mm": steps_apart})
     cabi_status = gpuk.cabi.lib.gpuk_fp8_linear_status()
-    return {"case": "fp8_linear", "kernel": "fp8_linear_skinny_kernel (mma.sync e4m3, weights streamed once)", "status": cabi_status,
+    return {"case": "fp8_linear", "kernel": "stream_linear_kernel (tcgen05, weights streamed once) or fp8_linear_skinny_kernel (mma.sync)", "status": cabi_status,
             "hbm_peak_gbs": peak, "rows": rows}
 
 

@@ -2,17 +2,18 @@
 // for a handful of tokens (decode), i.e. the linear layer that follows the norm in a tensor-parallel
 // block (F.linear in model/tensor_parallel.py:66 of the reference, which has no FP8 path of its own).
 //
-// With at most 32 tokens the product is a weight-streaming problem: every weight byte is read once
-// and used for 32 multiply-adds, so the kernel is bound by HBM, not by the tensor pipe.  That decides
-// the design:
+// The product is a weight-streaming problem: every weight byte is read once and used for at most 32 multiply-adds.  Two kernels share
+// the work.  This one, on warp-level mma, takes at most 8 tokens on weights of up to 12 MiB: it has no tensor map, tensor memory or
+// ring to set up and ends a microsecond sooner.  Beyond, its conversions (below) bound it, and the tcgen05 kernel of stream_linear.cu is the
+// faster one.  Measured, here / there, 8 tokens: 1024 x 1024 2.8 / 3.5 us, 1280 x 8192 5.4 / 6.6, 5120 x 2048 5.1 / 5.3, 4096 x 8192
+// 9.4 / 9.5 (row-major 10.9 / 9.5), 7168 x 8192 14.7 / 12.4, 57344 x 8192 82 / 73; with 16 and 32 tokens, 7168 x 8192: 15.4 / 12.6 and
+// 21.7 / 13.2.
 //
 //   * weights [n, k] (k contiguous, e4m3) are the 16-row operand of the warp-level mma and the
-//     activations [tokens, k] its 8-column operand, so one weight fragment is used for all four
-//     groups of 8 tokens; every thread fetches exactly the bytes of its own fragment registers.
+//     activations [tokens, k] its 8-column operand; every thread fetches exactly the bytes of its own fragment registers.
 //     sm_100 has no native FP8 path for mma.sync (ptxas expands an e4m3 mma into conversions and
 //     f16 HMMAs per instruction, 170 instructions per 64-byte k step as first written), so the
-//     kernel converts e4m3 -> f16 itself (exact), once per weight fragment instead of once per
-//     token group, and issues mma.sync.m16n8k16.f16.f16.f32.  Products of two e4m3 values are exact
+//     kernel converts e4m3 -> f16 itself (exact) and issues mma.sync.m16n8k16.f16.f16.f32.  Products of two e4m3 values are exact
 //     in the fp32 accumulator either way.
 //   * fragment loads are 16 bytes per thread.  The instruction wants thread (g, t) of a warp to hold
 //     k = 2t, 2t+1 and 2t+8, 2t+9 of row g; a dot product does not care about the order of k as
@@ -26,8 +27,8 @@
 //     the kernel).  The KS partial tiles are summed through distributed shared memory in a fixed
 //     order (deterministic, no atomics), scaled, rounded once and stored.
 //
-// Activation traffic is (n / 128) x tokens x k bytes out of L2 against n x k bytes of weights from
-// HBM: a quarter of it at 32 tokens.
+// Weights that the ring takes first are brought into L2 before griddepcontrol.wait, while the kernel in front still runs: 6.4 -> 5.4 us
+// at 8 tokens, 1280 x 8192, launches back to back.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -36,6 +37,7 @@
 
 #include "../../include/gpuk_b200.h"
 #include "launch.cuh"
+#include "linear.cuh"
 
 namespace gpuk {
 namespace {
@@ -44,14 +46,16 @@ constexpr int kTileN = 128;        // output channels per cluster
 constexpr int kWarps = 8;          // per CTA; each owns kTileN / kWarps = 16 channels = one 16-row fragment
 constexpr int kThreads = kWarps * 32;
 constexpr int kDepth = 8;          // k steps of weights in flight per thread (cp.async groups): 7 x 32 bytes
-constexpr int kTokens = 32;        // token capacity of one pass: four groups of 8
+constexpr int kTokens = 8;         // token capacity: the columns of one mma
 constexpr int kStepBytes = 64;     // k bytes one warp-wide 16-byte load covers per row
 constexpr int kXSteps = 8;         // k steps of activations staged together (two such buffers)
 constexpr int kXRow = kXSteps * kStepBytes + 64;   // shared-memory row pitch; 64 mod 128 keeps 16-byte reads conflict-free
 constexpr int kXBuf = kTokens * kXRow;              // one activation buffer
 constexpr int kWSlot = 2 * kThreads * 16;           // one k step of the CTA's weights: two 16-byte vectors per thread
 constexpr int kPartPitch = kTileN + 4;              // floats per token row of the partial tile (128 channels + padding)
-constexpr int kSmemBytes = kDepth * kWSlot + 2 * kXBuf;   // 64 KiB + 36 KiB: two CTAs per SM
+constexpr int kSmemBytes = kDepth * kWSlot + 2 * kXBuf;   // 64 KiB + 9 KiB: three CTAs per SM
+constexpr int64_t kWarpMaxBytes = 12 << 20;      // weights up to which this kernel is the faster one (see the entry point)
+constexpr int kMaxTokens = 32;     // ... of the entry point
 static_assert(kTokens * kPartPitch * 4 <= kDepth * kWSlot, "the partial tile reuses the weight ring");
 static_assert((kDepth & (kDepth - 1)) == 0 && kXSteps == kDepth, "slot and buffer arithmetic below");
 
@@ -101,8 +105,6 @@ __device__ __forceinline__ float ld_cluster_f32(const float *local, int cta) {
     return v;
 }
 
-// QN = groups of 8 tokens in use (1 .. 4): the token loop has no run-time bounds.
-//
 // Pipeline of one thread.  Weights: step j of the CTA's k range is fetched with two 16-byte cp.async into the
 // thread's own place in slot j % kDepth of a shared-memory ring (it will read them back itself, so no barrier is
 // involved) and committed as group j; before step i is multiplied, step i + kDepth - 1 is issued and
@@ -114,15 +116,17 @@ __device__ __forceinline__ float ld_cluster_f32(const float *local, int cta) {
 // before last used, inside the same group; when the multiply front enters the chunk, every thread has waited for
 // its own copies and one block barrier makes the chunk visible to all warps.
 //
-// FR = 16-row fragments per warp (1: eight warps per CTA, 2: four).  With two fragments a warp converts an
-// activation vector once for both, and the per-step bookkeeping is shared: worth it when there are many token groups.
-template <int QN, int FR>
+// FR = 16-row fragments per warp (1: eight warps per CTA, 2: four).  With two fragments a warp converts an activation vector
+// once for both, and the per-step bookkeeping is shared: the faster form from 2048 channels (2048 x 5120: 5.1 / 4.9 us, 2048 x 2048: 3.8 / 3.5 us, one / two
+// fragments, 8 tokens), not below (1024 x 1024: 2.8 / 3.2 us, 1280 x 8192: 5.4 / 5.6 us).
+__device__ __forceinline__ void prefetch_l2(const void *p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
+template <int FR>
 __global__ void __launch_bounds__(kThreads / FR, 2) fp8_linear_skinny_kernel(const __grid_constant__ Fp8LinearParams p) {
     constexpr int T = kThreads / FR;                      // threads per CTA; FR * T 16-byte vectors per half fragment row set
     extern __shared__ __align__(128) unsigned char smem[];
     unsigned char *wring = smem;                          // [kDepth][2 * FR][T] x 16 bytes
     unsigned char *xbuf = smem + kDepth * kWSlot;         // [2][kTokens][kXRow]
-    grid_dependency_sync();
     const int ks = cluster_size(), part = cluster_cta_rank();
     if (ks != p.ks) {
         if (threadIdx.x == 0) *p.status = 1;
@@ -137,13 +141,11 @@ __global__ void __launch_bounds__(kThreads / FR, 2) fp8_linear_skinny_kernel(con
     const int s_begin = part * base + (part < extra ? part : extra);
     const int nsteps = base + (part < extra ? 1 : 0);
 
-    float acc[FR][QN][4];
+    float acc[FR][4];
 #pragma unroll
     for (int f = 0; f < FR; ++f)
 #pragma unroll
-        for (int q = 0; q < QN; ++q)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) acc[f][q][e] = 0.f;
+        for (int e = 0; e < 4; ++e) acc[f][e] = 0.f;
 
     // Row-major weights: a k step of the warp's fragment is 64 bytes of 16 rows that lie k bytes apart.  Blocked
     // weights: the same 16 x 64 bytes are one contiguous KiB (row r of the fragment at r * 64) and consecutive k steps
@@ -154,6 +156,17 @@ __global__ void __launch_bounds__(kThreads / FR, 2) fp8_linear_skinny_kernel(con
     const size_t half = p.packed ? static_cast<size_t>(8) * kStepBytes : static_cast<size_t>(8) * p.k;
     const size_t frag = static_cast<size_t>(16) * p.k;      // from one fragment to the next: 16 rows, in either layout
     const uint8_t *xk = p.x + static_cast<size_t>(s_begin) * kStepBytes;
+
+    // what the ring will take first comes into L2 while the kernel in front of this one ends: a hint, read only after the wait
+    if ((t & 1) == 0) {
+        for (int j = 0; j < min(kDepth - 1, nsteps); ++j)
+#pragma unroll
+            for (int f = 0; f < FR; ++f) {
+                prefetch_l2(w0 + f * frag + j * step_stride);
+                prefetch_l2(w0 + f * frag + half + j * step_stride);
+            }
+    }
+    grid_dependency_sync();
 
     auto issue = [&](int j) {      // group j: the weights of step j and, at a chunk start, the activations of the chunk
         if (j < nsteps) {
@@ -168,7 +181,7 @@ __global__ void __launch_bounds__(kThreads / FR, 2) fp8_linear_skinny_kernel(con
                 unsigned char *dst = xbuf + ((j / kXSteps) & 1) * kXBuf;
                 const int left = nsteps - j < kXSteps ? nsteps - j : kXSteps;     // steps of this chunk that exist
 #pragma unroll
-                for (int r = 0; r < QN * FR; ++r) {
+                for (int r = 0; r < FR; ++r) {
                     const int idx = tid + r * T;
                     const int tok = idx >> 5, c = idx & 31;      // 32 vectors of 16 bytes per token and chunk
                     const bool valid = tok < p.m && (c >> 2) < left;
@@ -195,16 +208,13 @@ __global__ void __launch_bounds__(kThreads / FR, 2) fp8_linear_skinny_kernel(con
             e4m3x16_to_f16(*reinterpret_cast<const uint4 *>(slot + (2 * f + 1) * T * 16), wb[f]);
         }
         const unsigned char *xs = xbuf + ((i / kXSteps) & 1) * kXBuf + g * kXRow + (i & (kXSteps - 1)) * kStepBytes + 16 * t;
+        uint32_t xh[8];
+        e4m3x16_to_f16(*reinterpret_cast<const uint4 *>(xs), xh);
 #pragma unroll
-        for (int q = 0; q < QN; ++q) {
-            uint32_t xh[8];
-            e4m3x16_to_f16(*reinterpret_cast<const uint4 *>(xs + q * 8 * kXRow), xh);
+        for (int v = 0; v < 4; ++v)
 #pragma unroll
-            for (int v = 0; v < 4; ++v)
-#pragma unroll
-                for (int f = 0; f < FR; ++f)
-                    mma_f16(acc[f][q], wa[f][2 * v], wb[f][2 * v], wa[f][2 * v + 1], wb[f][2 * v + 1], xh[2 * v], xh[2 * v + 1]);
-        }
+            for (int f = 0; f < FR; ++f)
+                mma_f16(acc[f], wa[f][2 * v], wb[f][2 * v], wa[f][2 * v + 1], wb[f][2 * v + 1], xh[2 * v], xh[2 * v + 1]);
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();      // every warp is done with the ring: it becomes the partial tile
@@ -212,29 +222,27 @@ __global__ void __launch_bounds__(kThreads / FR, 2) fp8_linear_skinny_kernel(con
     // this CTA's partial tile: token-major, fp32 (channels of a token are contiguous, as in the output)
     float *partial = reinterpret_cast<float *>(smem);
 #pragma unroll
-    for (int f = 0; f < FR; ++f)
-#pragma unroll
-        for (int q = 0; q < QN; ++q) {
-            const int ch = (warp * FR + f) * 16 + g, tok = q * 8 + 2 * t;
-            partial[tok * kPartPitch + ch] = acc[f][q][0];
-            partial[(tok + 1) * kPartPitch + ch] = acc[f][q][1];
-            partial[tok * kPartPitch + ch + 8] = acc[f][q][2];
-            partial[(tok + 1) * kPartPitch + ch + 8] = acc[f][q][3];
-        }
+    for (int f = 0; f < FR; ++f) {
+        const int ch = (warp * FR + f) * 16 + g, tok = 2 * t;
+        partial[tok * kPartPitch + ch] = acc[f][0];
+        partial[(tok + 1) * kPartPitch + ch] = acc[f][1];
+        partial[tok * kPartPitch + ch + 8] = acc[f][2];
+        partial[(tok + 1) * kPartPitch + ch + 8] = acc[f][3];
+    }
     cluster_barrier();
     // CTA `part` finishes channels [part * per, part * per + per) of the tile: sum over the cluster in CTA order
     const int per = kTileN / ks;
-    for (int e = tid; e < per * QN * 8; e += T) {
+    for (int e = tid; e < per * p.m; e += T) {
         const int ch = part * per + e % per, tok = e / per;
         float sum = 0.f;
         for (int c = 0; c < ks; ++c) sum += ld_cluster_f32(partial + tok * kPartPitch + ch, c);
         const int n = tile * kTileN + ch;
-        if (tok < p.m) p.out[static_cast<size_t>(tok) * p.n + n] = __float2bfloat16_rn(sum * p.x_scale[tok] * p.w_scale[n]);
+        p.out[static_cast<size_t>(tok) * p.n + n] = __float2bfloat16_rn(sum * p.x_scale[tok] * p.w_scale[n]);
     }
     cluster_barrier();     // nobody leaves while its partial tile may still be read
 }
 
-__global__ void clear_status_kernel(int *status) { *status = 0; }
+__device__ int decode_status;      // zero when the library is loaded: nothing to allocate, also under stream capture
 
 // [n, k] row-major -> blocked: block (n / 16, k / 64) holds 16 rows x 64 bytes, row r at r * 64; blocks of one
 // 16-row band follow each other along k.  One 16-byte vector per thread.
@@ -248,12 +256,35 @@ __global__ void pack_weight_kernel(const uint4 *w, uint4 *packed, int n, int k) 
     }
 }
 
-int *g_status_by_device[64] = {};   // one device word per GPU, allocated by the first call on it
+int *g_status_by_device[64] = {};   // the address of decode_status on each GPU, set by the first call on it
+int g_sms_by_device[64] = {};
 
 }  // namespace
 }  // namespace gpuk
 
 int gpuk::fp8_frags_per_warp_tuning = 0;
+
+int gpuk::decode_device(int *sms, int **status) {
+    int device = 0;
+    if (cudaGetDevice(&device) != cudaSuccess) return set_last_error(GPUK_ERR_CUDA, "no current device");
+    if (device < 0 || device >= 64) return set_last_error(GPUK_ERR_UNSUPPORTED, "device index %d", device);
+    // guarded for concurrent callers
+    static std::mutex init_mutex;
+    std::lock_guard<std::mutex> lock(init_mutex);
+    if (!g_status_by_device[device]) {
+        void *word = nullptr;
+        cudaError_t e = cudaGetSymbolAddress(&word, decode_status);
+        for (const void *fn : {reinterpret_cast<const void *>(&fp8_linear_skinny_kernel<1>), reinterpret_cast<const void *>(&fp8_linear_skinny_kernel<2>)})
+            if (e == cudaSuccess) e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
+        if (e == cudaSuccess) e = stream_linear_setup();
+        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&g_sms_by_device[device], cudaDevAttrMultiProcessorCount, device);
+        if (e != cudaSuccess) return set_last_error(GPUK_ERR_CUDA, "cannot prepare the kernels of a decode step: %s", cudaGetErrorString(e));
+        g_status_by_device[device] = static_cast<int *>(word);
+    }
+    *sms = g_sms_by_device[device];
+    *status = g_status_by_device[device];
+    return GPUK_OK;
+}
 
 using namespace gpuk;
 
@@ -262,7 +293,7 @@ extern "C" int gpuk_fp8_linear_skinny(const void *x_fp8, const float *x_scale, c
     if (!x_fp8 || !x_scale || !w_fp8 || !w_scale || !out_bf16) return set_last_error(GPUK_ERR_INVALID_ARGUMENT, "fp8_linear: null pointer");
     if (m < 0 || n <= 0 || k <= 0) return set_last_error(GPUK_ERR_INVALID_ARGUMENT, "fp8_linear: bad shape %d x %d x %d", m, n, k);
     if (m == 0) return GPUK_OK;
-    if (m > kTokens) return set_last_error(GPUK_ERR_UNSUPPORTED, "fp8_linear: %d tokens; this kernel is built for at most %d (use a library GEMM beyond)", m, kTokens);
+    if (m > kMaxTokens) return set_last_error(GPUK_ERR_UNSUPPORTED, "fp8_linear: %d tokens; this kernel is built for at most %d (use a library GEMM beyond)", m, kMaxTokens);
     if (n % kTileN || k % kStepBytes)
         return set_last_error(GPUK_ERR_UNSUPPORTED, "fp8_linear: n must be a multiple of %d and k of %d (got %d, %d)", kTileN, kStepBytes, n, k);
     if ((reinterpret_cast<uintptr_t>(x_fp8) | reinterpret_cast<uintptr_t>(w_fp8)) & 15u)
@@ -270,45 +301,25 @@ extern "C" int gpuk_fp8_linear_skinny(const void *x_fp8, const float *x_scale, c
     if (w_layout != 0 && w_layout != 1) return set_last_error(GPUK_ERR_INVALID_ARGUMENT, "fp8_linear: w_layout must be 0 (row-major) or 1 (blocked)");
     if (k_split != 0 && k_split != 1 && k_split != 2 && k_split != 4 && k_split != 8)
         return set_last_error(GPUK_ERR_INVALID_ARGUMENT, "fp8_linear: k_split must be 0, 1, 2, 4 or 8");
-    int device = 0, sms = 148;
-    if (cudaGetDevice(&device) != cudaSuccess) return set_last_error(GPUK_ERR_CUDA, "fp8_linear: no current device");
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    int sms = 0, *status = nullptr;
+    const int rc = decode_device(&sms, &status);
+    if (rc != GPUK_OK) return rc;
+    if (m > kTokens || (!fp8_frags_per_warp_tuning && static_cast<int64_t>(n) * k > kWarpMaxBytes)) {
+        StreamLinearCall c = {x_fp8, x_scale, w_scale, w_fp8, out_bf16, m, n, k, w_layout == 1, k_split, sms};
+        return stream_linear(c, status, static_cast<cudaStream_t>(stream));
+    }
     // split k as far as the whole grid still runs as one wave (two CTAs per SM) and every part keeps a few steps
     int ks = k_split;
     if (ks == 0) {
         ks = 1;
         while (ks < 8 && (n / kTileN) * ks * 2 <= 2 * sms && k / kStepBytes >= 8 * ks) ks *= 2;
     }
-    if (device < 0 || device >= 64) return set_last_error(GPUK_ERR_UNSUPPORTED, "fp8_linear: device index %d", device);
-    // one fragment per warp (eight warps), or two (four warps) for more than 16 tokens on 4096 channels or more: measured
-    // at 32 tokens, one / two fragments: n = 1280 9.1 / 10.3 us, n = 4096 14.0 / 13.1 us, n = 7168 21.8 / 21.2 us (k = 8192)
-    const void *fns[8] = {reinterpret_cast<const void *>(&fp8_linear_skinny_kernel<1, 1>), reinterpret_cast<const void *>(&fp8_linear_skinny_kernel<2, 1>),
-                          reinterpret_cast<const void *>(&fp8_linear_skinny_kernel<3, 1>), reinterpret_cast<const void *>(&fp8_linear_skinny_kernel<4, 1>),
-                          reinterpret_cast<const void *>(&fp8_linear_skinny_kernel<1, 2>), reinterpret_cast<const void *>(&fp8_linear_skinny_kernel<2, 2>),
-                          reinterpret_cast<const void *>(&fp8_linear_skinny_kernel<3, 2>), reinterpret_cast<const void *>(&fp8_linear_skinny_kernel<4, 2>)};
-    {
-        // first call on a device (guarded for concurrent callers): the status word, and the opt-in to more than
-        // 48 KiB of dynamic shared memory for every instantiation, so that no later call has set-up left to do
-        static std::mutex init_mutex;
-        std::lock_guard<std::mutex> lock(init_mutex);
-        if (!g_status_by_device[device]) {
-            for (const void *fn : fns) {
-                cudaError_t ea = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
-                if (ea != cudaSuccess)
-                    return set_last_error(GPUK_ERR_CUDA, "fp8_linear: cannot opt in to %d bytes of shared memory: %s", kSmemBytes, cudaGetErrorString(ea));
-            }
-            int *s = nullptr;
-            if (cudaMalloc(&s, sizeof(int)) != cudaSuccess) return set_last_error(GPUK_ERR_CUDA, "fp8_linear: cannot allocate the status word");
-            clear_status_kernel<<<1, 1, 0, static_cast<cudaStream_t>(stream)>>>(s);
-            g_status_by_device[device] = s;
-        }
-    }
     Fp8LinearParams p = {static_cast<const uint8_t *>(x_fp8), x_scale, static_cast<const uint8_t *>(w_fp8), w_scale,
-                         static_cast<__nv_bfloat16 *>(out_bf16), m, n, k, ks, w_layout, g_status_by_device[device]};
-    const int qn = (m + 7) / 8;
-    const int fr = (fp8_frags_per_warp_tuning == 1 || fp8_frags_per_warp_tuning == 2) ? fp8_frags_per_warp_tuning : ((qn >= 3 && n >= 4096) ? 2 : 1);
+                         static_cast<__nv_bfloat16 *>(out_bf16), m, n, k, ks, w_layout, status};
+    const int fr = fp8_frags_per_warp_tuning ? fp8_frags_per_warp_tuning : n >= 2048 ? 2 : 1;
+    const void *fn = fr == 2 ? reinterpret_cast<const void *>(&fp8_linear_skinny_kernel<2>) : reinterpret_cast<const void *>(&fp8_linear_skinny_kernel<1>);
     void *args[] = {&p};
-    cudaError_t e = launch_kernel(fns[(fr - 1) * 4 + qn - 1], (n / kTileN) * ks, kThreads / fr, ks, false, args, static_cast<cudaStream_t>(stream), kSmemBytes);
+    cudaError_t e = launch_kernel(fn, (n / kTileN) * ks, kThreads / fr, ks, false, args, static_cast<cudaStream_t>(stream), kSmemBytes);
     if (e != cudaSuccess) return set_last_error(GPUK_ERR_CUDA, "fp8_linear: launch failed: %s", cudaGetErrorString(e));
     return GPUK_OK;
 }

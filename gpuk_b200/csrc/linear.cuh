@@ -1,0 +1,24 @@
+// What the kernels of a decode step share: their set-up per device, and the call of the streaming linear layer.
+#pragma once
+
+#include <cuda_runtime.h>
+
+namespace gpuk {
+
+struct StreamLinearCall {
+    const void *x;                          // [m, k]
+    const float *x_scale, *w_scale;         // [m], [n]; nullptr: bf16 operands
+    const void *w;                          // [n, k] row-major, or blocked
+    void *out;                              // bf16 [m, n]
+    int m, n, k;                            // m <= 32, n a multiple of 128, rows of k a multiple of 16 bytes
+    bool blocked;                           // FP8 weights in the order of gpuk_fp8_pack_weight
+    int ks;                                 // CTAs that share a tile (0: chosen from the shape)
+    int sms;
+};
+cudaError_t stream_linear_setup();          // once per device
+// The current device's SMs and the status word that kernels of a decode step set (gpuk_fp8_linear_status); the first call on a device
+// opts the kernels in to their shared memory, so that no later call has set-up left to do.
+int decode_device(int *sms, int **status);
+int stream_linear(const StreamLinearCall &c, int *status, cudaStream_t stream);
+
+}  // namespace gpuk

@@ -74,11 +74,27 @@ PyObject *silu_mul(PyObject *, PyObject *const *args, Py_ssize_t n) {
     END_HANDLE_TH_ERRORS
 }
 
+// linear(x [m, k], w [n, k]) -> [m, n], bf16, m <= 32
+PyObject *linear(PyObject *, PyObject *const *args, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    expect_args(n, 2, "linear");
+    const Tensor &x = cuda_arg(args[0], "x", at::kBFloat16);
+    const Tensor &w = cuda_arg(args[1], "w", at::kBFloat16, x.get_device());
+    TORCH_CHECK(x.dim() == 2 && w.dim() == 2 && x.size(1) == w.size(1), "gpuk: linear operand shapes do not match");
+    c10::cuda::CUDAGuard guard(x.device());
+    Tensor out = empty_like_on(x, {x.size(0), w.size(0)}, at::kBFloat16);
+    check(gpuk_linear_skinny(x.data_ptr(), w.data_ptr(), out.data_ptr(), static_cast<int>(x.size(0)), static_cast<int>(w.size(0)), static_cast<int>(x.size(1)), 0,
+                             stream_of(x)), "linear");
+    return THPVariable_Wrap(std::move(out));
+    END_HANDLE_TH_ERRORS
+}
+
 template <PyObject *(*F)(PyObject *, PyObject *const *, Py_ssize_t)>
 constexpr PyCFunction fast() { return reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(F)); }
 
 PyMethodDef methods[] = {
     {"rope_append", fast<rope_append>(), METH_FASTCALL, nullptr},
+    {"linear", fast<linear>(), METH_FASTCALL, nullptr},
     {"silu_mul", fast<silu_mul>(), METH_FASTCALL, nullptr},
     {nullptr, nullptr, 0, nullptr},
 };

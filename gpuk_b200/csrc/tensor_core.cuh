@@ -1,0 +1,106 @@
+// The fifth-generation tensor core and the tensor-map copies that feed it, as thin device functions: tcgen05.mma on
+// operands in shared memory with the accumulator in tensor memory, and tiled TMA loads.  Names follow the PTX ISA.
+#pragma once
+
+#include <cuda.h>
+#include <cuda_runtime.h>
+
+#include "common.cuh"
+
+namespace gpuk {
+
+// ---- shared-memory operands ---------------------------------------------------------------
+// Descriptor of a K-major operand tile whose rows are one swizzle span (64 or 128 bytes) of K: groups of eight rows follow
+// each other, eight spans apart.  The tile starts on a boundary of eight spans; a step along K inside the span adds its bytes
+// to the start address, since the swizzle is a function of the address.
+template <int SPAN>
+__device__ __forceinline__ uint64_t kmajor_desc(uint32_t addr) {
+    static_assert(SPAN == 64 || SPAN == 128, "swizzle span");
+    constexpr uint64_t swizzle = SPAN == 128 ? 2 : 4;
+    return static_cast<uint64_t>((addr & 0x3ffffu) >> 4) | (1ull << 16) | (static_cast<uint64_t>(8 * SPAN / 16) << 32) | (1ull << 46) | (swizzle << 61);
+}
+
+// Instruction descriptor: fp32 accumulator, operand types `fa` and `fb` (kind::f16: 0 f16, 1 bf16; kind::f8f6f4: 0 e4m3), both operands K-major
+// unless `b_mn_major`.
+__host__ __device__ constexpr uint32_t mma_desc(int fa, int fb, int m, int n, bool b_mn_major = false) {
+    return (1u << 4) | (static_cast<uint32_t>(fa) << 7) | (static_cast<uint32_t>(fb) << 10) | (b_mn_major ? 1u << 16 : 0u) |
+           (static_cast<uint32_t>(n >> 3) << 17) | (static_cast<uint32_t>(m >> 4) << 24);
+}
+
+// ---- matrix multiplication (one thread issues) ------------------------------------------------
+__device__ __forceinline__ void tc_mma_f16(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, bool accumulate) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+                 ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(static_cast<uint32_t>(accumulate)) : "memory");
+}
+__device__ __forceinline__ void tc_mma_f8(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, bool accumulate) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}"
+                 ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(static_cast<uint32_t>(accumulate)) : "memory");
+}
+// `bar` gets one arrival once every multiplication this thread has issued so far is complete.
+__device__ __forceinline__ void tc_commit(uint64_t *bar) {
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_addr(bar)) : "memory");
+}
+
+// ---- tensor memory ---------------------------------------------------------------------------
+template <int COLS>
+__device__ __forceinline__ void tmem_alloc(uint32_t *slot) {      // one whole warp
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(slot)), "n"(COLS) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+}
+template <int COLS>
+__device__ __forceinline__ void tmem_free(uint32_t addr) {        // the same warp
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(addr), "n"(COLS) : "memory");
+}
+__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+
+// 16 columns of this warp's 32 lanes: register j of a thread is column j of its lane.
+__device__ __forceinline__ void tmem_ld16(float *r, uint32_t addr) {
+    uint32_t v[16];
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]),
+                   "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+                 : "r"(addr) : "memory");
+#pragma unroll
+    for (int i = 0; i < 16; ++i) r[i] = __uint_as_float(v[i]);
+}
+
+// ---- tiled copies ------------------------------------------------------------------------------
+__device__ __forceinline__ void prefetch_map(const CUtensorMap *map) {
+    asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
+}
+// L2 eviction priorities of a copy, as createpolicy would encode them for the whole access.
+__device__ __forceinline__ uint64_t policy_evict_first() {
+    uint64_t p;
+    asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
+    return p;
+}
+__device__ __forceinline__ uint64_t policy_evict_last() {
+    uint64_t p;
+    asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(p));
+    return p;
+}
+__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map, int x, int y, uint64_t *bar, uint64_t policy) {
+    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%2, %3}], [%4], %5;"
+                 ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(smem_addr(bar)), "l"(policy) : "memory");
+}
+__device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap *map, int x, int y, int z, int w, uint64_t *bar, uint64_t policy) {
+    asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%2, %3, %4, %5}], [%6], %7;"
+                 ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "r"(w), "r"(smem_addr(bar)), "l"(policy) : "memory");
+}
+// The same tile into L2 only: a hint, which may come before the data is final (L2 is where all SMs' accesses meet).
+__device__ __forceinline__ void tma_prefetch_2d(const CUtensorMap *map, int x, int y) {
+    asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y) : "memory");
+}
+__device__ __forceinline__ void tma_prefetch_4d(const CUtensorMap *map, int x, int y, int z, int w) {
+    asm volatile("cp.async.bulk.prefetch.tensor.4d.L2.global.tile [%0, {%1, %2, %3, %4}];"
+                 ::"l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
+}
+
+// Host: a tensor map of `rank` dimensions (sizes and box innermost first, strides in bytes of dimensions 1 and up).  Nonzero where
+// the driver refuses it.
+int encode_map(CUtensorMap *map, CUtensorMapDataType type, const void *base, int rank, const uint64_t *sizes, const uint64_t *strides, const uint32_t *box,
+               CUtensorMapSwizzle swizzle);
+
+}  // namespace gpuk

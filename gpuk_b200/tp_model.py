@@ -12,10 +12,10 @@ replaces ``reduce_from_tensor_parallel_region`` + ``x + ...`` + the following ``
 (``tensor_parallel.py:117-118``, ``transformer_model.py:610-618``) at both sites of every
 layer.  With ``fp8=True`` the normalised activations leave the operator as FP8-e4m3 with one
 scale per token, and the column-parallel projections that consume them run as FP8 GEMMs with
-row-wise scales: for decode batches this library's own weight-streaming kernel (``gpuk_b200.fp8_linear``,
-``csrc/fp8_linear.cu``) where it is the faster one on B200 (up to 16 tokens, or up to 32 tokens and at most 4096
-output channels per shard; measured in ``bench.py --case fp8_linear``), otherwise ``torch._scaled_mm`` (a library
-GEMM; ``own_fp8_gemm=False`` uses it everywhere).  Both give the same results to within one bf16 step.
+row-wise scales: for decode batches of up to 32 tokens this library's own weight-streaming kernels
+(``gpuk_b200.fp8_linear``, ``csrc/fp8_linear.cu`` and ``csrc/stream_linear.cu``; the row-parallel projections in bf16 likewise),
+otherwise ``torch._scaled_mm`` (a library GEMM; ``own_fp8_gemm=False`` uses libraries everywhere).  Both give the same results to
+within one bf16 step.
 
 ``fused=False`` runs the reference arrangement on the same weights -- NCCL ``all_reduce``, then
 add, RMSNorm (and quantisation) as separate PyTorch operators -- and is the comparison arm.
@@ -75,26 +75,30 @@ class _Linear:
     def __init__(self, weight: torch.Tensor, fp8: bool, own_gemm: bool = True):
         self.weight = weight                                  # [out_local, in]
         self.fp8 = fp8
-        self.own_gemm = own_gemm                              # decode batches: this library's weight-streaming FP8 kernel
-        self.w_packed = None                                  # ... its blocked copy of the weights, made at first use
+        self.own_gemm = own_gemm                              # decode batches: this library's weight-streaming kernels
+        self.w_packed = None                                  # ... and a blocked copy of FP8 weights, made at first use
         if fp8:
             amax = weight.float().abs().amax(dim=1, keepdim=True).clamp_(min=1e-12)
             self.w_scale = (amax / 448.0).t().contiguous()    # [1, out_local] fp32, one scale per output channel
             self.w_q = (weight.float() / amax * 448.0).clamp_(-448, 448).to(torch.float8_e4m3fn)   # [out, in] row-major
 
     def __call__(self, x: torch.Tensor, x_scale: Optional[torch.Tensor] = None) -> torch.Tensor:
+        # measured on B200: at up to 32 tokens the streaming kernels are the faster ones at the decoder's shapes (fp8_linear.cu, stream_linear.cu)
+        own = self.own_gemm and x.is_cuda and 0 < x.shape[0] <= 32 and self.weight.dtype == torch.bfloat16
         if self.fp8 and x.dtype == torch.float8_e4m3fn:
-            if self.own_gemm and x.is_cuda:
+            if own:
                 import gpuk_b200 as gpuk
-                # measured on B200 (bench.py --case fp8_linear): faster than the library GEMM up to 16 tokens at every
-                # shape of the decoder, and up to 32 tokens where the shard has at most 4096 output channels
-                m, n = x.shape[0], self.w_q.shape[0]
-                if (gpuk.fp8_linear_supported(m, n, self.w_q.shape[1]) and (m <= 16 or n <= 4096)
-                        and self.weight.dtype == torch.bfloat16):
+                if gpuk.fp8_linear_supported(x.shape[0], *self.w_q.shape):
+                    if x.shape[0] > 8:
+                        return gpuk.fp8_linear(x, x_scale, self.w_q, self.w_scale)
+                    # up to 8 tokens blocked weights are 3 to 12 % faster (2048 x 5120: 4.9 / 5.7 us), beyond within 2 % of row-major ones
                     if self.w_packed is None:
                         self.w_packed = gpuk.fp8_pack_weight(self.w_q)
                     return gpuk.fp8_linear(x, x_scale, self.w_packed, self.w_scale, packed=True)
             return torch._scaled_mm(x, self.w_q.t(), scale_a=x_scale, scale_b=self.w_scale, out_dtype=self.weight.dtype)
+        if own and x.dtype == torch.bfloat16 and self.weight.shape[0] % 128 == 0 and self.weight.shape[1] % 8 == 0:
+            from gpuk_b200 import _native
+            return _native.linear(x, self.weight)
         return F.linear(x, self.weight)
 
 
@@ -136,9 +140,9 @@ class TPDecoder:
             self.layers.append({
                 # one GEMM for q|k|v and one for w1|w3: they share their input
                 "wqkv": _Linear(torch.cat([wq, wk, wv], 0), fp8, own_fp8_gemm),
-                "wo": _Linear(make(a.dim, a.n_heads * hd, t + 4, "cols"), False),
+                "wo": _Linear(make(a.dim, a.n_heads * hd, t + 4, "cols"), False, own_fp8_gemm),
                 "w13": _Linear(torch.cat([w1, w3], 0), fp8, own_fp8_gemm),
-                "w2": _Linear(make(a.dim, a.ffn_dim, t + 7, "cols"), False),
+                "w2": _Linear(make(a.dim, a.ffn_dim, t + 7, "cols"), False, own_fp8_gemm),
                 "attention_norm": (1 + 0.1 * torch.randn(a.dim, generator=norm_gen)).to(a.dtype).to(self.device),
                 "ffn_norm": (1 + 0.1 * torch.randn(a.dim, generator=norm_gen)).to(a.dtype).to(self.device),
                 "k_cache": torch.zeros(max_batch, self.kv_local, a.max_seq_len, hd, dtype=a.dtype, device=self.device),
@@ -223,6 +227,8 @@ class TPDecoder:
             from gpuk_b200 import _native
             if last > a.max_seq_len:
                 raise RuntimeError(f"position {last - 1} is beyond the KV cache ({a.max_seq_len} positions)")
+            if input_pos.shape != (t,):
+                raise RuntimeError(f"{t} tokens a sequence at positions of shape {tuple(input_pos.shape)}")
             pos = input_pos.to(device=self.device, dtype=torch.int64).contiguous()
         else:
             cos, sin = self.cos[input_pos], self.sin[input_pos]
@@ -240,8 +246,8 @@ class TPDecoder:
                 layer["k_cache"][:b, :, input_pos] = k.transpose(1, 2)
                 layer["v_cache"][:b, :, input_pos] = v.transpose(1, 2)
             att = F.scaled_dot_product_attention(q.transpose(1, 2), layer["k_cache"][:b, :, :last], layer["v_cache"][:b, :, :last],
-                                                 attn_mask=mask, enable_gqa=True)
-            partial = layer["wo"](att.transpose(1, 2).reshape(b * t, self.h_local * hd))
+                                                 attn_mask=mask, enable_gqa=True).transpose(1, 2).reshape(b * t, self.h_local * hd)
+            partial = layer["wo"](att)
             h, normed, scale = self._reduce_add_norm(partial, h, layer["ffn_norm"])
             g13 = layer["w13"](normed, scale)
             if own:

@@ -280,8 +280,9 @@ int gpuk_ws_set_option(gpuk_ws *ws, const char *name, int64_t value);
  * 0 = never use it, -1 = default), "k1_staged_min_rows" (rows from which that variant runs,
  * -1 = default: more rows than the plain kernel has resident CTAs), "k1_ctas_per_sm" (cap on its
  * resident CTAs per SM, 0 = as many as fit).  One more name belongs to gpuk_fp8_linear_skinny:
- * "fp8_frags_per_warp" (16-row fragments a warp multiplies per k step: 1 = eight warps per CTA, 2 = four warps
- * that convert each activation vector once for two fragments; 0 = default: 2 for more than 16 tokens on at least 4096 output channels, else 1).
+ * "fp8_frags_per_warp" (16-row fragments a warp of its warp-level kernel multiplies per k step: 1 = eight warps per CTA, 2 = four
+ * warps that convert each activation vector once for two fragments, either for all calls of at most 8 tokens; 0 = default: that kernel for
+ * at most 8 tokens on weights of up to 12 MiB, with 2 fragments from 2048 output channels; the tcgen05 kernel beyond).
  * Not thread-safe against concurrent calls.
  */
 int gpuk_set_tuning(const char *name, int64_t value);
@@ -350,8 +351,14 @@ int gpuk_fp8_linear_skinny(const void *x_fp8, const float *x_scale, const void *
  */
 int gpuk_fp8_pack_weight(const void *w_fp8, void *packed, int n, int k, void *stream);
 /*
- * Synchronises the current device and returns GPUK_ERR_BAD_LAUNCH if a gpuk_fp8_linear_skinny launch on it
- * found itself in another thread-block cluster than planned (it then wrote nothing), else GPUK_OK.
+ * The same in bf16: out[m, n] = (x . w^T)[m, n] with x [m, k] and w [n, k] row-major, fp32 accumulation, one rounding.
+ * For the row-parallel projections of a decode batch (F.linear in model/tensor_parallel.py:117).  m <= 32, n a multiple of
+ * 128, k of 8, operands 16-byte aligned.  k_split as above, any value from 1 to 8; 0: chosen from the shape.
+ */
+int gpuk_linear_skinny(const void *x_bf16, const void *w_bf16, void *out_bf16, int m, int n, int k, int k_split, void *stream);
+/*
+ * Synchronises the current device and returns GPUK_ERR_BAD_LAUNCH if a launch of one of the two calls above on it
+ * found itself in another thread-block cluster than planned (it then wrote nothing) or gave up a wait, else GPUK_OK.
  * Same contract as status 3 of gpuk_ws_status; the reference has no counterpart (impl.h launches no clusters).
  */
 int gpuk_fp8_linear_status(void);
