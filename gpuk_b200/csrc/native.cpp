@@ -89,12 +89,32 @@ PyObject *linear(PyObject *, PyObject *const *args, Py_ssize_t n) {
     END_HANDLE_TH_ERRORS
 }
 
+// decode_attention(q [batch, heads, 128], k_cache, v_cache [>= batch, kv_heads, max_seq, 128], len) -> [batch, heads * 128]
+PyObject *decode_attention(PyObject *, PyObject *const *args, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    expect_args(n, 4, "decode_attention");
+    const Tensor &q = cuda_arg(args[0], "q", at::kBFloat16);
+    const int dev = q.get_device();
+    const Tensor &kc = cuda_arg(args[1], "k_cache", at::kBFloat16, dev), &vc = cuda_arg(args[2], "v_cache", at::kBFloat16, dev);
+    const int64_t len = int_arg(args[3]);
+    TORCH_CHECK(q.dim() == 3 && kc.dim() == 4 && vc.sizes() == kc.sizes() && q.size(0) <= kc.size(0) && q.size(2) == kc.size(3) && len <= kc.size(2),
+                "gpuk: decode_attention shapes do not match");
+    c10::cuda::CUDAGuard guard(q.device());
+    Tensor out = empty_like_on(q, {q.size(0), q.size(1) * q.size(2)}, at::kBFloat16);
+    check(gpuk_decode_attention(q.data_ptr(), kc.data_ptr(), vc.data_ptr(), out.data_ptr(), static_cast<int>(q.size(0)), static_cast<int>(q.size(1)),
+                                static_cast<int>(kc.size(1)), static_cast<int>(q.size(2)), static_cast<int>(len), static_cast<int>(kc.size(2)), 0, stream_of(q)),
+          "decode_attention");
+    return THPVariable_Wrap(std::move(out));
+    END_HANDLE_TH_ERRORS
+}
+
 template <PyObject *(*F)(PyObject *, PyObject *const *, Py_ssize_t)>
 constexpr PyCFunction fast() { return reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(F)); }
 
 PyMethodDef methods[] = {
     {"rope_append", fast<rope_append>(), METH_FASTCALL, nullptr},
     {"linear", fast<linear>(), METH_FASTCALL, nullptr},
+    {"decode_attention", fast<decode_attention>(), METH_FASTCALL, nullptr},
     {"silu_mul", fast<silu_mul>(), METH_FASTCALL, nullptr},
     {nullptr, nullptr, 0, nullptr},
 };

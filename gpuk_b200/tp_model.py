@@ -157,6 +157,8 @@ class TPDecoder:
         self._zeros = {}
         # the elementwise steps between the projections as this library's kernels (csrc/decoder_ops.cu)
         self.own_elementwise = fused and self.device.type == "cuda" and a.dtype == torch.bfloat16 and hd % 16 == 0 and a.ffn_dim // w % 8 == 0
+        # ... and so attention over the cache for one new token per sequence (csrc/attention.cu)
+        self.own_attention = hd == 128 and self.h_local % self.kv_local == 0 and self.h_local // self.kv_local <= 16
 
     # ------------------------------------------------------------------------------------
     def fill_kv_cache(self, upto: int, seed: int = 7) -> None:
@@ -245,8 +247,11 @@ class TPDecoder:
                 q, k = self._rope(q, cos, sin), self._rope(k, cos, sin)
                 layer["k_cache"][:b, :, input_pos] = k.transpose(1, 2)
                 layer["v_cache"][:b, :, input_pos] = v.transpose(1, 2)
-            att = F.scaled_dot_product_attention(q.transpose(1, 2), layer["k_cache"][:b, :, :last], layer["v_cache"][:b, :, :last],
-                                                 attn_mask=mask, enable_gqa=True).transpose(1, 2).reshape(b * t, self.h_local * hd)
+            if own and t == 1 and self.own_attention:
+                att = _native.decode_attention(q.view(b, self.h_local, hd), layer["k_cache"], layer["v_cache"], last)
+            else:
+                att = F.scaled_dot_product_attention(q.transpose(1, 2), layer["k_cache"][:b, :, :last], layer["v_cache"][:b, :, :last],
+                                                     attn_mask=mask, enable_gqa=True).transpose(1, 2).reshape(b * t, self.h_local * hd)
             partial = layer["wo"](att)
             h, normed, scale = self._reduce_add_norm(partial, h, layer["ffn_norm"])
             g13 = layer["w13"](normed, scale)

@@ -357,7 +357,15 @@ int gpuk_fp8_pack_weight(const void *w_fp8, void *packed, int n, int k, void *st
  */
 int gpuk_linear_skinny(const void *x_bf16, const void *w_bf16, void *out_bf16, int m, int n, int k, int k_split, void *stream);
 /*
- * Synchronises the current device and returns GPUK_ERR_BAD_LAUNCH if a launch of one of the two calls above on it
+ * Attention of one new token per sequence over a KV cache: out[b, h] = softmax(q[b, h] . k[b, h / group]^T / sqrt(128)) . v, over
+ * positions [0, len) of caches [>= batch, kv_heads, max_seq, 128]; q and out [batch, heads, 128], all bf16, group = heads / kv_heads
+ * at most 16.  q and caches 16-byte aligned.  splits = CTAs of a thread-block cluster that share the keys of a (sequence, kv head),
+ * 1 to 8; 0: chosen from the shape.
+ */
+int gpuk_decode_attention(const void *q, const void *k_cache, const void *v_cache, void *out, int batch, int heads, int kv_heads, int head_dim,
+                          int len, int max_seq, int splits, void *stream);
+/*
+ * Synchronises the current device and returns GPUK_ERR_BAD_LAUNCH if a launch of one of the three calls above on it
  * found itself in another thread-block cluster than planned (it then wrote nothing) or gave up a wait, else GPUK_OK.
  * Same contract as status 3 of gpuk_ws_status; the reference has no counterpart (impl.h launches no clusters).
  */

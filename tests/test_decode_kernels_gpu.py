@@ -1,4 +1,4 @@
-"""The kernels of a decode step -- streaming linear layers in FP8 and bf16 -- against float64."""
+"""The kernels of a decode step -- streaming linear layers in FP8 and bf16, attention over the KV cache -- against float64."""
 import pytest
 import torch
 
@@ -58,9 +58,34 @@ def test_fp8_linear_around_the_dispatch(m, n, k, packed):
     assert torch.equal(again.view(torch.int16), got.view(torch.int16)) and bool(torch.isnan(out[0]))
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("splits", [0, 1, 3, 8])
+@pytest.mark.parametrize("batch,heads,kv_heads,length,max_seq", [(1, 8, 2, 1, 1), (3, 16, 1, 17, 32), (2, 4, 4, 64, 64), (4, 16, 4, 129, 256), (5, 8, 1, 1000, 1024),
+                                                                (40, 64, 8, 80, 256)])
+def test_decode_attention(batch, heads, kv_heads, length, max_seq, splits):
+    """One key, ends inside a block of 16, parts of the cluster without keys, 1 to 16 query heads per kv head, both ring depths.  What lies behind
+    the keys is NaN.  Probabilities are rounded to bf16 before the second product (a relative 2^-8 each, half of the last of eight bits) and
+    the result once more: 2 * 2^-8 of sum(p |v|)."""
+    g = torch.Generator().manual_seed(batch + heads + length)
+    q = (torch.randn(batch, heads, 128, generator=g) * 2).bfloat16()
+    k, v = (torch.randn(batch + 1, kv_heads, max_seq, 128, generator=g).bfloat16() for _ in range(2))
+    k[:, :, length:], v[:, :, length:] = float("nan"), float("nan")
+    kk, vv = (t[:batch, :, :length].repeat_interleave(heads // kv_heads, 1).double() for t in (k, v))
+    p = torch.softmax(torch.einsum("bhd,bhkd->bhk", q.double(), kk) / 128 ** 0.5, -1)
+    want, bound = torch.einsum("bhk,bhkd->bhd", p, vv), torch.einsum("bhk,bhkd->bhd", p, vv.abs()) * 2.0 ** -7 + 1e-6
+    dq, dk, dv = q.cuda(), k.cuda(), v.cuda()
+    out = torch.full_like(dq, float("nan"))
+    cabi.check(cabi.lib.gpuk_decode_attention(_ptr(dq), _ptr(dk), _ptr(dv), _ptr(out), batch, heads, kv_heads, 128, length, max_seq, splits, _stream()))
+    _status_ok()
+    assert bool(((out.cpu().double() - want).abs() <= bound).all())
+
+
 def test_refused_shapes():
-    f = cabi.lib.gpuk_linear_skinny
+    f, a = cabi.lib.gpuk_linear_skinny, cabi.lib.gpuk_decode_attention
     assert f(16, 16, 16, 33, 128, 64, 0, None) == cabi.ERR_UNSUPPORTED and f(16, 16, 16, 8, 100, 64, 0, None) == cabi.ERR_UNSUPPORTED
     assert f(16, 16, 16, 8, 128, 12, 0, None) == cabi.ERR_UNSUPPORTED and f(16, 16, 16, 8, 128, 64, 9, None) == cabi.ERR_INVALID_ARGUMENT
     assert f(16, 8, 16, 8, 128, 64, 0, None) == cabi.ERR_INVALID_ARGUMENT and f(None, 16, 16, 8, 128, 64, 0, None) == cabi.ERR_INVALID_ARGUMENT
     assert f(16, 16, 16, 0, 128, 64, 0, None) == cabi.OK
+    assert a(16, 16, 16, 16, 1, 34, 2, 128, 4, 8, 0, None) == cabi.ERR_UNSUPPORTED      # 17 query heads per kv head
+    assert a(16, 16, 16, 16, 1, 8, 2, 64, 4, 8, 0, None) == cabi.ERR_UNSUPPORTED and a(16, 16, 16, 16, 1, 8, 2, 128, 9, 8, 0, None) == cabi.ERR_INVALID_ARGUMENT
+    assert a(16, 16, 16, 16, 0, 8, 2, 128, 4, 8, 0, None) == cabi.OK
