@@ -118,27 +118,7 @@ def fp8_linear(x_fp8: torch.Tensor, x_scale: torch.Tensor, w_fp8: torch.Tensor, 
     ``packed=True`` says ``w_fp8`` came from ``fp8_pack_weight``.
     Hand-written weight-streaming kernel (``csrc/fp8_linear.cu``); raises for shapes it is not built for --
     ``fp8_linear_supported`` tells, and larger batches belong to a library GEMM."""
-    import ctypes
-    if x_fp8.dtype != torch.float8_e4m3fn or w_fp8.dtype != torch.float8_e4m3fn:
-        raise RuntimeError("gpuk: fp8_linear takes float8_e4m3fn operands")
-    if not (x_fp8.is_cuda and x_fp8.is_contiguous() and w_fp8.is_contiguous() and x_fp8.dim() == 2 and w_fp8.dim() == 2):
-        raise RuntimeError("gpuk: fp8_linear takes contiguous 2-d CUDA tensors")
-    m, k = x_fp8.shape
-    n = w_fp8.shape[0]
-    if w_fp8.shape[1] != k or x_scale.numel() != m or w_scale.numel() != n:
-        raise RuntimeError("gpuk: fp8_linear operand shapes do not match")
-    if x_scale.dtype != torch.float32 or w_scale.dtype != torch.float32 or not x_scale.is_contiguous() or not w_scale.is_contiguous():
-        raise RuntimeError("gpuk: fp8_linear takes contiguous fp32 scales")
-    if out is None:
-        out = torch.empty(m, n, dtype=torch.bfloat16, device=x_fp8.device)
-    elif out.dtype != torch.bfloat16 or out.shape != (m, n) or not out.is_contiguous():
-        raise RuntimeError("gpuk: fp8_linear writes a contiguous bf16 [tokens, n] tensor")
-    with torch.cuda.device(x_fp8.device):
-        cabi.check(cabi.lib.gpuk_fp8_linear_skinny(
-            ctypes.c_void_p(x_fp8.data_ptr()), ctypes.c_void_p(x_scale.data_ptr()), ctypes.c_void_p(w_fp8.data_ptr()),
-            ctypes.c_void_p(w_scale.data_ptr()), ctypes.c_void_p(out.data_ptr()), m, n, k, 1 if packed else 0, k_split,
-            ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)))
-    return out
+    return _native.fp8_linear(x_fp8, x_scale, w_fp8, w_scale, out, packed, k_split)
 
 
 class _TorchOps:
@@ -397,7 +377,8 @@ class GPUKDistEnv:
         ``set_option("ws_max_ctas", n)``.  The reference has no counterpart.
         """
         self._require_workspace()
-        self.capture_(allreduce_in)
+        if self.fptr:
+            self.capture_(allreduce_in)      # without a workspace there is nothing to register
         if ready is not None:
             import ctypes
             words, rows_per_word, value = ready
@@ -408,6 +389,14 @@ class GPUKDistEnv:
                 raise RuntimeError(f"gpuk: {need} ready words needed, {words.numel()} given")
             cabi.check(cabi.lib.gpuk_ws_set_ready_words(ctypes.c_void_p(self.fptr), ctypes.c_void_p(words.data_ptr()),
                                                         int(rows_per_word), int(value)))
+        if self._o is _TorchOps and not torch.compiler.is_compiling():
+            qt = (QUANT_STATIC_E4M3FN_448 if static_scale is not None else
+                  QUANT_NONE if not fp8_out else fp8_policy_id if quant_type is None else quant_type)
+            if static_scale is None or isinstance(static_scale, torch.Tensor):
+                results = _native.add_rms(self.fptr or 0, allreduce_in, residual_in, rms_weight, eps, qt,
+                                          None if static_scale is None else static_scale.reshape(-1))
+                if results is not None:
+                    return results
         residual_out = torch.empty_like(residual_in)
         if static_scale is not None:
             fp8_out = True

@@ -184,6 +184,9 @@ class TPDecoder:
             if z is None:
                 z = self._zeros[h.shape] = torch.zeros_like(h)
             import gpuk_b200 as gpuk
+            results = gpuk._native.add_rms(0, h, z, weight, self.args.norm_eps, 3 if self.fp8 else 0, None)
+            if results is not None:
+                return results[1], results[2] if self.fp8 else None
             residual_out = torch.empty_like(h)
             if self.fp8:
                 normed = torch.empty(h.shape, dtype=torch.float8_e4m3fn, device=h.device)
