@@ -278,6 +278,7 @@ int gpuk::decode_device(int *sms, int **status) {
             if (e == cudaSuccess) e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
         if (e == cudaSuccess) e = stream_linear_setup();
         if (e == cudaSuccess) e = decode_attention_setup();
+        if (e == cudaSuccess) e = prefill_attention_setup();
         if (e == cudaSuccess) e = cudaDeviceGetAttribute(&g_sms_by_device[device], cudaDevAttrMultiProcessorCount, device);
         if (e != cudaSuccess) return set_last_error(GPUK_ERR_CUDA, "cannot prepare the kernels of a decode step: %s", cudaGetErrorString(e));
         g_status_by_device[device] = static_cast<int *>(word);

@@ -17,6 +17,7 @@ struct StreamLinearCall {
 };
 cudaError_t stream_linear_setup();          // once per device
 cudaError_t decode_attention_setup();
+cudaError_t prefill_attention_setup();
 // The current device's SMs and the status word that kernels of a decode step set (gpuk_fp8_linear_status); the first call on a device
 // opts the kernels in to their shared memory, so that no later call has set-up left to do.
 int decode_device(int *sms, int **status);

@@ -134,6 +134,30 @@ PyObject *decode_attention(PyObject *, PyObject *const *args, Py_ssize_t n) {
     END_HANDLE_TH_ERRORS
 }
 
+// prefill_attention(q [batch, t, heads, 128], k_cache, v_cache, pos [t], len) -> [batch * t, heads * 128]
+PyObject *prefill_attention(PyObject *, PyObject *const *args, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    expect_args(n, 5, "prefill_attention");
+    const Tensor &q = cuda_arg(args[0], "q", at::kBFloat16);
+    const int dev = q.get_device();
+    const Tensor &kc = cuda_arg(args[1], "k_cache", at::kBFloat16, dev), &vc = cuda_arg(args[2], "v_cache", at::kBFloat16, dev);
+    const Tensor &pos = cuda_arg(args[3], "positions", at::kLong, dev);
+    const int64_t len = int_arg(args[4]);
+    TORCH_CHECK(q.dim() == 4 && kc.dim() == 4 && vc.sizes() == kc.sizes() && q.size(0) <= kc.size(0) && q.size(3) == kc.size(3) && pos.numel() == q.size(1) && len <= kc.size(2),
+                "gpuk: prefill_attention shapes do not match");
+    Tensor out;
+    {
+        NoGil unlocked;
+        c10::cuda::CUDAGuard guard(q.device());
+        out = empty_like_on(q, {q.size(0) * q.size(1), q.size(2) * q.size(3)}, at::kBFloat16);
+        check(gpuk_prefill_attention(q.data_ptr(), kc.data_ptr(), vc.data_ptr(), pos.data_ptr<int64_t>(), out.data_ptr(), static_cast<int>(q.size(0)),
+                                     static_cast<int>(q.size(1)), static_cast<int>(q.size(2)), static_cast<int>(kc.size(1)), static_cast<int>(q.size(3)),
+                                     static_cast<int>(len), static_cast<int>(kc.size(2)), stream_of(q)), "prefill_attention");
+    }
+    return THPVariable_Wrap(std::move(out));
+    END_HANDLE_TH_ERRORS
+}
+
 // fp8_linear(x [m, k], x_scale, w [n, k], w_scale, out or None, packed, k_split) -> [m, n]
 PyObject *fp8_linear(PyObject *, PyObject *const *args, Py_ssize_t n) {
     HANDLE_TH_ERRORS
@@ -240,6 +264,7 @@ PyMethodDef methods[] = {
     {"rope_append", fast<rope_append>(), METH_FASTCALL, nullptr},
     {"linear", fast<linear>(), METH_FASTCALL, nullptr},
     {"decode_attention", fast<decode_attention>(), METH_FASTCALL, nullptr},
+    {"prefill_attention", fast<prefill_attention>(), METH_FASTCALL, nullptr},
     {"fp8_linear", fast<fp8_linear>(), METH_FASTCALL, nullptr},
     {"add_rms", fast<add_rms>(), METH_FASTCALL, nullptr},
     {"silu_mul", fast<silu_mul>(), METH_FASTCALL, nullptr},

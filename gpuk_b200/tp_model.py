@@ -157,8 +157,8 @@ class TPDecoder:
         self._zeros = {}
         # the elementwise steps between the projections as this library's kernels (csrc/decoder_ops.cu)
         self.own_elementwise = fused and self.device.type == "cuda" and a.dtype == torch.bfloat16 and hd % 16 == 0 and a.ffn_dim // w % 8 == 0
-        # ... and so attention over the cache for one new token per sequence (csrc/attention.cu)
-        self.own_attention = hd == 128 and self.h_local % self.kv_local == 0 and self.h_local // self.kv_local <= 16
+        # ... and so attention over the cache, for one new token per sequence (csrc/attention.cu) and for more (csrc/prefill_attention.cu)
+        self.own_attention = hd == 128 and self.h_local % self.kv_local == 0
 
     # ------------------------------------------------------------------------------------
     def fill_kv_cache(self, upto: int, seed: int = 7) -> None:
@@ -237,8 +237,9 @@ class TPDecoder:
             pos = input_pos.to(device=self.device, dtype=torch.int64).contiguous()
         else:
             cos, sin = self.cos[input_pos], self.sin[input_pos]
+        own_attention = own and self.own_attention
         mask = None
-        if t > 1:
+        if t > 1 and not own_attention:
             mask = (torch.arange(last, device=self.device)[None, :] <= input_pos[:, None])[None, None]
         normed, scale = self._norm_only(h, self.layers[0]["attention_norm"])
         for li, layer in enumerate(self.layers):
@@ -250,8 +251,10 @@ class TPDecoder:
                 q, k = self._rope(q, cos, sin), self._rope(k, cos, sin)
                 layer["k_cache"][:b, :, input_pos] = k.transpose(1, 2)
                 layer["v_cache"][:b, :, input_pos] = v.transpose(1, 2)
-            if own and t == 1 and self.own_attention:
+            if own_attention and t == 1 and self.h_local // self.kv_local <= 16:
                 att = _native.decode_attention(q.view(b, self.h_local, hd), layer["k_cache"], layer["v_cache"], last)
+            elif own_attention and t > 1:
+                att = _native.prefill_attention(q, layer["k_cache"], layer["v_cache"], pos, last)
             else:
                 att = F.scaled_dot_product_attention(q.transpose(1, 2), layer["k_cache"][:b, :, :last], layer["v_cache"][:b, :, :last],
                                                      attn_mask=mask, enable_gqa=True).transpose(1, 2).reshape(b * t, self.h_local * hd)

@@ -365,7 +365,13 @@ int gpuk_linear_skinny(const void *x_bf16, const void *w_bf16, void *out_bf16, i
 int gpuk_decode_attention(const void *q, const void *k_cache, const void *v_cache, void *out, int batch, int heads, int kv_heads, int head_dim,
                           int len, int max_seq, int splits, void *stream);
 /*
- * Synchronises the current device and returns GPUK_ERR_BAD_LAUNCH if a launch of one of the three calls above on it
+ * The same for t new tokens per sequence at positions pos [t] (int64, on the device): token i sees the cached positions [0, min(pos[i], len - 1)];
+ * one that sees none gets zeros.  q and out [batch, t, heads, 128]; any number of query heads per kv head.  Pointers 16-byte aligned.
+ */
+int gpuk_prefill_attention(const void *q, const void *k_cache, const void *v_cache, const int64_t *pos, void *out, int batch, int t, int heads, int kv_heads,
+                           int head_dim, int len, int max_seq, void *stream);
+/*
+ * Synchronises the current device and returns GPUK_ERR_BAD_LAUNCH if a launch of one of the four calls above on it
  * found itself in another thread-block cluster than planned (it then wrote nothing) or gave up a wait, else GPUK_OK.
  * Same contract as status 3 of gpuk_ws_status; the reference has no counterpart (impl.h launches no clusters).
  */

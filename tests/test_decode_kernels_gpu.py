@@ -1,4 +1,4 @@
-"""The kernels of a decode step -- streaming linear layers in FP8 and bf16, attention over the KV cache -- against float64."""
+"""The kernels of a decode step -- streaming linear layers in FP8 and bf16, attention over the KV cache for one and for many new tokens -- against float64."""
 import pytest
 import torch
 
@@ -80,6 +80,32 @@ def test_decode_attention(batch, heads, kv_heads, length, max_seq, splits):
     assert bool(((out.cpu().double() - want).abs() <= bound).all())
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("batch,t,heads,kv_heads,past", [(1, 2, 2, 1, 0), (1, 128, 4, 4, 0), (2, 129, 8, 2, 127), (1, 257, 17, 1, 0), (3, 40, 4, 2, 300), (1, 300, 2, 1, 1700)])
+@pytest.mark.parametrize("order", ["rising", "mixed"])
+def test_prefill_attention(batch, t, heads, kv_heads, past, order):
+    """Both tiles of a CTA, ends at, before and behind a tile of queries and a block of keys, a ring that wraps, queries of a next sequence in the tile;
+    positions in order, and in any order with one that sees no key and one beyond the cache.  Bound as for one token."""
+    g = torch.Generator().manual_seed(batch + t + heads)
+    length, max_seq = past + t, past + t + 5
+    q = (torch.randn(batch, t, heads, 128, generator=g) * 2).bfloat16()
+    k, v = (torch.randn(batch, kv_heads, max_seq, 128, generator=g).bfloat16() for _ in range(2))
+    k[:, :, length:], v[:, :, length:] = float("nan"), float("nan")
+    pos = torch.arange(past, length)
+    if order == "mixed":
+        pos = pos[torch.randperm(t, generator=g)]
+        pos[0], pos[-1] = -1, length + 3
+    kk, vv = (x[:, :, :length].repeat_interleave(heads // kv_heads, 1).double() for x in (k, v))
+    s = torch.einsum("bthd,bhkd->bhtk", q.double(), kk) / 128 ** 0.5
+    p = torch.softmax(s.masked_fill(torch.arange(length) > pos[:, None], float("-inf")), -1).nan_to_num(0.0)
+    want, bound = torch.einsum("bhtk,bhkd->bthd", p, vv), torch.einsum("bhtk,bhkd->bthd", p, vv.abs()) * 2.0 ** -7 + 1e-6
+    dq, dk, dv, dp = q.cuda(), k.cuda(), v.cuda(), pos.cuda()
+    out = torch.full_like(dq, float("nan"))
+    cabi.check(cabi.lib.gpuk_prefill_attention(_ptr(dq), _ptr(dk), _ptr(dv), _ptr(dp), _ptr(out), batch, t, heads, kv_heads, 128, length, max_seq, _stream()))
+    _status_ok()
+    assert bool(((out.cpu().double() - want).abs() <= bound).all())
+
+
 def test_refused_shapes():
     f, a = cabi.lib.gpuk_linear_skinny, cabi.lib.gpuk_decode_attention
     assert f(16, 16, 16, 33, 128, 64, 0, None) == cabi.ERR_UNSUPPORTED and f(16, 16, 16, 8, 100, 64, 0, None) == cabi.ERR_UNSUPPORTED
@@ -89,3 +115,7 @@ def test_refused_shapes():
     assert a(16, 16, 16, 16, 1, 34, 2, 128, 4, 8, 0, None) == cabi.ERR_UNSUPPORTED      # 17 query heads per kv head
     assert a(16, 16, 16, 16, 1, 8, 2, 64, 4, 8, 0, None) == cabi.ERR_UNSUPPORTED and a(16, 16, 16, 16, 1, 8, 2, 128, 9, 8, 0, None) == cabi.ERR_INVALID_ARGUMENT
     assert a(16, 16, 16, 16, 0, 8, 2, 128, 4, 8, 0, None) == cabi.OK
+    b = cabi.lib.gpuk_prefill_attention
+    assert b(16, 16, 16, 16, 16, 1, 4, 8, 2, 64, 4, 8, None) == cabi.ERR_UNSUPPORTED and b(16, 16, 16, 16, 16, 1, 4, 8, 3, 128, 4, 8, None) == cabi.ERR_UNSUPPORTED
+    assert b(16, 16, 16, 16, 16, 1, 4, 8, 2, 128, 9, 8, None) == cabi.ERR_INVALID_ARGUMENT and b(16, 16, 8, 16, 16, 1, 4, 8, 2, 128, 4, 8, None) == cabi.ERR_INVALID_ARGUMENT
+    assert b(16, 16, 16, 16, 16, 1, 0, 8, 2, 128, 4, 8, None) == cabi.OK
