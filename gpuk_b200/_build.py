@@ -28,7 +28,7 @@ NVCC_FLAGS = [
 ]
 CORE_SOURCES = ["core.cu", "launch_bf16.cu", "launch_f16.cu", "launch_f32.cu", "noalloc.cu", "fp8_linear.cu", "stream_linear.cu", "tensor_map.cu", "decoder_ops.cu",
                 "attention.cu", "prefill_attention.cu"]
-HEADERS = ["common.cuh", "epilogue.cuh", "kernels.cuh", "launch.cuh", "launch_impl.cuh", "linear.cuh", "tensor_core.cuh",
+HEADERS = ["common.cuh", "epilogue.cuh", "kernels.cuh", "launch.cuh", "launch_impl.cuh", "linear.cuh", "tensor_core.cuh", "decoder_math.cuh",
            os.path.join(ROOT, "include", "gpuk_b200.h")]
 
 

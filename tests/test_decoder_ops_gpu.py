@@ -65,3 +65,17 @@ def test_shapes_that_are_not_built_are_refused():
         _native.silu_mul(x.cpu())
     assert cabi.lib.gpuk_silu_mul(None, None, 0, 8, None) == cabi.OK
     assert gpuk_b200._native is _native
+
+
+@pytest.mark.parametrize("rows,f", [(1, 8), (3, 2048), (1, 2056), (1200, 4104)])
+def test_silu_mul_at_the_ends_of_a_chunk_and_of_the_range(rows, f):
+    """One and two vectors a thread, rows that end inside a chunk; infinities, NaN, zeros of both signs, quotients that leave the range."""
+    special = torch.tensor([float("inf"), float("-inf"), float("nan"), 0.0, -0.0, -88.5, -89.0, -104.0, 88.0, 3e38, -3e38, 1e-39, -70.0, -1e-31, 2e30, 1.0])
+    g = torch.Generator().manual_seed(rows + f)
+    x = torch.randn(rows, 2 * f, generator=g) * 3
+    x[0, :min(f, 16)] = special[:min(f, 16)]
+    x = x.bfloat16().cuda()
+    a, b = x.split(f, -1)
+    want, got = F.silu(a) * b, _native.silu_mul(x)
+    nan = want.isnan()
+    assert torch.equal(got.isnan(), nan) and torch.equal(got[~nan].view(torch.int16), want[~nan].view(torch.int16))
