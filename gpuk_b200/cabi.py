@@ -82,6 +82,8 @@ _SIGNATURES = {
     "gpuk_fp8_linear_status": (c_int, []),
     "gpuk_linear_skinny": (c_int, [_P, _P, _P, c_int, c_int, c_int, c_int, _P]),
     "gpuk_decode_attention": (c_int, [_P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int, c_int, c_int, _P]),
+    "gpuk_swiglu_skinny": (c_int, [_P, _P, _P, _P, _P, c_int, c_int, c_int, c_int, _P]),
+    "gpuk_qkv_rope_skinny": (c_int, [_P] * 10 + [c_int] * 8 + [_P]),
     "gpuk_prefill_attention": (c_int, [_P, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int, c_int, c_int, _P]),
     "gpuk_rope_append": (c_int, [_P, _P, _P, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int, c_int, c_int, _P]),
     "gpuk_silu_mul": (c_int, [_P, _P, c_int64, c_int, _P]),

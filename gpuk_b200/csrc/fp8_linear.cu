@@ -307,7 +307,7 @@ extern "C" int gpuk_fp8_linear_skinny(const void *x_fp8, const float *x_scale, c
     const int rc = decode_device(&sms, &status);
     if (rc != GPUK_OK) return rc;
     if (m > kTokens || (!fp8_frags_per_warp_tuning && static_cast<int64_t>(n) * k > kWarpMaxBytes)) {
-        StreamLinearCall c = {x_fp8, x_scale, w_scale, w_fp8, out_bf16, m, n, k, w_layout == 1, k_split, sms};
+        StreamLinearCall c = {x_fp8, x_scale, w_scale, w_fp8, out_bf16, m, n, k, w_layout == 1, kPlain, {}, k_split, sms};
         return stream_linear(c, status, static_cast<cudaStream_t>(stream));
     }
     // split k as far as the whole grid still runs as one wave (two CTAs per SM) and every part keeps a few steps

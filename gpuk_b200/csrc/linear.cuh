@@ -3,7 +3,18 @@
 
 #include <cuda_runtime.h>
 
+#include <cstdint>
+
 namespace gpuk {
+
+// What the streaming kernel does with its sums before it stores them.
+enum LinearEpilogue { kPlain, kSwiGlu, kRopeAppend };
+struct RopeCall {
+    const float *cos, *sin;                 // [table_rows, 64]
+    const int64_t *pos;                     // [t]
+    void *k_cache, *v_cache;                // bf16 [batch, kv_heads, max_seq, 128]
+    int t, heads, kv_heads, table_rows, max_seq;
+};
 
 struct StreamLinearCall {
     const void *x;                          // [m, k]
@@ -12,6 +23,8 @@ struct StreamLinearCall {
     void *out;                              // bf16 [m, n]
     int m, n, k;                            // m <= 32, n a multiple of 128, rows of k a multiple of 16 bytes
     bool blocked;                           // FP8 weights in the order of gpuk_fp8_pack_weight
+    LinearEpilogue epilogue;                // kSwiGlu: out [m, n / 2] = silu(first half) * second half; kRopeAppend: out [m, heads * 128], keys and values to the caches
+    RopeCall rope;
     int ks;                                 // CTAs that share a tile (0: chosen from the shape)
     int sms;
 };

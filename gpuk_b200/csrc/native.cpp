@@ -111,6 +111,62 @@ PyObject *linear(PyObject *, PyObject *const *args, Py_ssize_t n) {
     END_HANDLE_TH_ERRORS
 }
 
+// x [m, k] and w [n, k] in FP8 with their scales, or in bf16 with None for both: checked, and as the C ABI takes them.
+struct Operands {
+    const Tensor &x, &w;
+    const float *x_scale = nullptr, *w_scale = nullptr;
+    int m, n, k;
+    Operands(PyObject *const *args) : x(cuda_arg(args[0], "x", args[1] == Py_None ? at::kBFloat16 : at::kFloat8_e4m3fn)), w(cuda_arg(args[2], "w", x.scalar_type(), x.get_device())) {
+        TORCH_CHECK(x.dim() == 2 && w.dim() == 2 && x.size(1) == w.size(1) && (args[1] == Py_None) == (args[3] == Py_None), "gpuk: linear operand shapes do not match");
+        TORCH_CHECK(x.size(0) <= INT_MAX && w.size(0) <= INT_MAX && w.size(1) <= INT_MAX, "gpuk: linear sizes out of range");
+        m = static_cast<int>(x.size(0)), n = static_cast<int>(w.size(0)), k = static_cast<int>(w.size(1));
+        if (args[1] == Py_None) return;
+        const Tensor &xs = cuda_arg(args[1], "x_scale", at::kFloat, x.get_device()), &ws = cuda_arg(args[3], "w_scale", at::kFloat, x.get_device());
+        TORCH_CHECK(xs.numel() == m && ws.numel() == n, "gpuk: linear takes a scale per token and per channel");
+        x_scale = xs.data_ptr<float>(), w_scale = ws.data_ptr<float>();
+    }
+};
+
+// swiglu(x, x_scale, w [2 f, k], w_scale) -> [m, f]: silu of the first f channels times the others
+PyObject *swiglu(PyObject *, PyObject *const *args, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    expect_args(n, 4, "swiglu");
+    const Operands o(args);
+    Tensor out;
+    {
+        NoGil unlocked;
+        c10::cuda::CUDAGuard guard(o.x.device());
+        out = empty_like_on(o.x, {o.m, o.n / 2}, at::kBFloat16);
+        check(gpuk_swiglu_skinny(o.x.data_ptr(), o.x_scale, o.w.data_ptr(), o.w_scale, out.data_ptr(), o.m, o.n, o.k, 0, stream_of(o.x)), "swiglu");
+    }
+    return THPVariable_Wrap(std::move(out));
+    END_HANDLE_TH_ERRORS
+}
+
+// qkv_rope(x, x_scale, w, w_scale, cos, sin, pos [t], k_cache, v_cache, heads) -> q [m, heads * 128]; keys and values go to the caches
+PyObject *qkv_rope(PyObject *, PyObject *const *args, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    expect_args(n, 10, "qkv_rope");
+    const Operands o(args);
+    const int dev = o.x.get_device();
+    const Tensor &cos = cuda_arg(args[4], "cos", at::kFloat, dev), &sin = cuda_arg(args[5], "sin", at::kFloat, dev), &pos = cuda_arg(args[6], "positions", at::kLong, dev);
+    const Tensor &kc = cuda_arg(args[7], "k_cache", at::kBFloat16, dev), &vc = cuda_arg(args[8], "v_cache", at::kBFloat16, dev);
+    const int64_t heads = int_arg(args[9]), t = pos.numel();
+    TORCH_CHECK(kc.dim() == 4 && vc.sizes() == kc.sizes() && cos.dim() == 2 && sin.sizes() == cos.sizes() && kc.size(3) == 128 && cos.size(1) == 64 && heads > 0 &&
+                    o.n == (heads + 2 * kc.size(1)) * 128 && t > 0 && o.m % t == 0 && o.m / t <= kc.size(0), "gpuk: qkv_rope shapes do not match");
+    Tensor q;
+    {
+        NoGil unlocked;
+        c10::cuda::CUDAGuard guard(o.x.device());
+        q = empty_like_on(o.x, {o.m, heads * 128}, at::kBFloat16);
+        check(gpuk_qkv_rope_skinny(o.x.data_ptr(), o.x_scale, o.w.data_ptr(), o.w_scale, cos.data_ptr<float>(), sin.data_ptr<float>(), pos.data_ptr<int64_t>(), q.data_ptr(),
+                                   kc.data_ptr(), vc.data_ptr(), static_cast<int>(o.m / t), static_cast<int>(t), static_cast<int>(heads), static_cast<int>(kc.size(1)), o.k,
+                                   static_cast<int>(cos.size(0)), static_cast<int>(kc.size(2)), 0, stream_of(o.x)), "qkv_rope");
+    }
+    return THPVariable_Wrap(std::move(q));
+    END_HANDLE_TH_ERRORS
+}
+
 // decode_attention(q [batch, heads, 128], k_cache, v_cache [>= batch, kv_heads, max_seq, 128], len) -> [batch, heads * 128]
 PyObject *decode_attention(PyObject *, PyObject *const *args, Py_ssize_t n) {
     HANDLE_TH_ERRORS
@@ -262,6 +318,8 @@ constexpr PyCFunction fast() { return reinterpret_cast<PyCFunction>(reinterpret_
 
 PyMethodDef methods[] = {
     {"rope_append", fast<rope_append>(), METH_FASTCALL, nullptr},
+    {"swiglu", fast<swiglu>(), METH_FASTCALL, nullptr},
+    {"qkv_rope", fast<qkv_rope>(), METH_FASTCALL, nullptr},
     {"linear", fast<linear>(), METH_FASTCALL, nullptr},
     {"decode_attention", fast<decode_attention>(), METH_FASTCALL, nullptr},
     {"prefill_attention", fast<prefill_attention>(), METH_FASTCALL, nullptr},

@@ -22,6 +22,10 @@
 //     pair of rows in the second half of a band of 16 has changed places; the epilogue undoes that.  Either way
 //     an instruction multiplies the same 32 bytes of k, so both layouts give the same bits.
 //
+// The elementwise step that follows a projection in a decoder layer can be its epilogue: a tile is then 64 channels of w1 and the same 64 of w3, or
+// one head of q|k|v.  That saves two launches of 2.3 us a layer and the round trip of their inputs: decode step of four layers, 32 sequences, 1079 -> 1060
+// us; of two small layers, 4 sequences, 121 -> 112 us.
+//
 // Measured, 32 tokens, FP8: 57344 x 8192 75 us (6.3 TB/s; the warp-level kernel 136, the library GEMM 89), 10240 x 8192 16.6 (39, 20.7), 7168 x 8192 13.2
 // (21.7, 17.3), 4096 x 8192 10.1 (13.5, 15.8).  bf16: 8192 x 8192 23.8 us (library 25.3), 8192 x 28672 71.8 (71.2); 4 tokens: 3072 x 2048
 // 5.9 (7.5), 2048 x 4096 7.0 (12.4), 8192 x 2048 9.0 (8.0).  Below 30 MB what is left is a fixed 3 us of start and end.
@@ -33,6 +37,7 @@
 #include <cstdint>
 
 #include "../../include/gpuk_b200.h"
+#include "decoder_math.cuh"
 #include "launch.cuh"
 #include "linear.cuh"
 #include "tensor_core.cuh"
@@ -62,6 +67,7 @@ struct StreamParams {
     int stages;                          // depth of the ring
     int ks;                              // CTAs per cluster = parts the steps are split into (planned; checked in the kernel)
     int vec;                             // 1: out and w_scale are aligned for four channels at a time
+    RopeCall rope;
     int *status;                         // set to 1 when a launch did not carry the planned cluster or a wait gave up
 };
 
@@ -77,7 +83,13 @@ __device__ __forceinline__ float4 ld_cluster_f32x4(uint32_t local, int cta) {
     return v;
 }
 
-template <int W, int N>
+__device__ __forceinline__ uint32_t pack2(float lo, float hi) {
+    const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
+    return *reinterpret_cast<const uint32_t *>(&v);
+}
+__device__ __forceinline__ float rounded(float v) { return __bfloat162float(__float2bfloat16_rn(v)); }
+
+template <int W, int N, int EPI>
 __global__ void __launch_bounds__(kThreads, 2) stream_linear_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap xmap,
                                                                     const __grid_constant__ StreamParams p) {
     constexpr int kTmemCols = kAcc * N;
@@ -113,7 +125,10 @@ __global__ void __launch_bounds__(kThreads, 2) stream_linear_kernel(const __grid
             const uint32_t w = ring + s * stage_bytes<N>();
             mbar_expect_bytes(&full[s], stage_bytes<N>());
             if (W == kFp8Blocked) tma_load_4d(w, &wmap, 0, 0, tile * (kTileRows / 16), (begin + i) * 2, &full[s], once);
-            else tma_load_2d(w, &wmap, (begin + i) * (W == kBf16Rows ? kStep / 2 : kStep), tile * kTileRows, &full[s], once);
+            else if (EPI == kSwiGlu) {      // 64 channels of either half
+                for (int h = 0; h < 2; ++h)
+                    tma_load_2d(w + h * (kWBytes / 2), &wmap, (begin + i) * (W == kBf16Rows ? kStep / 2 : kStep), h * (p.n / 2) + tile * (kTileRows / 2), &full[s], once);
+            } else tma_load_2d(w, &wmap, (begin + i) * (W == kBf16Rows ? kStep / 2 : kStep), tile * kTileRows, &full[s], once);
         };
         auto load_x = [&](int i, int s) {
             tma_load_2d(ring + s * stage_bytes<N>() + kWBytes, &xmap, (begin + i) * (W == kBf16Rows ? kStep / 2 : kStep), 0, &full[s], keep);
@@ -122,7 +137,10 @@ __global__ void __launch_bounds__(kThreads, 2) stream_linear_kernel(const __grid
         const int fill = min(p.stages, nsteps);
         for (int i = 0; i < fill; ++i) {
             if (W == kFp8Blocked) tma_prefetch_4d(&wmap, 0, 0, tile * (kTileRows / 16), (begin + i) * 2);
-            else tma_prefetch_2d(&wmap, (begin + i) * (W == kBf16Rows ? kStep / 2 : kStep), tile * kTileRows);
+            else if (EPI == kSwiGlu) {
+                for (int h = 0; h < 2; ++h)
+                    tma_prefetch_2d(&wmap, (begin + i) * (W == kBf16Rows ? kStep / 2 : kStep), h * (p.n / 2) + tile * (kTileRows / 2));
+            } else tma_prefetch_2d(&wmap, (begin + i) * (W == kBf16Rows ? kStep / 2 : kStep), tile * kTileRows);
         }
         grid_dependency_sync();
         for (int i = 0; i < fill; ++i) load_w(i, i), load_x(i, i);
@@ -194,9 +212,7 @@ __global__ void __launch_bounds__(kThreads, 2) stream_linear_kernel(const __grid
         tmem_free<kTmemCols>(acc);
     }
     // the tile's outputs, four channels at a time, dealt out over the cluster; the sum over the cluster in CTA order
-    constexpr int quads = kTileRows / 4;
-    for (int e = part * kThreads + tid; e < quads * p.m; e += ks * kThreads) {
-        const int ch = (e % quads) * 4, tok = e / quads;
+    auto sum = [&](int tok, int ch, int n) {      // channels ch.. of the tile, n.. of the weights
         const uint32_t at = partial + (tok * kPitch + ch) * 4;
         float4 v = ld_cluster_f32x4(at, 0);
 #pragma unroll 8
@@ -204,35 +220,79 @@ __global__ void __launch_bounds__(kThreads, 2) stream_linear_kernel(const __grid
             const float4 o = ld_cluster_f32x4(at, c);
             v.x += o.x, v.y += o.y, v.z += o.z, v.w += o.w;
         }
-        const int n = tile * kTileRows + ch;
-        bf16 *out = p.out + static_cast<size_t>(tok) * p.n + n;
         if (W != kBf16Rows) {
             const float xs = p.x_scale[tok];
             const float *ws = p.w_scale + n;
             const float4 f = p.vec ? *reinterpret_cast<const float4 *>(ws) : make_float4(ws[0], ws[1], ws[2], ws[3]);
             v.x = v.x * xs * f.x, v.y = v.y * xs * f.y, v.z = v.z * xs * f.z, v.w = v.w * xs * f.w;
         }
-        const __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
-        if (p.vec) *reinterpret_cast<uint2 *>(out) = make_uint2(*reinterpret_cast<const uint32_t *>(&lo), *reinterpret_cast<const uint32_t *>(&hi));
-        else out[0] = lo.x, out[1] = lo.y, out[2] = hi.x, out[3] = hi.y;
+        return v;
+    };
+    constexpr int quads = (EPI == kSwiGlu ? kTileRows / 2 : kTileRows) / 4;
+    for (int e = part * kThreads + tid; e < quads * p.m; e += ks * kThreads) {
+        const int ch = (e % quads) * 4, tok = e / quads, n = tile * quads * 4 + ch;
+        const float4 v = sum(tok, ch, n);
+        if constexpr (EPI == kPlain) {
+            bf16 *out = p.out + static_cast<size_t>(tok) * p.n + n;
+            const uint2 o = make_uint2(pack2(v.x, v.y), pack2(v.z, v.w));
+            if (p.vec) *reinterpret_cast<uint2 *>(out) = o;
+            else
+                for (int i = 0; i < 4; ++i) out[i] = reinterpret_cast<const bf16 *>(&o)[i];
+        } else if constexpr (EPI == kSwiGlu) {
+            const float4 u = sum(tok, kTileRows / 2 + ch, p.n / 2 + n);
+            const float g[4] = {rounded(silu(rounded(v.x))), rounded(silu(rounded(v.y))), rounded(silu(rounded(v.z))), rounded(silu(rounded(v.w)))};
+            *reinterpret_cast<uint2 *>(p.out + static_cast<size_t>(tok) * (p.n / 2) + n) =
+                make_uint2(pack2(g[0] * rounded(u.x), g[1] * rounded(u.y)), pack2(g[2] * rounded(u.z), g[3] * rounded(u.w)));
+        } else {      // a tile is a head: rope_append_kernel's arithmetic
+            const RopeCall &r = p.rope;
+            const int b = tok / r.t, kv = tile - r.heads;
+            const int64_t raw = r.pos[tok % r.t];
+            const int64_t at = raw < 0 ? raw + r.max_seq : raw, angle = raw < 0 ? raw + r.table_rows : raw;
+            const bool in_cache = at >= 0 && at < r.max_seq;
+            if (kv >= r.kv_heads) {
+                if (in_cache)
+                    *reinterpret_cast<uint2 *>(static_cast<bf16 *>(r.v_cache) + ((static_cast<int64_t>(b) * r.kv_heads + kv - r.kv_heads) * r.max_seq + at) * kTileRows + ch) =
+                        make_uint2(pack2(v.x, v.y), pack2(v.z, v.w));
+                continue;
+            }
+            if ((kv >= 0 && !in_cache) || angle < 0 || angle >= r.table_rows) continue;
+            const int64_t row = angle * (kTileRows / 2) + ch / 2;
+            const float2 c = *reinterpret_cast<const float2 *>(r.cos + row), s = *reinterpret_cast<const float2 *>(r.sin + row);
+            float lo[2], hi[2];
+            rotate(rounded(v.x), rounded(v.y), c.x, s.x, lo[0], hi[0]);
+            rotate(rounded(v.z), rounded(v.w), c.y, s.y, lo[1], hi[1]);
+            bf16 *dst = kv < 0 ? p.out + (static_cast<size_t>(tok) * r.heads + tile) * kTileRows
+                               : static_cast<bf16 *>(r.k_cache) + ((static_cast<int64_t>(b) * r.kv_heads + kv) * r.max_seq + at) * kTileRows;
+            *reinterpret_cast<uint32_t *>(dst + ch / 2) = pack2(lo[0], lo[1]);
+            *reinterpret_cast<uint32_t *>(dst + kTileRows / 2 + ch / 2) = pack2(hi[0], hi[1]);
+        }
     }
     if (ks > 1) cluster_barrier();      // nobody leaves while its partial tile may still be read
 }
 
 
-template <int W>
-const void *kernel_of(int columns) {
-    return columns == 16 ? reinterpret_cast<const void *>(&stream_linear_kernel<W, 16>) : reinterpret_cast<const void *>(&stream_linear_kernel<W, 32>);
+template <int W, int EPI>
+const void *kernel_for(int columns) {
+    return columns == 16 ? reinterpret_cast<const void *>(&stream_linear_kernel<W, 16, EPI>) : reinterpret_cast<const void *>(&stream_linear_kernel<W, 32, EPI>);
+}
+// blocked weights only with the plain epilogue
+const void *kernel_of(int w, int epilogue, int columns) {
+    if (w == kFp8Blocked) return kernel_for<kFp8Blocked, kPlain>(columns);
+    if (epilogue == kSwiGlu) return w == kFp8Rows ? kernel_for<kFp8Rows, kSwiGlu>(columns) : kernel_for<kBf16Rows, kSwiGlu>(columns);
+    if (epilogue == kRopeAppend) return w == kFp8Rows ? kernel_for<kFp8Rows, kRopeAppend>(columns) : kernel_for<kBf16Rows, kRopeAppend>(columns);
+    return w == kFp8Rows ? kernel_for<kFp8Rows, kPlain>(columns) : kernel_for<kBf16Rows, kPlain>(columns);
 }
 
 }  // namespace
 
 cudaError_t stream_linear_setup() {
     for (int columns = 16; columns <= kMaxTokens; columns += 16)
-        for (const void *fn : {kernel_of<kFp8Blocked>(columns), kernel_of<kFp8Rows>(columns), kernel_of<kBf16Rows>(columns)}) {
-            const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes(columns, kMaxSmem / (kWBytes + columns * kStep)));
-            if (e != cudaSuccess) return e;
-        }
+        for (int w : {kFp8Blocked, kFp8Rows, kBf16Rows})
+            for (int epilogue : {kPlain, kSwiGlu, kRopeAppend}) {
+                const cudaError_t e = cudaFuncSetAttribute(kernel_of(w, epilogue, columns), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                           smem_bytes(columns, kMaxSmem / (kWBytes + columns * kStep)));
+                if (e != cudaSuccess) return e;
+            }
     return cudaSuccess;
 }
 
@@ -248,7 +308,7 @@ int stream_linear(const StreamLinearCall &c, int *status, cudaStream_t stream) {
         rc = encode_map(&wmap, type, c.w, 4, sizes, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
     } else {
         const uint64_t sizes[2] = {k, n}, strides[1] = {row};
-        const uint32_t box[2] = {static_cast<uint32_t>(kStep / es), kTileRows};
+        const uint32_t box[2] = {static_cast<uint32_t>(kStep / es), static_cast<uint32_t>(c.epilogue == kSwiGlu ? kTileRows / 2 : kTileRows)};
         rc = encode_map(&wmap, type, c.w, 2, sizes, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
     }
     if (!rc) {
@@ -272,8 +332,8 @@ int stream_linear(const StreamLinearCall &c, int *status, cudaStream_t stream) {
     stages = std::max(1, std::min({stages, part_steps, kRingMax}));
     const int smem = std::max(smem_bytes(columns, stages), 1024 + columns * kPitch * 4);
     const bool vec = ((reinterpret_cast<uintptr_t>(c.out) & 7u) | (reinterpret_cast<uintptr_t>(c.w_scale) & 15u)) == 0;
-    StreamParams p = {c.x_scale, c.w_scale, static_cast<bf16 *>(c.out), c.m, c.n, steps, stages, ks, vec, status};
-    const void *fn = es == 2 ? kernel_of<kBf16Rows>(columns) : c.blocked ? kernel_of<kFp8Blocked>(columns) : kernel_of<kFp8Rows>(columns);
+    StreamParams p = {c.x_scale, c.w_scale, static_cast<bf16 *>(c.out), c.m, c.n, steps, stages, ks, vec, c.rope, status};
+    const void *fn = kernel_of(es == 2 ? kBf16Rows : c.blocked ? kFp8Blocked : kFp8Rows, c.epilogue, columns);
     void *args[] = {&wmap, &xmap, &p};
     const cudaError_t e = launch_kernel(fn, tiles * ks, kThreads, ks, false, args, stream, smem);
     if (e != cudaSuccess) return set_last_error(GPUK_ERR_CUDA, "linear: launch failed: %s", cudaGetErrorString(e));
@@ -284,18 +344,41 @@ int stream_linear(const StreamLinearCall &c, int *status, cudaStream_t stream) {
 
 using namespace gpuk;
 
+// The checks every entry point makes; `what` names it.
+static int run_skinny(const char *what, StreamLinearCall c, void *stream) {
+    const int es = c.x_scale ? 1 : 2;
+    if (c.m < 0 || c.n <= 0 || c.k <= 0) return set_last_error(GPUK_ERR_INVALID_ARGUMENT, "%s: bad shape %d x %d x %d", what, c.m, c.n, c.k);
+    if (c.m > kMaxTokens) return set_last_error(GPUK_ERR_UNSUPPORTED, "%s: %d tokens; this kernel is built for at most %d", what, c.m, kMaxTokens);
+    if (c.n % kTileRows || static_cast<int64_t>(c.k) * es % 16)
+        return set_last_error(GPUK_ERR_UNSUPPORTED, "%s: n must be a multiple of %d and k of %d (got %d, %d)", what, kTileRows, 16 / es, c.n, c.k);
+    if (c.ks < 0 || c.ks > 8) return set_last_error(GPUK_ERR_INVALID_ARGUMENT, "%s: k_split must be 0 to 8", what);
+    if (c.m == 0) return GPUK_OK;
+    if (!c.x || !c.w || !c.out || !c.x_scale != !c.w_scale) return set_last_error(GPUK_ERR_INVALID_ARGUMENT, "%s: null pointer", what);
+    if ((reinterpret_cast<uintptr_t>(c.x) | reinterpret_cast<uintptr_t>(c.w)) & 15u) return set_last_error(GPUK_ERR_INVALID_ARGUMENT, "%s: operands must be 16-byte aligned", what);
+    int *status = nullptr;
+    const int rc = decode_device(&c.sms, &status);
+    return rc != GPUK_OK ? rc : stream_linear(c, status, static_cast<cudaStream_t>(stream));
+}
+
 extern "C" int gpuk_linear_skinny(const void *x_bf16, const void *w_bf16, void *out_bf16, int m, int n, int k, int k_split, void *stream) {
-    if (m < 0 || n <= 0 || k <= 0) return set_last_error(GPUK_ERR_INVALID_ARGUMENT, "linear: bad shape %d x %d x %d", m, n, k);
-    if (m > kMaxTokens) return set_last_error(GPUK_ERR_UNSUPPORTED, "linear: %d tokens; this kernel is built for at most %d", m, kMaxTokens);
-    if (n % kTileRows || k % 8) return set_last_error(GPUK_ERR_UNSUPPORTED, "linear: n must be a multiple of %d and k of 8 (got %d, %d)", kTileRows, n, k);
-    if (k_split < 0 || k_split > 8) return set_last_error(GPUK_ERR_INVALID_ARGUMENT, "linear: k_split must be 0 to 8");
-    if (m == 0) return GPUK_OK;
-    if (!x_bf16 || !w_bf16 || !out_bf16) return set_last_error(GPUK_ERR_INVALID_ARGUMENT, "linear: null pointer");
-    if ((reinterpret_cast<uintptr_t>(x_bf16) | reinterpret_cast<uintptr_t>(w_bf16)) & 15u)
-        return set_last_error(GPUK_ERR_INVALID_ARGUMENT, "linear: operands must be 16-byte aligned");
-    int sms = 0, *status = nullptr;
-    const int rc = decode_device(&sms, &status);
-    if (rc != GPUK_OK) return rc;
-    const StreamLinearCall c = {x_bf16, nullptr, nullptr, w_bf16, out_bf16, m, n, k, false, k_split, sms};
-    return stream_linear(c, status, static_cast<cudaStream_t>(stream));
+    return run_skinny("linear", {x_bf16, nullptr, nullptr, w_bf16, out_bf16, m, n, k, false, kPlain, {}, k_split, 0}, stream);
+}
+
+extern "C" int gpuk_swiglu_skinny(const void *x, const float *x_scale, const void *w, const float *w_scale, void *out_bf16, int m, int n, int k, int k_split, void *stream) {
+    if ((reinterpret_cast<uintptr_t>(out_bf16) & 7u) | (reinterpret_cast<uintptr_t>(w_scale) & 15u))
+        return set_last_error(GPUK_ERR_INVALID_ARGUMENT, "swiglu: scales must be 16-byte aligned, results 8-byte");
+    return run_skinny("swiglu", {x, x_scale, w_scale, w, out_bf16, m, n, k, false, kSwiGlu, {}, k_split, 0}, stream);
+}
+
+extern "C" int gpuk_qkv_rope_skinny(const void *x, const float *x_scale, const void *w, const float *w_scale, const float *cos, const float *sin, const int64_t *pos,
+                                    void *q_out, void *k_cache, void *v_cache, int batch, int t, int heads, int kv_heads, int k, int table_rows, int max_seq,
+                                    int k_split, void *stream) {
+    if (batch < 0 || t <= 0 || heads <= 0 || kv_heads <= 0 || table_rows <= 0 || max_seq <= 0 || batch > kMaxTokens || t > kMaxTokens || heads > (1 << 20) || kv_heads > (1 << 20))
+        return set_last_error(GPUK_ERR_INVALID_ARGUMENT, "qkv_rope: bad sizes");
+    if (!cos || !sin || !pos || !k_cache || !v_cache) return set_last_error(GPUK_ERR_INVALID_ARGUMENT, "qkv_rope: null pointer");
+    if ((reinterpret_cast<uintptr_t>(q_out) | reinterpret_cast<uintptr_t>(k_cache) | reinterpret_cast<uintptr_t>(v_cache) | reinterpret_cast<uintptr_t>(cos) |
+         reinterpret_cast<uintptr_t>(sin) | reinterpret_cast<uintptr_t>(w_scale)) & 15u)
+        return set_last_error(GPUK_ERR_INVALID_ARGUMENT, "qkv_rope: pointers must be 16-byte aligned");
+    return run_skinny("qkv_rope", {x, x_scale, w_scale, w, q_out, batch * t, (heads + 2 * kv_heads) * kTileRows, k, false, kRopeAppend,
+                                   {cos, sin, pos, k_cache, v_cache, t, heads, kv_heads, table_rows, max_seq}, k_split, 0}, stream);
 }

@@ -82,6 +82,16 @@ class _Linear:
             self.w_scale = (amax / 448.0).t().contiguous()    # [1, out_local] fp32, one scale per output channel
             self.w_q = (weight.float() / amax * 448.0).clamp_(-448, 448).to(torch.float8_e4m3fn)   # [out, in] row-major
 
+    def streamed(self, x: torch.Tensor):
+        """The weight and its scales (None in bf16) as the streaming kernels with a fused epilogue take them, or None where the projection runs
+        elsewhere: on the CPU, in a library, or -- 8 tokens at most on small FP8 weights -- on the warp-level kernel (csrc/fp8_linear.cu)."""
+        w = self.w_q if self.fp8 else self.weight
+        if not (self.own_gemm and x.is_cuda and 0 < x.shape[0] <= 32 and self.weight.dtype == torch.bfloat16 and x.dtype == w.dtype):
+            return None
+        if w.shape[0] % 128 or w.shape[1] % (64 if self.fp8 else 8) or (self.fp8 and x.shape[0] <= 8 and w.numel() <= 12 << 20):
+            return None
+        return w, (self.w_scale if self.fp8 else None)
+
     def __call__(self, x: torch.Tensor, x_scale: Optional[torch.Tensor] = None) -> torch.Tensor:
         # measured on B200: at up to 32 tokens the streaming kernels are the faster ones at the decoder's shapes (fp8_linear.cu, stream_linear.cu)
         own = self.own_gemm and x.is_cuda and 0 < x.shape[0] <= 32 and self.weight.dtype == torch.bfloat16
@@ -243,8 +253,11 @@ class TPDecoder:
             mask = (torch.arange(last, device=self.device)[None, :] <= input_pos[:, None])[None, None]
         normed, scale = self._norm_only(h, self.layers[0]["attention_norm"])
         for li, layer in enumerate(self.layers):
-            qkv = layer["wqkv"](normed, scale)
-            if own:
+            fused = layer["wqkv"].streamed(normed) if own and hd == 128 else None
+            qkv = layer["wqkv"](normed, scale) if fused is None else None
+            if fused is not None:
+                q = _native.qkv_rope(normed, scale, *fused, self.cos, self.sin, pos, layer["k_cache"], layer["v_cache"], self.h_local).view(b, t, self.h_local, hd)
+            elif own:
                 q = _native.rope_append(qkv, self.cos, self.sin, pos, layer["k_cache"], layer["v_cache"], self.h_local).view(b, t, self.h_local, hd)
             else:
                 q, k, v = qkv.view(b, t, self.h_local + 2 * self.kv_local, hd).split([self.h_local, self.kv_local, self.kv_local], dim=2)
@@ -260,11 +273,13 @@ class TPDecoder:
                                                      attn_mask=mask, enable_gqa=True).transpose(1, 2).reshape(b * t, self.h_local * hd)
             partial = layer["wo"](att)
             h, normed, scale = self._reduce_add_norm(partial, h, layer["ffn_norm"])
-            g13 = layer["w13"](normed, scale)
-            if own:
-                act = _native.silu_mul(g13)
+            fused = layer["w13"].streamed(normed) if own else None
+            if fused is not None:
+                act = _native.swiglu(normed, scale, *fused)
+            elif own:
+                act = _native.silu_mul(layer["w13"](normed, scale))
             else:
-                f1, f3 = g13.split(a.ffn_dim // self.world, dim=-1)
+                f1, f3 = layer["w13"](normed, scale).split(a.ffn_dim // self.world, dim=-1)
                 act = F.silu(f1) * f3
             partial = layer["w2"](act)
             nxt = self.layers[li + 1]["attention_norm"] if li + 1 < a.n_layers else self.norm

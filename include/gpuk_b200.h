@@ -357,6 +357,18 @@ int gpuk_fp8_pack_weight(const void *w_fp8, void *packed, int n, int k, void *st
  */
 int gpuk_linear_skinny(const void *x_bf16, const void *w_bf16, void *out_bf16, int m, int n, int k, int k_split, void *stream);
 /*
+ * The same streaming kernel with the elementwise step that follows it in a decoder layer as its epilogue, rounding for rounding what the two calls
+ * give.  FP8 operands with scales, or bf16 with null for both; weights row-major; sizes as above.
+ *
+ * gpuk_swiglu_skinny: out [m, n / 2] = silu(y[:, :n / 2]) * y[:, n / 2:] with y = x . w^T (gpuk_silu_mul).
+ * gpuk_qkv_rope_skinny: x [batch * t, k], w [(heads + 2 * kv_heads) * 128, k]; rotated queries to q_out, rotated keys and values to the caches
+ * (gpuk_rope_append with heads of 128).
+ */
+int gpuk_swiglu_skinny(const void *x, const float *x_scale, const void *w, const float *w_scale, void *out_bf16, int m, int n, int k, int k_split, void *stream);
+int gpuk_qkv_rope_skinny(const void *x, const float *x_scale, const void *w, const float *w_scale, const float *cos, const float *sin, const int64_t *pos,
+                         void *q_out, void *k_cache, void *v_cache, int batch, int t, int heads, int kv_heads, int k, int table_rows, int max_seq,
+                         int k_split, void *stream);
+/*
  * Attention of one new token per sequence over a KV cache: out[b, h] = softmax(q[b, h] . k[b, h / group]^T / sqrt(128)) . v, over
  * positions [0, len) of caches [>= batch, kv_heads, max_seq, 128]; q and out [batch, heads, 128], all bf16, group = heads / kv_heads
  * at most 16.  q and caches 16-byte aligned.  splits = CTAs of a thread-block cluster that share the keys of a (sequence, kv head),
@@ -371,7 +383,7 @@ int gpuk_decode_attention(const void *q, const void *k_cache, const void *v_cach
 int gpuk_prefill_attention(const void *q, const void *k_cache, const void *v_cache, const int64_t *pos, void *out, int batch, int t, int heads, int kv_heads,
                            int head_dim, int len, int max_seq, void *stream);
 /*
- * Synchronises the current device and returns GPUK_ERR_BAD_LAUNCH if a launch of one of the four calls above on it
+ * Synchronises the current device and returns GPUK_ERR_BAD_LAUNCH if a launch of one of the calls above on it
  * found itself in another thread-block cluster than planned (it then wrote nothing) or gave up a wait, else GPUK_OK.
  * Same contract as status 3 of gpuk_ws_status; the reference has no counterpart (impl.h launches no clusters).
  */

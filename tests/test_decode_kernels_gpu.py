@@ -2,7 +2,8 @@
 import pytest
 import torch
 
-from gpuk_b200 import cabi
+import gpuk_b200 as gpuk
+from gpuk_b200 import _native, cabi
 from oracle import fp8_linear_oracle as fo
 
 E4M3 = torch.float8_e4m3fn
@@ -41,7 +42,6 @@ def test_bf16_linear(m, n, k, k_split):
 def test_fp8_linear_around_the_dispatch(m, n, k, packed):
     """The weight size and the token count at which the entry point changes kernels, k with an odd number of 64-byte blocks, and an
     output and channel scales that are aligned for single elements only."""
-    import gpuk_b200 as gpuk
     g = torch.Generator().manual_seed(m + n + k)
     x, w = (torch.randn(m, k, generator=g) * 100).clamp_(-448, 448).to(E4M3), (torch.randn(n, k, generator=g) * 100).clamp_(-448, 448).to(E4M3)
     xs, ws = torch.rand(m, 1, generator=g) * 0.02 + 1e-3, torch.rand(1, n, generator=g) * 0.02 + 1e-3
@@ -56,6 +56,61 @@ def test_fp8_linear_around_the_dispatch(m, n, k, packed):
     again = gpuk.fp8_linear(dx, dxs, dw, shifted, out[1:].view(m, n), packed=packed)
     _status_ok()
     assert torch.equal(again.view(torch.int16), got.view(torch.int16)) and bool(torch.isnan(out[0]))
+
+
+def _fused_operands(m, n, k, fp8, g):
+    """x, its scales, w, its scales, as the native calls take them."""
+    if not fp8:
+        return torch.randn(m, k, generator=g).bfloat16().cuda(), None, (torch.randn(n, k, generator=g) / k ** 0.5).bfloat16().cuda(), None
+    x, w = (torch.randn(m, k, generator=g) * 100).clamp_(-448, 448).to(E4M3), (torch.randn(n, k, generator=g) * 100).clamp_(-448, 448).to(E4M3)
+    return x.cuda(), (torch.rand(m, 1, generator=g) * 0.01 + 1e-3).cuda(), w.cuda(), (torch.rand(1, n, generator=g) * 0.01 + 1e-3).div_(k ** 0.5).cuda()
+
+
+def _streamed(x, xs, w, ws):
+    """The projection alone, by the same kernel: `w` repeated until the entry point leaves the warp-level kernel out."""
+    if xs is None:
+        return _native.linear(x, w)
+    reps = 1 if x.shape[0] > 8 else -(-((12 << 20) + 1) // w.numel())
+    return gpuk.fp8_linear(x, xs, w.repeat(reps, 1), ws.repeat(1, reps))[:, :w.shape[0]].contiguous()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("fp8", [False, True])
+@pytest.mark.parametrize("m,f,k", [(1, 64, 64), (8, 192, 1024), (16, 4096, 2048), (17, 64, 4160), (32, 7168, 1024)])
+def test_swiglu(m, f, k, fp8):
+    """One tile and many, both column counts: the projection in float64, its two halves rounded, silu rounded, product rounded -- each of the four
+    roundings can fall the other way by a step: 2^-7 of the projection's larger half carries through as at most four steps of the result."""
+    ops = _fused_operands(m, 2 * f, k, fp8, torch.Generator().manual_seed(m + f))
+    got = _native.swiglu(*ops)
+    _status_ok()
+    y = ops[0].double() @ ops[2].double().t() * (ops[1].double() * ops[3].double() if fp8 else 1.0)
+    a, b = y.bfloat16().double().split(f, -1)
+    want = (a / (1 + torch.exp(-a))).bfloat16().double() * b
+    assert bool(((got.double() - want).abs() <= 4 * 2.0 ** -8 * want.abs() + 1e-5).all())
+    if m > 8 or not fp8:      # the projection's parts of k may be cut elsewhere: a step apart in a few places, no more
+        same = _native.silu_mul(_streamed(*ops))
+        assert float((got.view(torch.int16) == same.view(torch.int16)).float().mean()) > 0.99
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("fp8", [False, True])
+@pytest.mark.parametrize("batch,t,heads,kv,k,positions", [(1, 1, 8, 1, 64, [0]), (32, 1, 16, 4, 2048, [39]), (3, 5, 4, 2, 1024, [7, 0, 39, 38, 12]), (1, 2, 2, 1, 4160, [-1, -40]),
+                                                         (2, 2, 2, 1, 1024, [40, 3])])
+def test_qkv_rope(batch, t, heads, kv, k, positions, fp8):
+    """Against the projection and gpuk_rope_append: both ends of the cache, positions from its end, one outside that is not written."""
+    g = torch.Generator().manual_seed(batch + heads)
+    ops = _fused_operands(batch * t, (heads + 2 * kv) * 128, k, fp8, g)
+    freqs = torch.outer(torch.arange(80).float(), 1.0 / (10000.0 ** (torch.arange(0, 128, 2).float() / 128)))
+    cos, sin, pos = freqs.cos().cuda(), freqs.sin().cuda(), torch.tensor(positions).cuda()
+    caches = [torch.randn(batch + 1, kv, 40, 128, generator=g).bfloat16().cuda() for _ in range(2)]
+    mine = [c.clone() for c in caches]
+    q = _native.qkv_rope(*ops, cos, sin, pos, *mine, heads)
+    _status_ok()
+    want = _native.rope_append(_streamed(*ops), cos, sin, pos, *caches, heads)
+    for a, b in zip((q, *mine), (want, *caches)):
+        # sums in another order of k: a projection may fall one bf16 step aside, and a rotated pair with it by the larger of the two
+        scale = float(b.float().abs().max())
+        assert float((a.float() - b.float()).abs().max()) <= 2.0 ** -7 * scale and float((a == b).float().mean()) > 0.99
 
 
 @pytest.mark.gpu
@@ -119,3 +174,10 @@ def test_refused_shapes():
     assert b(16, 16, 16, 16, 16, 1, 4, 8, 2, 64, 4, 8, None) == cabi.ERR_UNSUPPORTED and b(16, 16, 16, 16, 16, 1, 4, 8, 3, 128, 4, 8, None) == cabi.ERR_UNSUPPORTED
     assert b(16, 16, 16, 16, 16, 1, 4, 8, 2, 128, 9, 8, None) == cabi.ERR_INVALID_ARGUMENT and b(16, 16, 8, 16, 16, 1, 4, 8, 2, 128, 4, 8, None) == cabi.ERR_INVALID_ARGUMENT
     assert b(16, 16, 16, 16, 16, 1, 0, 8, 2, 128, 4, 8, None) == cabi.OK
+    c = cabi.lib.gpuk_swiglu_skinny
+    assert c(16, 16, 16, None, 16, 8, 128, 64, 0, None) == cabi.ERR_INVALID_ARGUMENT and c(16, None, 16, None, 12, 8, 128, 64, 0, None) == cabi.ERR_INVALID_ARGUMENT
+    assert c(16, None, 16, None, 16, 33, 128, 64, 0, None) == cabi.ERR_UNSUPPORTED and c(16, None, 16, None, 16, 8, 64, 64, 0, None) == cabi.ERR_UNSUPPORTED
+    d = cabi.lib.gpuk_qkv_rope_skinny
+    assert d(16, None, 16, None, 16, 16, 16, 16, 16, 16, 33, 1, 8, 1, 64, 80, 40, 0, None) == cabi.ERR_INVALID_ARGUMENT
+    assert d(16, None, 16, None, 16, 16, 16, 16, 16, 16, 17, 2, 8, 1, 64, 80, 40, 0, None) == cabi.ERR_UNSUPPORTED
+    assert d(16, None, 16, None, 16, 16, None, 16, 16, 16, 1, 1, 8, 1, 64, 80, 40, 0, None) == cabi.ERR_INVALID_ARGUMENT
