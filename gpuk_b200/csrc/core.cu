@@ -132,12 +132,9 @@ constexpr uint64_t kDefaultTimeoutNs = 2000000000ull;
 constexpr size_t kFlagBytes = 4096;             // the allocation behind the "barrier handle"
 constexpr int64_t kTailBytes = 256;             // never written by an exchange
 constexpr int kPlainRowVecs = 1024;             // the plain all-reduce views its input as 16 KiB rows
-// The one-GPU kernel for many rows (persistent CTAs, rows staged through shared memory).  Measured on
-// B200 at hidden 8192, fraction of the HBM copy peak, one row per CTA / staged with 512 threads and two
-// stages: 1024 rows 0.70 / 0.63, 2048 rows 0.84 / 0.82, 4096 rows 0.89 / 0.93, 16384 x 7168 0.97 / 0.98.
+// The one-GPU kernel for many rows (persistent CTAs, rows staged through shared memory); choose_k1 says when it runs.
 constexpr int kDefaultK1Threads = 512;          // preferred CTA size of that kernel
 constexpr int kDefaultK1Stages = 2;             // its shared-memory stages (0: never use it)
-constexpr int64_t kK1StagedMinRows(int sms) { return 20ll * sms; }   // ... used from this many rows
 
 // process-wide tuning of the one-GPU kernel (gpuk_set_tuning); negative / zero: built-in choice
 struct Tuning {
@@ -964,6 +961,28 @@ int gpuk_ws_selftest_wait(gpuk_ws *ws, void *stream) {
     return GPUK_OK;
 }
 
+// Which of the one-GPU kernels takes a call.  Measured in us, calls back to back, bf16 with dynamic scales:
+//   a warp per row: rows of at most 256 vectors, 2 MiB of input and more.  16384 x 2048 37.3 (persistent CTAs 47.7, a CTA per row 52.9), 1500 x 1024 3.4
+//     (4.1, 4.1); 600 x 1024, 1.2 MiB, 2.7 (2.4 with a CTA per row).
+//   persistent CTAs, 2 stages of 512 threads: rows of at least 640 vectors, 32 rows per SM and more: 16384 x 6144 108 (a CTA per row 116), 6000 x 8192 56.1 (57.3);
+//     fewer rows 3500 x 6144 25.8 (23.1), shorter ones 6000 x 4096 38.2 (30.6).  At 1024 vectors a CTA per row comes ahead again from 48
+//     rows per SM: 16384 x 8192 151 (160).
+//   ... 4 stages of 256 threads: rows of up to 640 vectors from 64 rows per SM: 16384 x 3072 61 (a CTA per row 66.6), 16384 x 5120 94 (106).
+//   a CTA per row otherwise.
+struct K1Choice {
+    bool warp;
+    int stages;      // 0: not the persistent kernel
+    int threads;     // its preferred CTA size
+};
+static K1Choice choose_k1(int64_t rows, int row_vecs, int sms) {
+    const int threads = g_tuning.k1_threads > 0 ? g_tuning.k1_threads : kDefaultK1Threads, stages = g_tuning.k1_stages < 0 ? kDefaultK1Stages : g_tuning.k1_stages;
+    if (g_tuning.k1_staged_min_rows >= 0) return {false, rows >= g_tuning.k1_staged_min_rows ? stages : 0, threads};      // as asked for
+    if (row_vecs <= 256) return {rows * row_vecs >= 131072, 0, threads};
+    if (row_vecs <= 640 && rows >= 64ll * sms) return {false, g_tuning.k1_stages < 0 ? 4 : stages, g_tuning.k1_threads > 0 ? threads : 256};
+    const bool full_tile = row_vecs > 896 && row_vecs <= 1024;
+    return {false, row_vecs >= 640 && rows >= 32ll * sms && !(full_tile && rows >= 48ll * sms) ? stages : 0, threads};
+}
+
 int gpuk_residual_rms_quant(const void *in, const void *residual_in, const void *rms_gamma,
                             void *residual_out, void *norm_out, float *scale_out, int64_t numel,
                             int hidden, int dtype, float eps, int quant_type, void *stream) {
@@ -984,23 +1003,20 @@ int gpuk_residual_rms_quant(const void *in, const void *residual_in, const void 
     p.in = in;
     p.rows = plan.rows;
     fill_epilogue(a, q, plan.row_vecs, &p.ep);
-    // rows beyond one per resident CTA: persistent CTAs that stage rows through shared memory by bulk
-    // copies, so that the next rows are in flight while the current one is reduced
-    const int stages = g_tuning.k1_stages < 0 ? kDefaultK1Stages : g_tuning.k1_stages;
-    const int64_t staged_min = g_tuning.k1_staged_min_rows < 0 ? kK1StagedMinRows(sms) : g_tuning.k1_staged_min_rows;
-    const bool staged = stages >= 1 && plan.rows >= staged_min;
+    const K1Choice c = choose_k1(plan.rows, plan.row_vecs, sms);
     return by_dtype(dtype, [&](auto *t) {
         using T = std::remove_pointer_t<decltype(t)>;
         cudaError_t e = cudaErrorInvalidConfiguration;
-        if (staged) {
+        if (c.warp) {
+            e = launch_norm_quant_warp<T>(p, static_cast<cudaStream_t>(stream));
+        } else if (c.stages) {
             // the persistent variant may use a wider CTA than the one-row-per-CTA kernel: fewer, faster row passes
             int vpt = plan.vpt, threads = plan.threads;
-            const int want = g_tuning.k1_threads > 0 ? g_tuning.k1_threads : kDefaultK1Threads;
-            while (vpt > 1 && threads * 2 <= want) { vpt /= 2; threads = ((plan.row_vecs + vpt - 1) / vpt + 31) / 32 * 32; }
-            e = launch_norm_quant_staged<T>(p, vpt, threads, stages, sms, g_tuning.k1_ctas_per_sm, static_cast<cudaStream_t>(stream));
+            while (vpt > 1 && threads * 2 <= c.threads) { vpt /= 2; threads = ((plan.row_vecs + vpt - 1) / vpt + 31) / 32 * 32; }
+            e = launch_norm_quant_staged<T>(p, vpt, threads, c.stages, sms, g_tuning.k1_ctas_per_sm, static_cast<cudaStream_t>(stream));
         }
         if (e == cudaErrorInvalidConfiguration) {
-            if (staged) cudaGetLastError();
+            if (c.stages) cudaGetLastError();
             e = launch_norm_quant<T>(p, plan.vpt, plan.threads, plan.grid, static_cast<cudaStream_t>(stream));
         }
         if (e != cudaSuccess) return fail(GPUK_ERR_CUDA, "kernel launch failed: %s", cudaGetErrorString(e));

@@ -114,6 +114,34 @@ __global__ void __launch_bounds__(tile_max_threads<VPT>(), tile_min_blocks<VPT>(
     else norm_quant_rows<T, VPT, false>(p, sm);
 }
 
+// The same operation for short rows, a warp per row: no block barriers, so that the rows of a CTA do not wait for one another, and
+// twice VPT loads a thread in flight.
+constexpr int kWarpRowsPerCta = 8;
+template <typename T, int VPT>
+__global__ void __launch_bounds__(kWarpRowsPerCta * 32, VPT == 8 ? 2 : 4) fused_norm_quant_warp_kernel(const __grid_constant__ NormQuantParams p) {
+    __shared__ EpilogueSmem sm;      // untouched: one warp reduces by shuffles alone
+    const int64_t row = static_cast<int64_t>(blockIdx.x) * kWarpRowsPerCta + (threadIdx.x >> 5);
+    const Group warp = {static_cast<int>(threadIdx.x & 31), 32, 0};
+    grid_dependency_sync();
+    if (row >= p.rows) return;
+    const float static_scale = p.ep.q.mode == kQuantStatic ? *p.ep.scale_out : 1.f;
+    const RowSeg seg = whole_row(p.ep.row_vecs);
+    const uint4 *src = reinterpret_cast<const uint4 *>(p.in) + row * p.ep.row_vecs;
+    auto run = [&](auto full) {
+        constexpr bool FULL = decltype(full)::value;
+        uint4 x[VPT], res[VPT];
+#pragma unroll
+        for (int i = 0; i < VPT; ++i) {
+            const int v = warp.tid + i * 32;
+            x[i] = (FULL || v < p.ep.row_vecs) ? ld_stream(src + v) : make_uint4(0, 0, 0, 0);
+        }
+        load_residual<T, VPT, FULL>(p.ep, seg, row, warp, res);
+        row_epilogue<T, VPT, FULL>(p.ep, seg, row, warp, x, res, sm, 0, static_scale);
+    };
+    if (p.full) run(std::true_type());
+    else run(std::false_type());
+}
+
 // The same operation on persistent CTAs: each takes rows blockIdx.x, + gridDim.x, ... and fetches
 // every row (input and residual, contiguous in global memory) into a ring of `stages`
 // shared-memory stages with two bulk copies that one thread issues.  A stage is refilled with

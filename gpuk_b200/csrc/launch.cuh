@@ -34,6 +34,10 @@ cudaError_t resident_ctas(const void *fn, int threads, int cluster, int sm_count
 template <typename T>
 cudaError_t launch_norm_quant(const NormQuantParams &p, int vpt, int threads, int grid, cudaStream_t stream);
 
+// A warp per row, for rows of at most 256 vectors (cudaErrorInvalidConfiguration beyond).
+template <typename T>
+cudaError_t launch_norm_quant_warp(const NormQuantParams &p, cudaStream_t stream);
+
 // Staged variant (rows through shared memory by bulk copies) on persistent CTAs: as many as fit
 // the GPU at once (at most `ctas_per_sm` per SM if that is positive), but no more than it takes
 // to give every CTA the same number of rows.  Returns cudaErrorInvalidConfiguration when the tile

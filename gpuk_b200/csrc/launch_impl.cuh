@@ -89,6 +89,20 @@ cudaError_t launch_norm_quant(const NormQuantParams &p, int vpt, int threads, in
     return launch_kernel(fn, grid, threads, 1, false, args, stream);
 }
 
+template <typename T>
+cudaError_t launch_norm_quant_warp(const NormQuantParams &p0, cudaStream_t stream) {
+    NormQuantParams p = p0;
+    const void *fn = nullptr;
+    int vpt = 0;
+    if (p.ep.row_vecs <= 64) fn = reinterpret_cast<const void *>(&fused_norm_quant_warp_kernel<T, 2>), vpt = 2;
+    else if (p.ep.row_vecs <= 128) fn = reinterpret_cast<const void *>(&fused_norm_quant_warp_kernel<T, 4>), vpt = 4;
+    else if (p.ep.row_vecs <= 256) fn = reinterpret_cast<const void *>(&fused_norm_quant_warp_kernel<T, 8>), vpt = 8;
+    else return cudaErrorInvalidConfiguration;
+    p.full = p.ep.row_vecs == vpt * 32 ? 1 : 0;
+    void *args[] = {&p};
+    return launch_kernel(fn, static_cast<int>((p.rows + kWarpRowsPerCta - 1) / kWarpRowsPerCta), kWarpRowsPerCta * 32, 1, false, args, stream);
+}
+
 template <typename T, int VPT>
 static cudaError_t launch_staged_one(const NormQuantParams &p0, int threads, int stages, int sm_count, int ctas_per_sm, cudaStream_t stream) {
     const void *fn = reinterpret_cast<const void *>(&fused_norm_quant_staged_kernel<T, VPT>);
@@ -178,6 +192,7 @@ cudaError_t ar_resident_ctas(const ArShape &s, bool emulated, int sm_count, int6
 
 #define GPUK_INSTANTIATE_LAUNCHERS(T)                                                                          \
     template cudaError_t launch_norm_quant<T>(const NormQuantParams &, int, int, int, cudaStream_t);           \
+    template cudaError_t launch_norm_quant_warp<T>(const NormQuantParams &, cudaStream_t);                     \
     template cudaError_t launch_norm_quant_staged<T>(const NormQuantParams &, int, int, int, int, int, cudaStream_t); \
     template cudaError_t launch_ar<T>(const ArParams &, const ArShape &, cudaStream_t);                        \
     template cudaError_t launch_ar_emulated<T>(const ArParams *, const ArShape &, cudaStream_t);               \

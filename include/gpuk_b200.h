@@ -278,7 +278,8 @@ int gpuk_ws_set_option(gpuk_ws *ws, const char *name, int64_t value);
  * Process-wide tuning of the one-GPU kernel behind gpuk_residual_rms_quant (which has no
  * workspace to carry options): "k1_stages" (shared-memory stages of the persistent variant: 2, 3,
  * 0 = never use it, -1 = default), "k1_staged_min_rows" (rows from which that variant runs,
- * -1 = default: more rows than the plain kernel has resident CTAs), "k1_ctas_per_sm" (cap on its
+ * -1 = default: by rows and row size, as are the calls that give a warp a row; a value lets only the persistent variant and the
+ * one with a CTA per row run), "k1_ctas_per_sm" (cap on its
  * resident CTAs per SM, 0 = as many as fit).  One more name belongs to gpuk_fp8_linear_skinny:
  * "fp8_frags_per_warp" (16-row fragments a warp of its warp-level kernel multiplies per k step: 1 = eight warps per CTA, 2 = four
  * warps that convert each activation vector once for two fragments, either for all calls of at most 8 tokens; 0 = default: that kernel for
