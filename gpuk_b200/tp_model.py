@@ -240,6 +240,8 @@ class TPDecoder:
         own = self.own_elementwise
         if own:
             from gpuk_b200 import _native
+            if last > a.max_seq_len and t == 1 and cache_len is not None:
+                last = a.max_seq_len      # as a slice of the cache takes it
             if last > a.max_seq_len:
                 raise RuntimeError(f"position {last - 1} is beyond the KV cache ({a.max_seq_len} positions)")
             if input_pos.shape != (t,):
@@ -247,7 +249,7 @@ class TPDecoder:
             pos = input_pos.to(device=self.device, dtype=torch.int64).contiguous()
         else:
             cos, sin = self.cos[input_pos], self.sin[input_pos]
-        own_attention = own and self.own_attention
+        own_attention = own and self.own_attention and last >= 1
         mask = None
         if t > 1 and not own_attention:
             mask = (torch.arange(last, device=self.device)[None, :] <= input_pos[:, None])[None, None]

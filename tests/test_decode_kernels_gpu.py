@@ -181,3 +181,21 @@ def test_refused_shapes():
     assert d(16, None, 16, None, 16, 16, 16, 16, 16, 16, 33, 1, 8, 1, 64, 80, 40, 0, None) == cabi.ERR_INVALID_ARGUMENT
     assert d(16, None, 16, None, 16, 16, 16, 16, 16, 16, 17, 2, 8, 1, 64, 80, 40, 0, None) == cabi.ERR_UNSUPPORTED
     assert d(16, None, 16, None, 16, 16, None, 16, 16, 16, 1, 1, 8, 1, 64, 80, 40, 0, None) == cabi.ERR_INVALID_ARGUMENT
+
+
+@pytest.mark.gpu
+def test_decoder_takes_the_cache_lengths_it_took():
+    """A length beyond the cache means all of it for one token and is refused for several; so is a position beyond it, and a wrong number of positions."""
+    import torch.distributed as dist
+    from gpuk_b200.tp_model import DecoderArgs, TPDecoder
+    if not dist.is_initialized():
+        dist.init_process_group("gloo", store=dist.HashStore(), rank=0, world_size=1)
+    env = gpuk.GPUKDistEnv(group=None, device_id=0)
+    m = TPDecoder(DecoderArgs(dim=512, n_layers=1, n_heads=4, n_kv_heads=2, ffn_dim=1024, vocab_size=256, max_seq_len=64), env, device="cuda:0", fp8=False, max_batch=2)
+    m.fill_kv_cache(64)
+    one, pos = torch.zeros(2, 1, dtype=torch.long, device="cuda"), torch.tensor([63], device="cuda")
+    assert torch.equal(m.forward(one, pos, cache_len=70), m.forward(one, pos, cache_len=64))
+    for tokens, positions, n in ((one, torch.tensor([64], device="cuda"), None), (one.expand(2, 2), torch.tensor([62, 63], device="cuda"), 70),
+                                 (one, torch.tensor([62, 63], device="cuda"), 64)):
+        with pytest.raises(RuntimeError):
+            m.forward(tokens, positions, cache_len=n)
