@@ -3,6 +3,8 @@
 
 #include <cuda_runtime.h>
 
+#include <cstdint>
+
 namespace gpuk {
 
 // f / (1 + exp(-f)): the quotient by reciprocal and one exact-residual correction (bf16 results as with the division on everything tried), the
@@ -21,5 +23,17 @@ __device__ __forceinline__ void rotate(float x1, float x2, float c, float s, flo
     lo = __fsub_rn(__fmul_rn(x1, c), __fmul_rn(x2, s));
     hi = __fadd_rn(__fmul_rn(x2, c), __fmul_rn(x1, s));
 }
+
+// Where a position points in the cache and in the table of angles.  A negative one counts from the end of what it indexes, as in an indexed tensor.
+struct Place {
+    int64_t at, angle;
+    bool valid;      // inside both: otherwise nothing goes to the caches, the queries become NaN, and the status word says so
+};
+__device__ __forceinline__ Place place_of(int64_t position, int max_seq, int table_rows) {
+    Place p = {position < 0 ? position + max_seq : position, position < 0 ? position + table_rows : position, false};
+    p.valid = p.at >= 0 && p.at < max_seq && p.angle >= 0 && p.angle < table_rows;
+    return p;
+}
+constexpr uint32_t kNan2 = 0x7fff7fffu;      // two bf16
 
 }  // namespace gpuk

@@ -19,6 +19,7 @@
 #include "../../include/gpuk_b200.h"
 #include "decoder_math.cuh"
 #include "launch.cuh"
+#include "linear.cuh"
 
 namespace gpuk {
 namespace {
@@ -34,6 +35,7 @@ struct RopeParams {
     bf16 *q_out;             // [batch * t, heads * head_dim]
     bf16 *k_cache, *v_cache; // [batch, kv_heads, max_seq, head_dim]
     int64_t total;           // threads with work
+    int *status;             // of positions
     int t, heads, kv_heads, head_dim, table_rows, max_seq;
 };
 
@@ -50,21 +52,22 @@ __global__ void __launch_bounds__(kThreads) rope_append_kernel(const __grid_cons
     const int b = static_cast<int>(row) / p.t;
     const uint4 *src = reinterpret_cast<const uint4 *>(p.qkv + (row * all + head) * p.head_dim + part * kRopeVec);
     const uint4 in0 = ld_stream(src), in1 = ld_stream(src + 1);
-    const int64_t raw = p.pos[static_cast<int>(row) % p.t];
-    // a negative position counts from the end of what it indexes, as in an indexed tensor
-    const int64_t at = raw < 0 ? raw + p.max_seq : raw, angle = raw < 0 ? raw + p.table_rows : raw;
-    const bool in_cache = at >= 0 && at < p.max_seq;      // the caller checks; nothing is written past the cache in any case
-    const int kv = head - p.heads;
+    const Place place = place_of(p.pos[static_cast<int>(row) % p.t], p.max_seq, p.table_rows);
+    const int kv = head - p.heads, half = p.head_dim / 2, first = part * (kRopeVec / 2);
+    if (!place.valid) {
+        *p.status = 1;
+        if (kv >= 0) return;
+        bf16 *q = p.q_out + (row * p.heads + head) * p.head_dim;
+        *reinterpret_cast<uint4 *>(q + first) = *reinterpret_cast<uint4 *>(q + half + first) = make_uint4(kNan2, kNan2, kNan2, kNan2);
+        return;
+    }
+    const int64_t at = place.at, angle = place.angle;
     if (kv >= p.kv_heads) {      // v: as it is
-        if (!in_cache) return;
         uint4 *dst = reinterpret_cast<uint4 *>(p.v_cache + ((static_cast<int64_t>(b) * p.kv_heads + kv - p.kv_heads) * p.max_seq + at) * p.head_dim + part * kRopeVec);
         dst[0] = in0;
         dst[1] = in1;
         return;
     }
-    if (kv >= 0 && !in_cache) return;
-    if (angle < 0 || angle >= p.table_rows) return;
-    const int half = p.head_dim / 2, first = part * (kRopeVec / 2);
     float c[8], s[8];
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
@@ -126,8 +129,11 @@ extern "C" int gpuk_rope_append(const void *qkv, const float *cos, const float *
     if (!qkv || !cos || !sin || !pos || !q_out || !k_cache || !v_cache) return set_last_error(GPUK_ERR_INVALID_ARGUMENT, "rope_append: null pointer");
     if (!aligned16(qkv) || !aligned16(cos) || !aligned16(sin) || !aligned16(q_out) || !aligned16(k_cache) || !aligned16(v_cache))
         return set_last_error(GPUK_ERR_INVALID_ARGUMENT, "rope_append: pointers must be 16-byte aligned");
+    int sms = 0, *status = nullptr;
+    const int rc = decode_device(&sms, &status);
+    if (rc != GPUK_OK) return rc;
     RopeParams p = {static_cast<const bf16 *>(qkv), cos, sin, pos, static_cast<bf16 *>(q_out), static_cast<bf16 *>(k_cache), static_cast<bf16 *>(v_cache),
-                    static_cast<int64_t>(batch) * t * (heads + 2 * kv_heads) * (head_dim / kRopeVec), t, heads, kv_heads, head_dim, table_rows, max_seq};
+                    static_cast<int64_t>(batch) * t * (heads + 2 * kv_heads) * (head_dim / kRopeVec), status + kStatusPosition, t, heads, kv_heads, head_dim, table_rows, max_seq};
     const int64_t grid = (p.total + kThreads - 1) / kThreads;
     if (grid > 0x7fffffffll || static_cast<int64_t>(batch) * t > 0x7fffffffll) return set_last_error(GPUK_ERR_UNSUPPORTED, "rope_append: too many rows");
     void *args[] = {&p};

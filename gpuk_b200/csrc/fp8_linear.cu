@@ -242,7 +242,7 @@ __global__ void __launch_bounds__(kThreads / FR, 2) fp8_linear_skinny_kernel(con
     cluster_barrier();     // nobody leaves while its partial tile may still be read
 }
 
-__device__ int decode_status;      // zero when the library is loaded: nothing to allocate, also under stream capture
+__device__ int decode_status[kDecodeStatusWords];      // zero when the library is loaded: nothing to allocate, also under stream capture
 
 // [n, k] row-major -> blocked: block (n / 16, k / 64) holds 16 rows x 64 bytes, row r at r * 64; blocks of one
 // 16-row band follow each other along k.  One 16-byte vector per thread.
@@ -342,8 +342,13 @@ extern "C" int gpuk_fp8_linear_status(void) {
     int device = 0;
     if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64) return set_last_error(GPUK_ERR_CUDA, "fp8_linear: no current device");
     if (!g_status_by_device[device]) return GPUK_OK;     // no call on this device yet
-    int v = 0;
-    if (cudaDeviceSynchronize() != cudaSuccess || cudaMemcpy(&v, g_status_by_device[device], sizeof(v), cudaMemcpyDeviceToHost) != cudaSuccess)
-        return set_last_error(GPUK_ERR_CUDA, "fp8_linear: cannot read the status word: %s", cudaGetErrorString(cudaGetLastError()));
-    return v ? set_last_error(GPUK_ERR_BAD_LAUNCH, "fp8_linear: a launch ran without its planned thread-block cluster and wrote nothing") : GPUK_OK;
+    int v[kDecodeStatusWords] = {};
+    cudaError_t e = cudaDeviceSynchronize();
+    if (e == cudaSuccess) e = cudaMemcpy(v, g_status_by_device[device], sizeof(v), cudaMemcpyDeviceToHost);
+    // a position is the caller's mistake and is reported once; a launch that went wrong stays on record
+    if (e == cudaSuccess && v[kStatusPosition]) e = cudaMemset(g_status_by_device[device] + kStatusPosition, 0, sizeof(int));
+    if (e != cudaSuccess) return set_last_error(GPUK_ERR_CUDA, "fp8_linear: cannot read the status words: %s", cudaGetErrorString(e));
+    if (v[0]) return set_last_error(GPUK_ERR_BAD_LAUNCH, "fp8_linear: a launch ran without its planned thread-block cluster and wrote nothing, or gave up a wait");
+    if (v[kStatusPosition]) return set_last_error(GPUK_ERR_INVALID_ARGUMENT, "decoder: a position outside the KV cache or the table of angles; its keys and values were not written, its queries are NaN");
+    return GPUK_OK;
 }

@@ -31,8 +31,10 @@ struct StreamLinearCall {
 cudaError_t stream_linear_setup();          // once per device
 cudaError_t decode_attention_setup();
 cudaError_t prefill_attention_setup();
-// The current device's SMs and the status word that kernels of a decode step set (gpuk_fp8_linear_status); the first call on a device
+// The current device's SMs and the status words that kernels of a decode step set (gpuk_fp8_linear_status): the first where a launch went wrong, the
+// one at kStatusPosition where a position pointed outside the cache or the table of angles.  The first call on a device
 // opts the kernels in to their shared memory, so that no later call has set-up left to do.
+constexpr int kStatusPosition = 1, kDecodeStatusWords = 2;
 int decode_device(int *sms, int **status);
 int stream_linear(const StreamLinearCall &c, int *status, cudaStream_t stream);
 

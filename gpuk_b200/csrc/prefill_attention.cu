@@ -44,6 +44,7 @@ constexpr int kSmemBytes = (kTiles + kSlots) * kBlockBytes + 1024;
 
 struct PrefillAttentionParams {
     const int64_t *pos;       // [t]: keys [0, pos] are seen
+    const bf16 *q;            // [batch, t, heads, 128], as the tensor map has it
     bf16 *out;                // [batch, t, heads, 128]
     int t, heads, kv_heads;
     int len;                  // keys in the cache
@@ -244,8 +245,11 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_attention_kernel(const __
             ok = mbar_wait(&o_done[t], (blocks[t] - 1) & 1) && ok;
             tc_fence_after();
         }
-        const float r = l == 0.f ? 0.f : 1.f / l;      // a query that sees no key: zero
-        uint4 *out = reinterpret_cast<uint4 *>(p.out + ((static_cast<int64_t>(b) * p.t + query) * p.heads + head) * kHeadDim);
+        const float r = l == 0.f ? 0.f : 1.f / l;
+        const int64_t row = ((static_cast<int64_t>(b) * p.t + query) * p.heads + head) * kHeadDim;
+        uint4 *out = reinterpret_cast<uint4 *>(p.out + row);
+        // a query that sees no key: zeros, or NaN where it is one that the rotary embedding marked
+        const uint32_t nothing = limit < 0 && query < p.t && __hisnan(p.q[row]) ? 0x7fff7fffu : 0u;
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
             uint32_t o[32];
@@ -259,7 +263,7 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_attention_kernel(const __
                     uint32_t w[4];
 #pragma unroll
                     for (int e = 0; e < 4; ++e)
-                        w[e] = limit < 0 ? 0u : pack_bf16(__uint_as_float(o[8 * i + 2 * e]) * r, __uint_as_float(o[8 * i + 2 * e + 1]) * r);
+                        w[e] = limit < 0 ? nothing : pack_bf16(__uint_as_float(o[8 * i + 2 * e]) * r, __uint_as_float(o[8 * i + 2 * e + 1]) * r);
                     out[c * 4 + i] = make_uint4(w[0], w[1], w[2], w[3]);
                 }
             }
@@ -309,7 +313,7 @@ extern "C" int gpuk_prefill_attention(const void *q, const void *k_cache, const 
     if (!e) e = encode_map(&kmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, k_cache, 3, kv_sizes, kv_strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
     if (!e) e = encode_map(&vmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, v_cache, 3, kv_sizes, kv_strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
     if (e) return set_last_error(GPUK_ERR_CUDA, "prefill_attention: the driver refused a tensor map (%d)", e);
-    PrefillAttentionParams p = {pos, static_cast<bf16 *>(out), t, heads, kv_heads, len, tiles, batch * heads, 1.4426950408889634f / std::sqrt(static_cast<float>(kHeadDim)), status};
+    PrefillAttentionParams p = {pos, static_cast<const bf16 *>(q), static_cast<bf16 *>(out), t, heads, kv_heads, len, tiles, batch * heads, 1.4426950408889634f / std::sqrt(static_cast<float>(kHeadDim)), status};
     void *args[] = {&qmap, &kmap, &vmap, &p};
     const cudaError_t err = launch_kernel(reinterpret_cast<const void *>(&prefill_attention_kernel), static_cast<int>(ctas), kThreads, 1, false, args,
                                           static_cast<cudaStream_t>(stream), kSmemBytes);

@@ -68,7 +68,7 @@ struct StreamParams {
     int ks;                              // CTAs per cluster = parts the steps are split into (planned; checked in the kernel)
     int vec;                             // 1: out and w_scale are aligned for four channels at a time
     RopeCall rope;
-    int *status;                         // set to 1 when a launch did not carry the planned cluster or a wait gave up
+    int *status;                         // set to 1 when a launch did not carry the planned cluster or a wait gave up; [kStatusPosition]: see place_of
 };
 
 template <int N>
@@ -246,17 +246,19 @@ __global__ void __launch_bounds__(kThreads, 2) stream_linear_kernel(const __grid
         } else {      // a tile is a head: rope_append_kernel's arithmetic
             const RopeCall &r = p.rope;
             const int b = tok / r.t, kv = tile - r.heads;
-            const int64_t raw = r.pos[tok % r.t];
-            const int64_t at = raw < 0 ? raw + r.max_seq : raw, angle = raw < 0 ? raw + r.table_rows : raw;
-            const bool in_cache = at >= 0 && at < r.max_seq;
-            if (kv >= r.kv_heads) {
-                if (in_cache)
-                    *reinterpret_cast<uint2 *>(static_cast<bf16 *>(r.v_cache) + ((static_cast<int64_t>(b) * r.kv_heads + kv - r.kv_heads) * r.max_seq + at) * kTileRows + ch) =
-                        make_uint2(pack2(v.x, v.y), pack2(v.z, v.w));
+            const Place place = place_of(r.pos[tok % r.t], r.max_seq, r.table_rows);
+            const int64_t at = place.at;
+            if (!place.valid) {
+                p.status[kStatusPosition] = 1;
+                if (kv < 0) *reinterpret_cast<uint2 *>(p.out + (static_cast<size_t>(tok) * r.heads + tile) * kTileRows + ch) = make_uint2(kNan2, kNan2);
                 continue;
             }
-            if ((kv >= 0 && !in_cache) || angle < 0 || angle >= r.table_rows) continue;
-            const int64_t row = angle * (kTileRows / 2) + ch / 2;
+            if (kv >= r.kv_heads) {
+                *reinterpret_cast<uint2 *>(static_cast<bf16 *>(r.v_cache) + ((static_cast<int64_t>(b) * r.kv_heads + kv - r.kv_heads) * r.max_seq + at) * kTileRows + ch) =
+                    make_uint2(pack2(v.x, v.y), pack2(v.z, v.w));
+                continue;
+            }
+            const int64_t row = place.angle * (kTileRows / 2) + ch / 2;
             const float2 c = *reinterpret_cast<const float2 *>(r.cos + row), s = *reinterpret_cast<const float2 *>(r.sin + row);
             float lo[2], hi[2];
             rotate(rounded(v.x), rounded(v.y), c.x, s.x, lo[0], hi[0]);

@@ -231,19 +231,26 @@ class TPDecoder:
     @torch.no_grad()
     def forward(self, tokens: torch.Tensor, input_pos: torch.Tensor, cache_len: Optional[int] = None) -> torch.Tensor:
         """tokens [b, t] at positions input_pos [t] (KV cache updated in place) -> logits [b, t, vocab/world]
-        of this rank's vocabulary shard.  cache_len = last position + 1; pass it to avoid a device read."""
+        of this rank's vocabulary shard.  cache_len = last position + 1; pass it to avoid a device read.
+
+        A position outside the cache is refused where it can be seen without a device read of its own (positions on the host, or no
+        cache_len).  Elsewhere this library's kernels write neither its key nor its value, its token's logits are NaN, and
+        ``gpuk_fp8_linear_status`` reports it."""
         a = self.args
         b, t = tokens.shape
         hd = a.head_dim
         h = F.embedding(tokens, self.tok_embeddings).view(b * t, a.dim)
-        last = int(input_pos[-1]) + 1 if cache_len is None else cache_len
         own = self.own_elementwise
+        here = input_pos if not input_pos.is_cuda else input_pos.cpu() if cache_len is None else None
+        last = int(here[-1]) + 1 if cache_len is None else cache_len
         if own:
             from gpuk_b200 import _native
             if last > a.max_seq_len and t == 1 and cache_len is not None:
                 last = a.max_seq_len      # as a slice of the cache takes it
             if last > a.max_seq_len:
                 raise RuntimeError(f"position {last - 1} is beyond the KV cache ({a.max_seq_len} positions)")
+            if here is not None and here.numel() and not -a.max_seq_len <= int(here.min()) <= int(here.max()) < a.max_seq_len:
+                raise RuntimeError(f"a position in [{int(here.min())}, {int(here.max())}] is beyond the KV cache ({a.max_seq_len} positions)")
             if input_pos.shape != (t,):
                 raise RuntimeError(f"{t} tokens a sequence at positions of shape {tuple(input_pos.shape)}")
             pos = input_pos.to(device=self.device, dtype=torch.int64).contiguous()
@@ -253,6 +260,8 @@ class TPDecoder:
         mask = None
         if t > 1 and not own_attention:
             mask = (torch.arange(last, device=self.device)[None, :] <= input_pos[:, None])[None, None]
+            if own:
+                mask = mask | (input_pos < -a.max_seq_len)[:, None]      # a token that the rotary embedding marked attends, and stays marked
         normed, scale = self._norm_only(h, self.layers[0]["attention_norm"])
         for li, layer in enumerate(self.layers):
             fused = layer["wqkv"].streamed(normed) if own and hd == 128 else None

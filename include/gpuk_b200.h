@@ -379,13 +379,14 @@ int gpuk_decode_attention(const void *q, const void *k_cache, const void *v_cach
                           int len, int max_seq, int splits, void *stream);
 /*
  * The same for t new tokens per sequence at positions pos [t] (int64, on the device): token i sees the cached positions [0, min(pos[i], len - 1)];
- * one that sees none gets zeros.  q and out [batch, t, heads, 128]; any number of query heads per kv head.  Pointers 16-byte aligned.
+ * one that sees none gets zeros, or NaN where its query starts with NaN.  q and out [batch, t, heads, 128]; any number of query heads per kv head.  Pointers 16-byte aligned.
  */
 int gpuk_prefill_attention(const void *q, const void *k_cache, const void *v_cache, const int64_t *pos, void *out, int batch, int t, int heads, int kv_heads,
                            int head_dim, int len, int max_seq, void *stream);
 /*
  * Synchronises the current device and returns GPUK_ERR_BAD_LAUNCH if a launch of one of the calls above on it
- * found itself in another thread-block cluster than planned (it then wrote nothing) or gave up a wait, else GPUK_OK.
+ * found itself in another thread-block cluster than planned (it then wrote nothing) or gave up a wait; GPUK_ERR_INVALID_ARGUMENT, once, if a position
+ * given to gpuk_qkv_rope_skinny or gpuk_rope_append lay outside the cache or the table of angles; else GPUK_OK.
  * Same contract as status 3 of gpuk_ws_status; the reference has no counterpart (impl.h launches no clusters).
  */
 int gpuk_fp8_linear_status(void);
@@ -397,8 +398,9 @@ int gpuk_fp8_linear_status(void);
  * gpuk_rope_append: qkv [batch * t, (heads + 2 * kv_heads) * head_dim] as the q|k|v projection wrote it; pos [t] int64
  * positions on the device; cos, sin [table_rows, head_dim / 2] fp32.  Interleaved pairs in, halves out.  Writes the rotated
  * queries to q_out [batch * t, heads * head_dim] and the rotated keys and the values to positions pos of the caches
- * [batch, kv_heads, max_seq, head_dim].  A negative position counts from the end; one outside a table or cache is not
- * written.  head_dim a multiple of 16, pointers 16-byte aligned.
+ * [batch, kv_heads, max_seq, head_dim].  A negative position counts from the end.  For one outside the table or the cache nothing is
+ * written to the caches, the token's queries are NaN, and gpuk_fp8_linear_status reports it.  head_dim a multiple of 16, pointers
+ * 16-byte aligned.
  *
  * gpuk_silu_mul: out [rows, f] = silu(in[:, :f]) * in[:, f:], in [rows, 2 * f]; f a multiple of 8.
  */

@@ -95,9 +95,9 @@ def test_swiglu(m, f, k, fp8):
 @pytest.mark.gpu
 @pytest.mark.parametrize("fp8", [False, True])
 @pytest.mark.parametrize("batch,t,heads,kv,k,positions", [(1, 1, 8, 1, 64, [0]), (32, 1, 16, 4, 2048, [39]), (3, 5, 4, 2, 1024, [7, 0, 39, 38, 12]), (1, 2, 2, 1, 4160, [-1, -40]),
-                                                         (2, 2, 2, 1, 1024, [40, 3])])
+                                                         (2, 2, 2, 1, 1024, [38, 3])])
 def test_qkv_rope(batch, t, heads, kv, k, positions, fp8):
-    """Against the projection and gpuk_rope_append: both ends of the cache, positions from its end, one outside that is not written."""
+    """Against the projection and gpuk_rope_append: both ends of the cache, positions from its end."""
     g = torch.Generator().manual_seed(batch + heads)
     ops = _fused_operands(batch * t, (heads + 2 * kv) * 128, k, fp8, g)
     freqs = torch.outer(torch.arange(80).float(), 1.0 / (10000.0 ** (torch.arange(0, 128, 2).float() / 128)))
@@ -111,6 +111,45 @@ def test_qkv_rope(batch, t, heads, kv, k, positions, fp8):
         # sums in another order of k: a projection may fall one bf16 step aside, and a rotated pair with it by the larger of the two
         scale = float(b.float().abs().max())
         assert float((a.float() - b.float()).abs().max()) <= 2.0 ** -7 * scale and float((a == b).float().mean()) > 0.99
+
+
+def _position_reported_once():
+    status = cabi.lib.gpuk_fp8_linear_status
+    assert status() == cabi.ERR_INVALID_ARGUMENT and "position" in cabi.last_error() and status() == cabi.OK
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("fp8", [False, True])
+@pytest.mark.parametrize("fused", [False, True])
+@pytest.mark.parametrize("table_rows,bad", [(80, 40), (80, 80), (80, -41), (80, -81), (20, 25), (20, -30), (80, 1 << 32), (80, -(1 << 33))])
+def test_positions_outside_the_cache_or_the_table(table_rows, bad, fused, fp8):
+    """Of such a token nothing goes to the caches, its queries are NaN, written in full, and the status call says so, once.  Tokens beside it are as without it."""
+    batch, heads, kv, k = 3, 4, 2, 1024
+    g = torch.Generator().manual_seed(5)
+    ops = _fused_operands(batch * 3, (heads + 2 * kv) * 128, k, fp8, g)
+    x, xs, w, ws = ops
+    cos, sin = torch.randn(table_rows, 64, generator=g).cuda(), torch.randn(table_rows, 64, generator=g).cuda()
+    start = [torch.randn(batch, kv, 40, 128, generator=g).bfloat16().cuda() for _ in range(2)]
+
+    def call(positions):
+        pos, caches = torch.tensor(positions).cuda(), [c.clone() for c in start]
+        q = torch.full((batch * 3, heads * 128), 7.0, dtype=torch.bfloat16, device="cuda")
+        common = (_ptr(cos), _ptr(sin), _ptr(pos), _ptr(q), *map(_ptr, caches), batch, 3, heads, kv)
+        if fused:
+            cabi.check(cabi.lib.gpuk_qkv_rope_skinny(_ptr(x), _ptr(xs) if fp8 else None, _ptr(w), _ptr(ws) if fp8 else None, *common, k, table_rows, 40, 0, _stream()))
+        else:
+            qkv = _streamed(*ops)
+            cabi.check(cabi.lib.gpuk_rope_append(_ptr(qkv), *common, 128, table_rows, 40, _stream()))
+        return q.view(batch, 3, heads * 128), caches
+    q, caches = call([3, bad, 7])
+    _position_reported_once()
+    assert bool(q[:, 1].isnan().all()) and not bool(q[:, 0::2].isnan().any())
+    want_q, want = call([3, 5, 7])
+    _status_ok()
+    assert torch.equal(q[:, 0::2], want_q[:, 0::2])
+    for c, d, s in zip(caches, want, start):
+        d[:, :, 5] = s[:, :, 5]
+        assert torch.equal(c, d)
 
 
 @pytest.mark.gpu
@@ -199,3 +238,61 @@ def test_decoder_takes_the_cache_lengths_it_took():
                                  (one, torch.tensor([62, 63], device="cuda"), 64)):
         with pytest.raises(RuntimeError):
             m.forward(tokens, positions, cache_len=n)
+
+
+@pytest.fixture
+def decoder():
+    """Makes a decoder on one GPU."""
+    import torch.distributed as dist
+    from gpuk_b200.tp_model import DecoderArgs, TPDecoder
+    if not dist.is_initialized():
+        dist.init_process_group("gloo", store=dist.HashStore(), rank=0, world_size=1)
+    env = gpuk.GPUKDistEnv(group=None, device_id=0)
+
+    def make(head_dim=128, fp8=False, batch=2, dim=512, **more):
+        args = dict(dim=dim, n_layers=2, n_heads=4, n_kv_heads=2, head_dim=head_dim, ffn_dim=1024, vocab_size=256, max_seq_len=64)
+        args.update(more)
+        m = TPDecoder(DecoderArgs(**args), env, device="cuda:0", fp8=fp8, max_batch=batch)
+        m.fill_kv_cache(64)
+        return m
+    return make
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("fp8", [False, True])
+@pytest.mark.parametrize("head_dim", [128, 64])
+def test_decoder_marks_positions_behind_its_cache(decoder, head_dim, fp8):
+    """No device read: NaN logits for the token that has no place, those of the others as without it, and the status.  With one: refused."""
+    m = decoder(head_dim, fp8)
+    keep = [layer[n].clone() for layer in m.layers for n in ("k_cache", "v_cache")]
+
+    def caches():
+        return [layer[n] for layer in m.layers for n in ("k_cache", "v_cache")]
+
+    def restore():
+        for c, k in zip(caches(), keep):
+            c.copy_(k)
+    one, three = torch.zeros(2, 1, dtype=torch.long, device="cuda"), torch.arange(6, device="cuda").view(2, 3)
+    for bad in (64, 70, 1000, -65, -1000):      # the next step of a full cache among them
+        logits = m.forward(one, torch.tensor([bad], device="cuda"), cache_len=65)
+        assert bool(logits.isnan().all())
+        _position_reported_once()
+        assert all(torch.equal(c, k) for c, k in zip(caches(), keep))
+        for places in ([10, bad, 12], [bad, 11, 12]):
+            logits = m.forward(three, torch.tensor(places, device="cuda"), cache_len=13)
+            _position_reported_once()
+            i = places.index(bad)
+            others = [j for j in range(3) if j != i]
+            restore()
+            # the bad token leaves the old key in its place: as if it stood behind what the others see
+            want = m.forward(three, torch.tensor([40 if p == bad else p for p in places], device="cuda"), cache_len=41)
+            restore()
+            assert bool(logits[:, i].isnan().all()) and not bool(logits[:, others].isnan().any())
+            assert float((logits[:, others].float() - want[:, others].float()).norm()) <= 0.03 * float(want[:, others].float().norm())
+        for positions, length in ((torch.tensor([bad]), 64), (torch.tensor([bad]), None), (torch.tensor([bad], device="cuda"), None)):
+            with pytest.raises(RuntimeError, match="beyond the KV cache"):
+                m.forward(one, positions, cache_len=length)
+        with pytest.raises(RuntimeError, match="beyond the KV cache"):
+            m.forward(three, torch.tensor([10, bad, 12], device="cuda"))
+    assert not bool(m.forward(one, torch.tensor([63], device="cuda"), cache_len=70).isnan().any())
+    _status_ok()

@@ -43,6 +43,7 @@ def test_rope_append_writes_nothing_outside_the_cache():
     caches = [torch.zeros(2, 1, 4, 16, device="cuda").bfloat16() for _ in range(2)]
     for at in (4, 19, 20, -5):
         _native.rope_append(qkv, cos, cos, torch.tensor([at], device="cuda"), caches[0], caches[1], 1)
+        assert cabi.lib.gpuk_fp8_linear_status() == cabi.ERR_INVALID_ARGUMENT
     assert not caches[0].any() and not caches[1].any()
 
 
