@@ -456,6 +456,9 @@ __device__ __forceinline__ int cluster_size() {
 __device__ __forceinline__ void cluster_barrier() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+// The two halves of it, for what a CTA can do between them.
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 // Stores `v` at the address `local` names, but in the shared memory of CTA `cta` of this cluster.
 __device__ __forceinline__ void st_cluster_f32(float *local, int cta, float v) {
     const uint32_t a = static_cast<uint32_t>(__cvta_generic_to_shared(local));

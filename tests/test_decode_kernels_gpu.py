@@ -37,6 +37,25 @@ def test_bf16_linear(m, n, k, k_split):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("fp8", [False, True])
+@pytest.mark.parametrize("m,k_split", [(32, 8), (16, 8), (32, 3)])
+def test_more_clusters_than_tensor_memory_holds(m, k_split, fp8):
+    """One step a part, or two: rings so short that shared memory and registers would let more CTAs on an SM than it has columns for."""
+    n, k = 128 * 400, 1024 if fp8 else 512
+    ops = _fused_operands(m, n, k, fp8, torch.Generator().manual_seed(m))
+    x, xs, w, ws = ops
+    want = x.double() @ w.double().t() * (xs.double() * ws.double() if fp8 else 1.0)
+    for _ in range(3):
+        out = torch.full((m, n), float("nan"), dtype=torch.bfloat16, device="cuda")
+        if fp8:
+            gpuk.fp8_linear(x, xs, w, ws, out, k_split=k_split if k_split != 3 else 4)
+        else:
+            cabi.check(cabi.lib.gpuk_linear_skinny(_ptr(x), _ptr(w), _ptr(out), m, n, k, k_split, _stream()))
+        _status_ok()
+        assert fo.within_one_bf16_step(out.cpu(), want.cpu())
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("packed", [False, True])
 @pytest.mark.parametrize("m,n,k", [(8, 1536, 8192), (8, 1664, 8192), (9, 128, 64), (16, 256, 192), (17, 256, 4160), (32, 10240, 1024)])
 def test_fp8_linear_around_the_dispatch(m, n, k, packed):
