@@ -94,9 +94,8 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_attention_kernel(const __
     int limit = -1;      // last key this thread's query sees
     const int query = first + tid;
     if (tid < kSoftmaxThreads && query < p.t) {
-        const int64_t at = p.pos[query];
-        limit = static_cast<int>(at < p.len - 1 ? at : p.len - 1);
-        if (limit < -1) limit = -1;
+        const int64_t at = p.pos[query], end = p.len - 1;
+        limit = static_cast<int>(at < -1 ? -1 : at < end ? at : end);      // bounded before it is cut to 32 bits
         atomicMax(&most[tid / kTile], limit);
         atomicMin(&least[tid / kTile], limit);
     }

@@ -195,19 +195,19 @@ def test_decode_attention(batch, heads, kv_heads, length, max_seq, splits):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("batch,t,heads,kv_heads,past", [(1, 2, 2, 1, 0), (1, 128, 4, 4, 0), (2, 129, 8, 2, 127), (1, 257, 17, 1, 0), (3, 40, 4, 2, 300), (1, 300, 2, 1, 1700)])
-@pytest.mark.parametrize("order", ["rising", "mixed"])
+@pytest.mark.parametrize("order", ["rising", "mixed", "far"])
 def test_prefill_attention(batch, t, heads, kv_heads, past, order):
     """Both tiles of a CTA, ends at, before and behind a tile of queries and a block of keys, a ring that wraps, queries of a next sequence in the tile;
-    positions in order, and in any order with one that sees no key and one beyond the cache.  Bound as for one token."""
+    positions in order, and in any order with one that sees no key and one beyond the cache, just so and far outside.  Bound as for one token."""
     g = torch.Generator().manual_seed(batch + t + heads)
     length, max_seq = past + t, past + t + 5
     q = (torch.randn(batch, t, heads, 128, generator=g) * 2).bfloat16()
     k, v = (torch.randn(batch, kv_heads, max_seq, 128, generator=g).bfloat16() for _ in range(2))
     k[:, :, length:], v[:, :, length:] = float("nan"), float("nan")
     pos = torch.arange(past, length)
-    if order == "mixed":
+    if order != "rising":
         pos = pos[torch.randperm(t, generator=g)]
-        pos[0], pos[-1] = -1, length + 3
+        pos[0], pos[-1] = (-1, length + 3) if order == "mixed" else (-(1 << 32), 1 << 32)      # far: the low halves are positions of the cache
     kk, vv = (x[:, :, :length].repeat_interleave(heads // kv_heads, 1).double() for x in (k, v))
     s = torch.einsum("bthd,bhkd->bhtk", q.double(), kk) / 128 ** 0.5
     p = torch.softmax(s.masked_fill(torch.arange(length) > pos[:, None], float("-inf")), -1).nan_to_num(0.0)
