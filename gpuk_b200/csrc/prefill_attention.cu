@@ -68,13 +68,13 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
 __global__ void __launch_bounds__(kThreads, 1) prefill_attention_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_constant__ CUtensorMap kmap,
                                                                         const __grid_constant__ CUtensorMap vmap, const __grid_constant__ PrefillAttentionParams p) {
     extern __shared__ unsigned char dyn[];
-    __shared__ alignas(8) uint64_t q_full, full[kSlots], empty[kSlots], s_full[kTiles], p_full[kTiles], o_done[kTiles];
+    __shared__ alignas(8) uint64_t q_full, full[kSlots], empty[kSlots], s_full[kTiles], p_full[kTiles], o_done[kTiles], drained;
     __shared__ uint32_t tmem_slot;
     __shared__ int most[kTiles], least[kTiles];      // largest and smallest position of a tile's queries
     const int tid = threadIdx.x, warp = tid >> 5;
     const uint32_t base = (smem_addr(dyn) + 1023u) & ~1023u, ring = base + kTiles * kBlockBytes;
     if (tid == 0) {
-        mbar_init(&q_full, 1);
+        mbar_init(&q_full, 1), mbar_init(&drained, 1);
         for (int s = 0; s < kSlots; ++s) mbar_init(&full[s], 1), mbar_init(&empty[s], 1);
         for (int t = 0; t < kTiles; ++t) {
             mbar_init(&s_full[t], 1), mbar_init(&p_full[t], kTile), mbar_init(&o_done[t], 1);
@@ -134,6 +134,10 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_attention_kernel(const __
         if ((tid & 31) == 0 && rounds > 0) {
             constexpr uint32_t s_desc = mma_desc(1, 1, kTile, kTile), o_desc = mma_desc(1, 1, kTile, kHeadDim, true);
             auto slot = [&](int i) { return ring + (i % kSlots) * kBlockBytes; };
+            // only a slot that the copies wait for: nothing may arrive in shared memory behind the CTA's end
+            auto release = [&](int i) {
+                if (i + kSlots < 2 * rounds) tc_commit(&empty[i % kSlots]);
+            };
             auto wait_slot = [&](int i) { ok = ok && mbar_wait(&full[i % kSlots], (i / kSlots) & 1); };
             auto scores = [&](int t, int j) {      // 16 of the 128 dimensions per instruction
                 const uint32_t q = base + t * kBlockBytes, k = slot(2 * j);
@@ -150,7 +154,7 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_attention_kernel(const __
             if (ok)
                 for (int t = 0; t < kTiles; ++t)
                     if (blocks[t] > 0) scores(t, 0);
-            tc_commit(&empty[0]);
+            release(0);
             for (int j = 0; ok && j < rounds; ++j) {
                 wait_slot(2 * j + 1);
                 if (j + 1 < rounds) wait_slot(2 * j + 2);
@@ -168,8 +172,12 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_attention_kernel(const __
                     tc_commit(&o_done[t]);
                     if (j + 1 < blocks[t]) scores(t, j + 1);
                 }
-                tc_commit(&empty[(2 * j + 1) % kSlots]);
-                if (j + 1 < rounds) tc_commit(&empty[(2 * j + 2) % kSlots]);
+                release(2 * j + 1);
+                release(2 * j + 2);
+            }
+            if (!ok) {      // a wait gave up: the row threads do not wait for what was issued, and the tensor memory is about to be freed
+                tc_commit(&drained);
+                mbar_wait(&drained, 0);
             }
         }
     } else {                                     // a row's thread

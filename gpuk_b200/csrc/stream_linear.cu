@@ -178,7 +178,8 @@ __global__ void __launch_bounds__(kThreads, 2) stream_linear_kernel(const __grid
                     if (W == kBf16Rows) tc_mma_f16(d, a, b, idesc, i >= kAcc || j > 0);
                     else tc_mma_f8(d, a, b, idesc, i >= kAcc || j > 0);
                 }
-                tc_commit(&empty[s]);
+                // only a slot that the copies wait for: `done` stands for the rest, and nothing arrives in shared memory behind it
+                if (i + p.stages < nsteps) tc_commit(&empty[s]);
                 if (++s == p.stages) s = 0, phase ^= 1u;
             }
             tc_commit(&done);      // an arrival at once where there was nothing to multiply
