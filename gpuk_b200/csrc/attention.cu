@@ -84,8 +84,10 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
     asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
     return r;
 }
-// weight of a partial result whose maximum is m, relative to the overall maximum (0 where the part saw no key)
-__device__ __forceinline__ float weight_of(float m, float overall) { return m == -INFINITY ? 0.f : exp2f(m - overall); }
+// A maximum starts below every finite score and stays finite where all scores are -infinity, so that no difference of two is undefined: scores of
+// -infinity weigh nothing beside others, and a part that saw no key, or only such, weighs nothing.
+constexpr float kLowest = -3.4e38f;
+__device__ __forceinline__ float weight_of(float m, float overall) { return exp2f(m - overall); }
 
 __device__ __forceinline__ float ld_cluster(const float *local, int cta) {
     const uint32_t a = static_cast<uint32_t>(__cvta_generic_to_shared(local));
@@ -171,7 +173,7 @@ __global__ void __launch_bounds__(kThreads, STAGES == kStages ? 2 : 1) decode_at
     for (int j = 0; j < kHeadDim / 8; ++j)
 #pragma unroll
         for (int e = 0; e < 4; ++e) o[j][e] = 0.f;
-    float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};      // rows g and g + 8
+    float m[2] = {kLowest, kLowest}, l[2] = {0.f, 0.f};      // rows g and g + 8
 
     for (int i = 0; i < mine; ++i) {
         issue(i + STAGES - 1);
@@ -201,8 +203,8 @@ __global__ void __launch_bounds__(kThreads, STAGES == kStages ? 2 : 1) decode_at
             mx[r] = fmaxf(fmaxf(sc[0][2 * r], sc[0][2 * r + 1]), fmaxf(sc[1][2 * r], sc[1][2 * r + 1]));
             mx[r] = fmaxf(mx[r], __shfl_xor_sync(0xffffffffu, mx[r], 1));
             mx[r] = fmaxf(mx[r], __shfl_xor_sync(0xffffffffu, mx[r], 2));
-            mx[r] = fmaxf(mx[r], m[r]);            // finite: a block has at least one key
-            fade[r] = exp2f(m[r] - mx[r]);         // 0 for the first block
+            mx[r] = fmaxf(mx[r], m[r]);
+            fade[r] = exp2f(m[r] - mx[r]);         // 0 for the first block with a finite score
         }
         if (__any_sync(0xffffffffu, mx[0] != m[0] || mx[1] != m[1])) {
 #pragma unroll
@@ -291,7 +293,7 @@ __global__ void __launch_bounds__(kThreads, STAGES == kStages ? 2 : 1) decode_at
                 pl[s] = ld_cluster(&st.l[kWarps][h], s);
                 ps[s] = ld_cluster4(sum + h * kOutPitch + d, s);
             }
-        float mm = -INFINITY, total = 0.f;
+        float mm = kLowest, total = 0.f;
         float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
         for (int s = 0; s < 8; ++s)

@@ -42,6 +42,8 @@ constexpr int kBlockBytes = 2 * kSpanBytes;
 constexpr int kSlots = 5;
 constexpr int kSmemBytes = (kTiles + kSlots) * kBlockBytes + 1024;
 
+constexpr float kLowest = -3.4e38f;              // a maximum where all scores are -infinity: finite, and any score behind it is larger
+
 struct PrefillAttentionParams {
     const int64_t *pos;       // [t]: keys [0, pos] are seen
     const bf16 *q;            // [batch, t, heads, 128], as the tensor map has it
@@ -211,7 +213,7 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_attention_kernel(const __
             }
             const float top = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * p.scale_log2;
             if (j == 0) {
-                m = top == -INFINITY ? 0.f : top;
+                m = fmaxf(top, kLowest);
             } else {
                 const bool grown = top > m;
                 if (__any_sync(0xffffffffu, grown)) {

@@ -219,6 +219,41 @@ def test_prefill_attention(batch, t, heads, kv_heads, past, order):
     assert bool(((out.cpu().double() - want).abs() <= bound).all())
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("hidden", [1, 40, 200, 290])
+@pytest.mark.parametrize("splits", [0, 1, 3])
+def test_scores_of_minus_infinity(hidden, splits):
+    """The first `hidden` keys score -infinity for some heads: whole blocks, warps and parts of the cluster of them, in front of scores far below zero.  They weigh
+    nothing; the others as in float64.  Bound as in test_decode_attention."""
+    batch, heads, length = 2, 4, 300
+    g = torch.Generator().manual_seed(hidden)
+    q, k, v = (torch.randn(batch, n, m, 128, generator=g).bfloat16() for n, m in ((1, heads), (1, length), (1, length)))
+    q = q.view(batch, heads, 128)
+    q[:, :, 0] = 2.0
+    k[:, :, :, 0] = -1000.0                                    # so far below zero that nothing is left of a weight measured from there
+    k[:, :, :hidden, 0] = float("-inf")
+
+    def reference(limit):
+        s = torch.einsum("bhd,bhkd->bhk", q.double(), k.double().expand(-1, heads, -1, -1)) / 128 ** 0.5
+        s = s.masked_fill(torch.arange(length) >= limit, float("-inf"))
+        p = torch.softmax(s, -1)
+        vv = v.double().expand(-1, heads, -1, -1)
+        return torch.einsum("bhk,bhkd->bhd", p, vv), torch.einsum("bhk,bhkd->bhd", p, vv.abs()) * 2.0 ** -7 + 1e-6
+    dq, dk, dv = q.cuda(), k.cuda(), v.cuda()
+    out = torch.full_like(dq, float("nan"))
+    cabi.check(cabi.lib.gpuk_decode_attention(_ptr(dq), _ptr(dk), _ptr(dv), _ptr(out), batch, heads, 1, 128, length, length, splits, _stream()))
+    want, bound = reference(length)
+    assert bool(((out.cpu().double() - want).abs() <= bound).all())
+    pos = torch.tensor([length - 1, 294], device="cuda")
+    many = torch.full((batch, 2, heads, 128), float("nan"), dtype=torch.bfloat16, device="cuda")
+    dq2 = dq.view(batch, 1, heads, 128).expand(-1, 2, -1, -1).contiguous()
+    cabi.check(cabi.lib.gpuk_prefill_attention(_ptr(dq2), _ptr(dk), _ptr(dv), _ptr(pos), _ptr(many), batch, 2, heads, 1, 128, length, length, _stream()))
+    _status_ok()
+    for i, limit in enumerate((length, 295)):
+        want, bound = reference(limit)
+        assert bool(((many[:, i].cpu().double() - want).abs() <= bound).all())
+
+
 def test_refused_shapes():
     f, a = cabi.lib.gpuk_linear_skinny, cabi.lib.gpuk_decode_attention
     assert f(16, 16, 16, 33, 128, 64, 0, None) == cabi.ERR_UNSUPPORTED and f(16, 16, 16, 8, 100, 64, 0, None) == cabi.ERR_UNSUPPORTED
