@@ -2,7 +2,8 @@
 // `gpuk_b200._native`, part of libgpuk_b200.so.  They take tensors as they are, allocate the results, and launch on the
 // current stream of the tensors' device, with the interpreter lock released as a dispatcher operator or ctypes would.  Why
 // neither of those: a call through them costs several microseconds of host time, which is what bounds a step of a few sequences
-// (fused epilogue, 8 rows: 11.0 -> 6.6 us a call; FP8 linear layer, 8 tokens, 1280 x 8192: 14.8 -> 5.7 us).
+// (fused epilogue, 8 rows: 11.0 -> 6.6 us a call; FP8 linear layer, 8 tokens, 1280 x 8192: 14.8 -> 5.7 us).  All but fp8_linear return None for a
+// call that belongs to the operators: see direct() and add_rms.
 #include <ATen/cuda/CUDAContext.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <ATen/PythonTorchFunctionTLS.h>
@@ -48,10 +49,55 @@ void expect_args(Py_ssize_t n, Py_ssize_t want, const char *what) { TORCH_CHECK(
 void *stream_of(const Tensor &t) { return at::cuda::getCurrentCUDAStream(t.get_device()).stream(); }
 Tensor empty_like_on(const Tensor &t, at::IntArrayRef sizes, at::ScalarType type) { return at::detail::empty_cuda(sizes, type, t.device(), std::nullopt); }
 
+// A tensor whose operators would go straight to the CUDA kernels: of the class Tensor itself, dense and contiguous, no transform or lazy bit on it.
+bool plain_class(PyObject *o) {
+    if (!THPVariable_CheckExact(o)) return false;
+    const Tensor &t = THPVariable_Unpack(o);
+    static const c10::DispatchKeySet other({c10::DispatchKey::Python, c10::DispatchKey::PythonTLSSnapshot, c10::DispatchKey::Functionalize, c10::DispatchKey::FuncTorchBatched,
+                                            c10::DispatchKey::FuncTorchGradWrapper, c10::DispatchKey::Batched, c10::DispatchKey::Negative, c10::DispatchKey::Conjugate,
+                                            c10::DispatchKey::ZeroTensor, c10::DispatchKey::NestedTensor});
+    return !t.key_set().has_any(other);
+}
+bool plain(PyObject *o, int device) {
+    if (!plain_class(o)) return false;
+    const Tensor &t = THPVariable_Unpack(o);
+    return t.is_cuda() && (device < 0 || t.get_device() == device) && t.layout() == at::kStrided && t.is_contiguous();
+}
+// No mode that wants to see operators: tracing, functional transforms, dispatch or function modes.
+bool no_modes() {
+    const c10::impl::LocalDispatchKeySet tls = c10::impl::tls_local_dispatch_key_set();
+    static const c10::DispatchKeySet front({c10::DispatchKey::FuncTorchDynamicLayerFrontMode, c10::DispatchKey::FuncTorchVmapMode, c10::DispatchKey::Functionalize,
+                                            c10::DispatchKey::Tracer, c10::DispatchKey::Python, c10::DispatchKey::PreDispatch});
+    return !tls.included_.has_any(front) && !c10::impl::TorchDispatchModeTLS::any_modes_set() && at::impl::PythonTorchFunctionTLS::stack_len() == 0;
+}
+// Whether the decode calls below read this tensor as it is.  Where one of theirs does not, or a mode wants to see operators, they return None and the caller takes
+// the operators, which accept any strides and types that go together.  What is no CUDA tensor is an error of the call.
+bool direct(PyObject *o, at::ScalarType type, uintptr_t align = 16) {
+    if (!THPVariable_Check(o) || !THPVariable_Unpack(o).is_cuda()) return true;
+    if (!plain(o, -1)) return false;
+    const Tensor &t = THPVariable_Unpack(o);
+    return t.scalar_type() == type && reinterpret_cast<uintptr_t>(t.const_data_ptr()) % align == 0;
+}
+
+// The same of a KV cache.  The library's attention reads it in vectors of 16 bytes and faults on one whose rows are not aligned for them: such a cache is refused.
+bool direct_cache(PyObject *o) {
+    if (direct(o, at::kBFloat16)) return true;
+    const Tensor &t = THPVariable_Unpack(o);
+    if (plain_class(o) && t.layout() == at::kStrided && t.dim() == 4 && t.stride(3) == 1) {
+        bool aligned = reinterpret_cast<uintptr_t>(t.const_data_ptr()) % 16 == 0;
+        for (int i = 0; i < 3; ++i) aligned = aligned && t.stride(i) * t.element_size() % 16 == 0;
+        TORCH_CHECK(aligned, "gpuk: rows of a KV cache must be 16-byte aligned");
+    }
+    return false;
+}
+
 // rope_append(qkv [rows, (heads + 2 kv_heads) * head_dim], cos, sin, pos [t], k_cache, v_cache, heads) -> q [rows, heads * head_dim]
 PyObject *rope_append(PyObject *, PyObject *const *args, Py_ssize_t n) {
     HANDLE_TH_ERRORS
     expect_args(n, 7, "rope_append");
+    if (!no_modes() || !direct(args[0], at::kBFloat16) || !direct(args[1], at::kFloat) || !direct(args[2], at::kFloat) || !direct(args[3], at::kLong, 8) ||
+        !direct_cache(args[4]) || !direct_cache(args[5]))
+        Py_RETURN_NONE;
     const Tensor &qkv = cuda_arg(args[0], "qkv", at::kBFloat16);
     const int dev = qkv.get_device();
     const Tensor &cos = cuda_arg(args[1], "cos", at::kFloat, dev), &sin = cuda_arg(args[2], "sin", at::kFloat, dev);
@@ -79,6 +125,7 @@ PyObject *rope_append(PyObject *, PyObject *const *args, Py_ssize_t n) {
 PyObject *silu_mul(PyObject *, PyObject *const *args, Py_ssize_t n) {
     HANDLE_TH_ERRORS
     expect_args(n, 1, "silu_mul");
+    if (!no_modes() || !direct(args[0], at::kBFloat16)) Py_RETURN_NONE;
     const Tensor &x = cuda_arg(args[0], "x", at::kBFloat16);
     TORCH_CHECK(x.dim() == 2 && x.size(1) % 2 == 0, "gpuk: silu_mul takes [rows, 2 f]");
     Tensor out;
@@ -96,6 +143,7 @@ PyObject *silu_mul(PyObject *, PyObject *const *args, Py_ssize_t n) {
 PyObject *linear(PyObject *, PyObject *const *args, Py_ssize_t n) {
     HANDLE_TH_ERRORS
     expect_args(n, 2, "linear");
+    if (!no_modes() || !direct(args[0], at::kBFloat16) || !direct(args[1], at::kBFloat16)) Py_RETURN_NONE;
     const Tensor &x = cuda_arg(args[0], "x", at::kBFloat16);
     const Tensor &w = cuda_arg(args[1], "w", at::kBFloat16, x.get_device());
     TORCH_CHECK(x.dim() == 2 && w.dim() == 2 && x.size(1) == w.size(1), "gpuk: linear operand shapes do not match");
@@ -116,6 +164,10 @@ struct Operands {
     const Tensor &x, &w;
     const float *x_scale = nullptr, *w_scale = nullptr;
     int m, n, k;
+    static bool are_direct(PyObject *const *args) {
+        const at::ScalarType type = args[1] == Py_None ? at::kBFloat16 : at::kFloat8_e4m3fn;
+        return direct(args[0], type) && direct(args[2], type) && direct(args[1], at::kFloat, 4) && direct(args[3], at::kFloat);
+    }
     Operands(PyObject *const *args) : x(cuda_arg(args[0], "x", args[1] == Py_None ? at::kBFloat16 : at::kFloat8_e4m3fn)), w(cuda_arg(args[2], "w", x.scalar_type(), x.get_device())) {
         TORCH_CHECK(x.dim() == 2 && w.dim() == 2 && x.size(1) == w.size(1) && (args[1] == Py_None) == (args[3] == Py_None), "gpuk: linear operand shapes do not match");
         TORCH_CHECK(x.size(0) <= INT_MAX && w.size(0) <= INT_MAX && w.size(1) <= INT_MAX, "gpuk: linear sizes out of range");
@@ -131,6 +183,7 @@ struct Operands {
 PyObject *swiglu(PyObject *, PyObject *const *args, Py_ssize_t n) {
     HANDLE_TH_ERRORS
     expect_args(n, 4, "swiglu");
+    if (!no_modes() || !Operands::are_direct(args)) Py_RETURN_NONE;
     const Operands o(args);
     Tensor out;
     {
@@ -147,6 +200,9 @@ PyObject *swiglu(PyObject *, PyObject *const *args, Py_ssize_t n) {
 PyObject *qkv_rope(PyObject *, PyObject *const *args, Py_ssize_t n) {
     HANDLE_TH_ERRORS
     expect_args(n, 10, "qkv_rope");
+    if (!no_modes() || !Operands::are_direct(args) || !direct(args[4], at::kFloat) || !direct(args[5], at::kFloat) || !direct(args[6], at::kLong, 8) ||
+        !direct_cache(args[7]) || !direct_cache(args[8]))
+        Py_RETURN_NONE;
     const Operands o(args);
     const int dev = o.x.get_device();
     const Tensor &cos = cuda_arg(args[4], "cos", at::kFloat, dev), &sin = cuda_arg(args[5], "sin", at::kFloat, dev), &pos = cuda_arg(args[6], "positions", at::kLong, dev);
@@ -171,6 +227,7 @@ PyObject *qkv_rope(PyObject *, PyObject *const *args, Py_ssize_t n) {
 PyObject *decode_attention(PyObject *, PyObject *const *args, Py_ssize_t n) {
     HANDLE_TH_ERRORS
     expect_args(n, 4, "decode_attention");
+    if (!no_modes() || !direct(args[0], at::kBFloat16) || !direct_cache(args[1]) || !direct_cache(args[2])) Py_RETURN_NONE;
     const Tensor &q = cuda_arg(args[0], "q", at::kBFloat16);
     const int dev = q.get_device();
     const Tensor &kc = cuda_arg(args[1], "k_cache", at::kBFloat16, dev), &vc = cuda_arg(args[2], "v_cache", at::kBFloat16, dev);
@@ -194,6 +251,8 @@ PyObject *decode_attention(PyObject *, PyObject *const *args, Py_ssize_t n) {
 PyObject *prefill_attention(PyObject *, PyObject *const *args, Py_ssize_t n) {
     HANDLE_TH_ERRORS
     expect_args(n, 5, "prefill_attention");
+    if (!no_modes() || !direct(args[0], at::kBFloat16) || !direct_cache(args[1]) || !direct_cache(args[2]) || !direct(args[3], at::kLong, 8))
+        Py_RETURN_NONE;
     const Tensor &q = cuda_arg(args[0], "q", at::kBFloat16);
     const int dev = q.get_device();
     const Tensor &kc = cuda_arg(args[1], "k_cache", at::kBFloat16, dev), &vc = cuda_arg(args[2], "v_cache", at::kBFloat16, dev);
@@ -246,23 +305,6 @@ PyObject *fp8_linear(PyObject *, PyObject *const *args, Py_ssize_t n) {
     END_HANDLE_TH_ERRORS
 }
 
-// A tensor whose operators would go straight to the CUDA kernels: of the class Tensor itself, dense and contiguous, no transform or lazy bit on it.
-bool plain(PyObject *o, int device) {
-    if (!THPVariable_CheckExact(o)) return false;
-    const Tensor &t = THPVariable_Unpack(o);
-    static const c10::DispatchKeySet other({c10::DispatchKey::Python, c10::DispatchKey::PythonTLSSnapshot, c10::DispatchKey::Functionalize, c10::DispatchKey::FuncTorchBatched,
-                                            c10::DispatchKey::FuncTorchGradWrapper, c10::DispatchKey::Batched, c10::DispatchKey::Negative, c10::DispatchKey::Conjugate,
-                                            c10::DispatchKey::ZeroTensor, c10::DispatchKey::NestedTensor});
-    return t.is_cuda() && (device < 0 || t.get_device() == device) && t.layout() == at::kStrided && t.is_contiguous() && !t.key_set().has_any(other);
-}
-// No mode that wants to see operators: tracing, functional transforms, dispatch or function modes.
-bool no_modes() {
-    const c10::impl::LocalDispatchKeySet tls = c10::impl::tls_local_dispatch_key_set();
-    static const c10::DispatchKeySet front({c10::DispatchKey::FuncTorchDynamicLayerFrontMode, c10::DispatchKey::FuncTorchVmapMode, c10::DispatchKey::Functionalize,
-                                            c10::DispatchKey::Tracer, c10::DispatchKey::Python, c10::DispatchKey::PreDispatch});
-    return !tls.included_.has_any(front) && !c10::impl::TorchDispatchModeTLS::any_modes_set() && at::impl::PythonTorchFunctionTLS::stack_len() == 0;
-}
-
 // add_rms(workspace, x, residual, weight, eps, quant_type, scale or None) -> (residual_out, norm_out, scale), what allreduce_rms computes, with the
 // results allocated here; None for a call that should take the operator instead: whatever is not plain tensors of matching sizes and types.
 PyObject *add_rms(PyObject *, PyObject *const *args, Py_ssize_t n) {
@@ -313,10 +355,18 @@ PyObject *add_rms(PyObject *, PyObject *const *args, Py_ssize_t n) {
     END_HANDLE_TH_ERRORS
 }
 
+// no_modes(): whether nothing but the kernels would see the operators of this thread's next call
+PyObject *no_modes_py(PyObject *, PyObject *) {
+    HANDLE_TH_ERRORS
+    return PyBool_FromLong(no_modes());
+    END_HANDLE_TH_ERRORS
+}
+
 template <PyObject *(*F)(PyObject *, PyObject *const *, Py_ssize_t)>
 constexpr PyCFunction fast() { return reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(F)); }
 
 PyMethodDef methods[] = {
+    {"no_modes", no_modes_py, METH_NOARGS, nullptr},
     {"rope_append", fast<rope_append>(), METH_FASTCALL, nullptr},
     {"swiglu", fast<swiglu>(), METH_FASTCALL, nullptr},
     {"qkv_rope", fast<qkv_rope>(), METH_FASTCALL, nullptr},

@@ -95,8 +95,10 @@ class _Linear:
     def __call__(self, x: torch.Tensor, x_scale: Optional[torch.Tensor] = None) -> torch.Tensor:
         # measured on B200: at up to 32 tokens the streaming kernels are the faster ones at the decoder's shapes (fp8_linear.cu, stream_linear.cu)
         own = self.own_gemm and x.is_cuda and 0 < x.shape[0] <= 32 and self.weight.dtype == torch.bfloat16
+        if own:
+            from gpuk_b200 import _native
         if self.fp8 and x.dtype == torch.float8_e4m3fn:
-            if own:
+            if own and _native.no_modes() and (x.shape[0] <= 8 or self.w_q.is_contiguous()):
                 import gpuk_b200 as gpuk
                 if gpuk.fp8_linear_supported(x.shape[0], *self.w_q.shape):
                     if x.shape[0] > 8:
@@ -107,8 +109,9 @@ class _Linear:
                     return gpuk.fp8_linear(x, x_scale, self.w_packed, self.w_scale, packed=True)
             return torch._scaled_mm(x, self.w_q.t(), scale_a=x_scale, scale_b=self.w_scale, out_dtype=self.weight.dtype)
         if own and x.dtype == torch.bfloat16 and self.weight.shape[0] % 128 == 0 and self.weight.shape[1] % 8 == 0:
-            from gpuk_b200 import _native
-            return _native.linear(x, self.weight)
+            y = _native.linear(x, self.weight)
+            if y is not None:      # weights that are views, and modes that want to see operators, belong to the library
+                return y
         return F.linear(x, self.weight)
 
 
@@ -240,8 +243,12 @@ class TPDecoder:
         b, t = tokens.shape
         hd = a.head_dim
         h = F.embedding(tokens, self.tok_embeddings).view(b * t, a.dim)
-        own = self.own_elementwise
-        here = input_pos if not input_pos.is_cuda else input_pos.cpu() if cache_len is None else None
+        # positions in any other form that indexes a tensor go to the operators, as do caches, tables and weights that the kernels cannot read as they are
+        own = self.own_elementwise and isinstance(input_pos, torch.Tensor) and input_pos.shape == (t,) and input_pos.dtype in (torch.int64, torch.int32) and \
+            (not input_pos.is_cuda or input_pos.device == self.cos.device)
+        here = input_pos
+        if own and input_pos.is_cuda:
+            here = input_pos.cpu() if cache_len is None else None
         last = int(here[-1]) + 1 if cache_len is None else cache_len
         if own:
             from gpuk_b200 import _native
@@ -251,35 +258,37 @@ class TPDecoder:
                 raise RuntimeError(f"position {last - 1} is beyond the KV cache ({a.max_seq_len} positions)")
             if here is not None and here.numel() and not -a.max_seq_len <= int(here.min()) <= int(here.max()) < a.max_seq_len:
                 raise RuntimeError(f"a position in [{int(here.min())}, {int(here.max())}] is beyond the KV cache ({a.max_seq_len} positions)")
-            if input_pos.shape != (t,):
-                raise RuntimeError(f"{t} tokens a sequence at positions of shape {tuple(input_pos.shape)}")
             pos = input_pos.to(device=self.device, dtype=torch.int64).contiguous()
-        else:
-            cos, sin = self.cos[input_pos], self.sin[input_pos]
-        own_attention = own and self.own_attention and last >= 1
-        mask = None
-        if t > 1 and not own_attention:
-            mask = (torch.arange(last, device=self.device)[None, :] <= input_pos[:, None])[None, None]
-            if own:
-                mask = mask | (input_pos < -a.max_seq_len)[:, None]      # a token that the rotary embedding marked attends, and stays marked
+        tables = mask = None      # what the operators need, once one of them is called
         normed, scale = self._norm_only(h, self.layers[0]["attention_norm"])
         for li, layer in enumerate(self.layers):
+            q = att = act = None      # a native call returns None where the operators are wanted
             fused = layer["wqkv"].streamed(normed) if own and hd == 128 else None
-            qkv = layer["wqkv"](normed, scale) if fused is None else None
             if fused is not None:
-                q = _native.qkv_rope(normed, scale, *fused, self.cos, self.sin, pos, layer["k_cache"], layer["v_cache"], self.h_local).view(b, t, self.h_local, hd)
-            elif own:
-                q = _native.rope_append(qkv, self.cos, self.sin, pos, layer["k_cache"], layer["v_cache"], self.h_local).view(b, t, self.h_local, hd)
+                q = _native.qkv_rope(normed, scale, *fused, self.cos, self.sin, pos, layer["k_cache"], layer["v_cache"], self.h_local)
+            if q is None:
+                qkv = layer["wqkv"](normed, scale)
+                if own:
+                    q = _native.rope_append(qkv, self.cos, self.sin, pos, layer["k_cache"], layer["v_cache"], self.h_local)
+            if q is not None:
+                q = q.view(b, t, self.h_local, hd)
             else:
+                if tables is None:
+                    tables = self.cos[input_pos], self.sin[input_pos]
                 q, k, v = qkv.view(b, t, self.h_local + 2 * self.kv_local, hd).split([self.h_local, self.kv_local, self.kv_local], dim=2)
-                q, k = self._rope(q, cos, sin), self._rope(k, cos, sin)
+                q, k = self._rope(q, *tables), self._rope(k, *tables)
                 layer["k_cache"][:b, :, input_pos] = k.transpose(1, 2)
                 layer["v_cache"][:b, :, input_pos] = v.transpose(1, 2)
-            if own_attention and t == 1 and self.h_local // self.kv_local <= 16:
-                att = _native.decode_attention(q.view(b, self.h_local, hd), layer["k_cache"], layer["v_cache"], last)
-            elif own_attention and t > 1:
-                att = _native.prefill_attention(q, layer["k_cache"], layer["v_cache"], pos, last)
-            else:
+            if own and self.own_attention and last >= 1:
+                if t > 1:
+                    att = _native.prefill_attention(q, layer["k_cache"], layer["v_cache"], pos, last)
+                elif self.h_local // self.kv_local <= 16:
+                    att = _native.decode_attention(q.reshape(b, self.h_local, hd), layer["k_cache"], layer["v_cache"], last)
+            if att is None:
+                if t > 1 and mask is None:
+                    mask = (torch.arange(last, device=self.device)[None, :] <= input_pos[:, None])[None, None]
+                    if own:
+                        mask = mask | (input_pos < -a.max_seq_len)[:, None]      # a token that the rotary embedding marked attends, and stays marked
                 att = F.scaled_dot_product_attention(q.transpose(1, 2), layer["k_cache"][:b, :, :last], layer["v_cache"][:b, :, :last],
                                                      attn_mask=mask, enable_gqa=True).transpose(1, 2).reshape(b * t, self.h_local * hd)
             partial = layer["wo"](att)
@@ -287,10 +296,12 @@ class TPDecoder:
             fused = layer["w13"].streamed(normed) if own else None
             if fused is not None:
                 act = _native.swiglu(normed, scale, *fused)
-            elif own:
-                act = _native.silu_mul(layer["w13"](normed, scale))
-            else:
-                f1, f3 = layer["w13"](normed, scale).split(a.ffn_dim // self.world, dim=-1)
+            if act is None:
+                f13 = layer["w13"](normed, scale)
+                if own:
+                    act = _native.silu_mul(f13)
+            if act is None:
+                f1, f3 = f13.split(a.ffn_dim // self.world, dim=-1)
                 act = F.silu(f1) * f3
             partial = layer["w2"](act)
             nxt = self.layers[li + 1]["attention_norm"] if li + 1 < a.n_layers else self.norm

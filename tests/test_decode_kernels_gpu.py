@@ -350,3 +350,122 @@ def test_decoder_marks_positions_behind_its_cache(decoder, head_dim, fp8):
             m.forward(three, torch.tensor([10, bad, 12], device="cuda"))
     assert not bool(m.forward(one, torch.tensor([63], device="cuda"), cache_len=70).isnan().any())
     _status_ok()
+
+
+def _strided(t):
+    """The same values with another order of the two dimensions in the middle or, of a matrix, as columns of a wider one."""
+    if t.dim() == 4:
+        return t.transpose(1, 2).contiguous().transpose(1, 2)
+    return torch.cat([t, t], 1)[:, :t.shape[1]]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("t", [1, 3])
+@pytest.mark.parametrize("what", ["caches", "weights", "tables", "everything"])
+def test_decoder_takes_tensors_the_kernels_do_not_read(decoder, what, t):
+    """Views in the place of caches and weights, tables in another type: what the operators took, they take.  Same values as without, up to the roundings of
+    bf16 between the operators."""
+    plain, m = decoder(), decoder()
+    tokens, pos = torch.arange(2 * t, device="cuda").view(2, t), torch.arange(20, 20 + t, device="cuda")
+    want = plain.forward(tokens, pos, cache_len=20 + t)
+    for layer in m.layers:
+        if what in ("caches", "everything"):
+            layer["k_cache"], layer["v_cache"] = _strided(layer["k_cache"]), _strided(layer["v_cache"])
+        if what in ("weights", "everything"):
+            for name in ("wqkv", "wo", "w13", "w2"):
+                layer[name].weight = _strided(layer[name].weight)
+    if what in ("tables", "everything"):
+        m.cos, m.sin = m.cos.double(), m.sin.double()
+    got = m.forward(tokens, pos, cache_len=20 + t)
+    _status_ok()
+    assert float((got.float() - want.float()).norm()) <= 0.03 * float(want.float().norm())
+    for a, b in zip(m.layers, plain.layers):
+        for name in ("k_cache", "v_cache"):
+            assert float((a[name].float() - b[name].float()).abs().max()) <= 0.06
+
+
+@pytest.mark.gpu
+def test_native_calls_hand_back_what_the_kernels_do_not_read():
+    """Odd addresses and strides: None, before any launch; a cache that the library's attention could not read either is refused."""
+    x, w = torch.zeros(2, 256, device="cuda").bfloat16(), torch.zeros(257 * 256, device="cuda").bfloat16()
+    odd = w[1:1 + 256 * 256].view(256, 256)
+    assert _native.linear(x, odd) is None and _native.swiglu(x, None, odd, None) is None and _native.linear(x, w[:65536].view(256, 256).t()) is None
+    assert _native.silu_mul(w[1:513].view(2, 256)) is None
+    q, pos = torch.zeros(2, 1, 128, device="cuda").bfloat16(), torch.zeros(1, dtype=torch.long, device="cuda")
+    cos, flat = torch.zeros(8, 64, device="cuda"), torch.zeros(2 * 4 * 136 + 1, device="cuda").bfloat16()
+    fine = flat[:1024].view(2, 1, 4, 128)
+    for bad in (flat[1:1025].view(2, 1, 4, 128), flat[:2 * 4 * 132].view(2, 1, 4, 132)[..., :128]):
+        for call in (lambda k, v: _native.decode_attention(q, k, v, 4), lambda k, v: _native.prefill_attention(q.view(1, 2, 1, 128), k, v, pos.expand(2).contiguous(), 4),
+                     lambda k, v: _native.rope_append(torch.zeros(2, 384, device="cuda").bfloat16(), cos, cos, pos, k, v, 1)):
+            with pytest.raises(RuntimeError, match="aligned"):
+                call(bad, fine)
+            with pytest.raises(RuntimeError, match="aligned"):
+                call(fine, bad)
+    wide = flat[:2 * 4 * 136].view(2, 1, 4, 136)[..., :128]
+    assert _native.decode_attention(q, wide, wide, 4) is None
+
+
+@pytest.mark.gpu
+def test_decoder_takes_the_positions_it_took(decoder):
+    """A list and 32-bit positions; what indexes no tensor is refused."""
+    m, one = decoder(), torch.zeros(2, 1, dtype=torch.long, device="cuda")
+    want = m.forward(one, torch.tensor([30], device="cuda"), cache_len=31)
+    for positions in (torch.tensor([30], device="cuda", dtype=torch.int32), torch.tensor([30]), [30], slice(30, 31)):
+        got = m.forward(one, positions, cache_len=31)
+        assert float((got.float() - want.float()).norm()) <= 0.03 * float(want.float().norm())
+    for positions in (torch.tensor([30.0], device="cuda"), torch.tensor([30], device="cuda", dtype=torch.int16)):
+        with pytest.raises((RuntimeError, IndexError)):
+            m.forward(one, positions, cache_len=31)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("fp8", [False, True])
+@pytest.mark.parametrize("t", [1, 20])
+def test_modes_see_the_decoder_s_operators(decoder, t, fp8):
+    m = decoder(fp8=fp8)
+    tokens, pos = torch.arange(2 * t, device="cuda").view(2, t), torch.arange(20, 20 + t, device="cuda")
+    want = m.forward(tokens, pos, cache_len=20 + t)
+    seen = []
+
+    class Mode(torch.utils._python_dispatch.TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            seen.append(str(func))
+            return func(*args, **(kwargs or {}))
+    with Mode():
+        got = m.forward(tokens, pos, cache_len=20 + t)
+    products = [f for f in seen if "mm" in f or "linear" in f]
+    assert len(products) == 4 * 2 + 1 and sum("scaled_dot_product" in f for f in seen) == 2 and sum("silu" in f for f in seen) == 2, seen
+    assert float((got.float() - want.float()).norm()) <= (0.08 if fp8 else 0.03) * float(want.float().norm())
+
+
+@pytest.mark.gpu
+def test_native_calls_of_other_streams_and_threads():
+    """Each kind of call on a stream of its own behind the kernels that make its inputs, from four threads at once: the bits of a call by itself."""
+    import threading
+
+    def work(i, results):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            g = torch.Generator(device="cuda").manual_seed(i % 2)
+            for _ in range(5):
+                x = torch.randn(5, 1024, generator=g, device="cuda").bfloat16()
+                w13, wq = (torch.randn(n, 1024, generator=g, device="cuda").bfloat16() * 0.03 for n in (1024, 1024))
+                caches = [torch.randn(5, 2, 40, 128, generator=g, device="cuda").bfloat16() for _ in range(2)]
+                cos, pos = torch.randn(80, 64, generator=g, device="cuda"), torch.tensor([11], device="cuda")
+                q = _native.qkv_rope(x, None, wq, None, cos, cos, pos, *caches, 4)
+                mine = [_native.silu_mul(_native.linear(x, w13)), _native.swiglu(x, None, w13, None), q, *caches, _native.decode_attention(q.view(5, 4, 128), *caches, 12),
+                        _native.rope_append(_native.linear(x, wq), cos, cos, pos, *caches, 4),
+                        _native.prefill_attention(q.view(1, 5, 4, 128), *caches, torch.arange(5, 10, device="cuda"), 12)]
+            torch.cuda.current_stream().synchronize()
+            results[i] = [t.clone() for t in mine]
+            torch.cuda.current_stream().synchronize()
+    alone, together = {}, {}
+    for i in range(2):
+        work(i, alone)
+    threads = [threading.Thread(target=work, args=(i, together)) for i in range(4)]
+    for th in threads:
+        th.start()
+    for th in threads:
+        th.join()
+    _status_ok()
+    for i in range(4):
+        assert all(torch.equal(a, b) for a, b in zip(together[i], alone[i % 2]))
