@@ -392,7 +392,8 @@ class GPUKDistEnv:
         if self._o is _TorchOps and not torch.compiler.is_compiling():
             qt = (QUANT_STATIC_E4M3FN_448 if static_scale is not None else
                   QUANT_NONE if not fp8_out else fp8_policy_id if quant_type is None else quant_type)
-            if static_scale is None or isinstance(static_scale, torch.Tensor):
+            # FP8 asked for with a policy that is none is an error of the operator
+            if (static_scale is None or isinstance(static_scale, torch.Tensor)) and not (fp8_out and qt == QUANT_NONE):
                 results = _native.add_rms(self.fptr or 0, allreduce_in, residual_in, rms_weight, eps, qt,
                                           None if static_scale is None else static_scale.reshape(-1))
                 if results is not None:

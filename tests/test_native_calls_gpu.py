@@ -42,6 +42,15 @@ def test_same_as_the_operator(env, shape, quant, dtype):
 
 
 @pytest.mark.gpu
+def test_policies_that_do_not_go_together_are_refused(env):
+    x, w = torch.randn(4, 1024, device="cuda"), torch.ones(1024, device="cuda")
+    for policy in (0, 7, -1):
+        with pytest.raises(RuntimeError):
+            env.allreduce_add_rms_fused(x, x, w, 1e-6, True, quant_type=policy)
+    assert env.allreduce_add_rms_fused(x, x, w, 1e-6, False, quant_type=3)[1].dtype == x.dtype
+
+
+@pytest.mark.gpu
 def test_what_is_not_plain_takes_the_operator(env):
     class Sub(torch.Tensor):
         pass
