@@ -125,6 +125,8 @@ extern "C" int gpuk_rope_append(const void *qkv, const float *cos, const float *
     if (batch < 0 || t < 0 || heads <= 0 || kv_heads <= 0 || table_rows <= 0 || max_seq <= 0)
         return set_last_error(GPUK_ERR_INVALID_ARGUMENT, "rope_append: bad sizes");
     if (head_dim <= 0 || head_dim % kRopeVec) return set_last_error(GPUK_ERR_UNSUPPORTED, "rope_append: head_dim %d is not a multiple of %d", head_dim, kRopeVec);
+    if (static_cast<int64_t>(batch) * t > 0x7fffffffll || (heads + 2ll * kv_heads) * (head_dim / kRopeVec) > 0x7fffffffll)
+        return set_last_error(GPUK_ERR_UNSUPPORTED, "rope_append: too many rows or heads");
     if (batch == 0 || t == 0) return GPUK_OK;
     if (!qkv || !cos || !sin || !pos || !q_out || !k_cache || !v_cache) return set_last_error(GPUK_ERR_INVALID_ARGUMENT, "rope_append: null pointer");
     if (!aligned16(qkv) || !aligned16(cos) || !aligned16(sin) || !aligned16(q_out) || !aligned16(k_cache) || !aligned16(v_cache))
@@ -135,7 +137,7 @@ extern "C" int gpuk_rope_append(const void *qkv, const float *cos, const float *
     RopeParams p = {static_cast<const bf16 *>(qkv), cos, sin, pos, static_cast<bf16 *>(q_out), static_cast<bf16 *>(k_cache), static_cast<bf16 *>(v_cache),
                     static_cast<int64_t>(batch) * t * (heads + 2 * kv_heads) * (head_dim / kRopeVec), status + kStatusPosition, t, heads, kv_heads, head_dim, table_rows, max_seq};
     const int64_t grid = (p.total + kThreads - 1) / kThreads;
-    if (grid > 0x7fffffffll || static_cast<int64_t>(batch) * t > 0x7fffffffll) return set_last_error(GPUK_ERR_UNSUPPORTED, "rope_append: too many rows");
+    if (grid > 0x7fffffffll) return set_last_error(GPUK_ERR_UNSUPPORTED, "rope_append: too many rows");
     void *args[] = {&p};
     cudaError_t e = launch_kernel(reinterpret_cast<const void *>(&rope_append_kernel), static_cast<int>(grid), kThreads, 1, false, args, static_cast<cudaStream_t>(stream));
     if (e != cudaSuccess) return set_last_error(GPUK_ERR_CUDA, "rope_append: launch failed: %s", cudaGetErrorString(e));
@@ -145,6 +147,7 @@ extern "C" int gpuk_rope_append(const void *qkv, const float *cos, const float *
 extern "C" int gpuk_silu_mul(const void *in, void *out, int64_t rows, int f, void *stream) {
     if (rows < 0 || f <= 0) return set_last_error(GPUK_ERR_INVALID_ARGUMENT, "silu_mul: bad sizes");
     if (f % 8) return set_last_error(GPUK_ERR_UNSUPPORTED, "silu_mul: %d channels are not a multiple of 8", f);
+    if (rows > 0x7fffffffll) return set_last_error(GPUK_ERR_UNSUPPORTED, "silu_mul: too many rows");
     if (rows == 0) return GPUK_OK;
     if (!in || !out || !aligned16(in) || !aligned16(out)) return set_last_error(GPUK_ERR_INVALID_ARGUMENT, "silu_mul: pointers must be 16-byte aligned and not null");
     // two vectors a thread keep enough loads in flight; a batch of a few tokens is better spread over more CTAs

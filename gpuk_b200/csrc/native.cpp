@@ -41,6 +41,11 @@ int64_t int_arg(PyObject *o) {
     if (v == -1 && PyErr_Occurred()) throw python_error();
     return v;
 }
+// A size as the C ABI takes it.
+int int_size(int64_t v) {
+    TORCH_CHECK(v >= 0 && v <= INT_MAX, "gpuk: a size of ", v, " is out of range");
+    return static_cast<int>(v);
+}
 struct NoGil {
     PyThreadState *state = PyEval_SaveThread();
     ~NoGil() { PyEval_RestoreThread(state); }
@@ -114,8 +119,8 @@ PyObject *rope_append(PyObject *, PyObject *const *args, Py_ssize_t n) {
         c10::cuda::CUDAGuard guard(qkv.device());
         q = empty_like_on(qkv, {rows, heads * hd}, at::kBFloat16);
         check(gpuk_rope_append(qkv.data_ptr(), cos.data_ptr<float>(), sin.data_ptr<float>(), pos.data_ptr<int64_t>(), q.data_ptr(), kc.data_ptr(), vc.data_ptr(),
-                               static_cast<int>(rows / t), static_cast<int>(t), static_cast<int>(heads), static_cast<int>(kv), static_cast<int>(hd),
-                               static_cast<int>(cos.size(0)), static_cast<int>(max_seq), stream_of(qkv)), "rope_append");
+                               int_size(rows / t), int_size(t), int_size(heads), int_size(kv), int_size(hd),
+                               int_size(cos.size(0)), int_size(max_seq), stream_of(qkv)), "rope_append");
     }
     return THPVariable_Wrap(std::move(q));
     END_HANDLE_TH_ERRORS
@@ -133,7 +138,7 @@ PyObject *silu_mul(PyObject *, PyObject *const *args, Py_ssize_t n) {
         NoGil unlocked;
         c10::cuda::CUDAGuard guard(x.device());
         out = empty_like_on(x, {x.size(0), x.size(1) / 2}, at::kBFloat16);
-        check(gpuk_silu_mul(x.data_ptr(), out.data_ptr(), x.size(0), static_cast<int>(x.size(1) / 2), stream_of(x)), "silu_mul");
+        check(gpuk_silu_mul(x.data_ptr(), out.data_ptr(), x.size(0), int_size(x.size(1) / 2), stream_of(x)), "silu_mul");
     }
     return THPVariable_Wrap(std::move(out));
     END_HANDLE_TH_ERRORS
@@ -152,7 +157,7 @@ PyObject *linear(PyObject *, PyObject *const *args, Py_ssize_t n) {
         NoGil unlocked;
         c10::cuda::CUDAGuard guard(x.device());
         out = empty_like_on(x, {x.size(0), w.size(0)}, at::kBFloat16);
-        check(gpuk_linear_skinny(x.data_ptr(), w.data_ptr(), out.data_ptr(), static_cast<int>(x.size(0)), static_cast<int>(w.size(0)), static_cast<int>(x.size(1)), 0,
+        check(gpuk_linear_skinny(x.data_ptr(), w.data_ptr(), out.data_ptr(), int_size(x.size(0)), int_size(w.size(0)), int_size(x.size(1)), 0,
                                  stream_of(x)), "linear");
     }
     return THPVariable_Wrap(std::move(out));
@@ -170,8 +175,7 @@ struct Operands {
     }
     Operands(PyObject *const *args) : x(cuda_arg(args[0], "x", args[1] == Py_None ? at::kBFloat16 : at::kFloat8_e4m3fn)), w(cuda_arg(args[2], "w", x.scalar_type(), x.get_device())) {
         TORCH_CHECK(x.dim() == 2 && w.dim() == 2 && x.size(1) == w.size(1) && (args[1] == Py_None) == (args[3] == Py_None), "gpuk: linear operand shapes do not match");
-        TORCH_CHECK(x.size(0) <= INT_MAX && w.size(0) <= INT_MAX && w.size(1) <= INT_MAX, "gpuk: linear sizes out of range");
-        m = static_cast<int>(x.size(0)), n = static_cast<int>(w.size(0)), k = static_cast<int>(w.size(1));
+        m = int_size(x.size(0)), n = int_size(w.size(0)), k = int_size(w.size(1));
         if (args[1] == Py_None) return;
         const Tensor &xs = cuda_arg(args[1], "x_scale", at::kFloat, x.get_device()), &ws = cuda_arg(args[3], "w_scale", at::kFloat, x.get_device());
         TORCH_CHECK(xs.numel() == m && ws.numel() == n, "gpuk: linear takes a scale per token and per channel");
@@ -216,8 +220,8 @@ PyObject *qkv_rope(PyObject *, PyObject *const *args, Py_ssize_t n) {
         c10::cuda::CUDAGuard guard(o.x.device());
         q = empty_like_on(o.x, {o.m, heads * 128}, at::kBFloat16);
         check(gpuk_qkv_rope_skinny(o.x.data_ptr(), o.x_scale, o.w.data_ptr(), o.w_scale, cos.data_ptr<float>(), sin.data_ptr<float>(), pos.data_ptr<int64_t>(), q.data_ptr(),
-                                   kc.data_ptr(), vc.data_ptr(), static_cast<int>(o.m / t), static_cast<int>(t), static_cast<int>(heads), static_cast<int>(kc.size(1)), o.k,
-                                   static_cast<int>(cos.size(0)), static_cast<int>(kc.size(2)), 0, stream_of(o.x)), "qkv_rope");
+                                   kc.data_ptr(), vc.data_ptr(), int_size(o.m / t), int_size(t), int_size(heads), int_size(kc.size(1)), o.k,
+                                   int_size(cos.size(0)), int_size(kc.size(2)), 0, stream_of(o.x)), "qkv_rope");
     }
     return THPVariable_Wrap(std::move(q));
     END_HANDLE_TH_ERRORS
@@ -239,8 +243,8 @@ PyObject *decode_attention(PyObject *, PyObject *const *args, Py_ssize_t n) {
         NoGil unlocked;
         c10::cuda::CUDAGuard guard(q.device());
         out = empty_like_on(q, {q.size(0), q.size(1) * q.size(2)}, at::kBFloat16);
-        check(gpuk_decode_attention(q.data_ptr(), kc.data_ptr(), vc.data_ptr(), out.data_ptr(), static_cast<int>(q.size(0)), static_cast<int>(q.size(1)),
-                                    static_cast<int>(kc.size(1)), static_cast<int>(q.size(2)), static_cast<int>(len), static_cast<int>(kc.size(2)), 0, stream_of(q)),
+        check(gpuk_decode_attention(q.data_ptr(), kc.data_ptr(), vc.data_ptr(), out.data_ptr(), int_size(q.size(0)), int_size(q.size(1)),
+                                    int_size(kc.size(1)), int_size(q.size(2)), int_size(len), int_size(kc.size(2)), 0, stream_of(q)),
               "decode_attention");
     }
     return THPVariable_Wrap(std::move(out));
@@ -265,9 +269,9 @@ PyObject *prefill_attention(PyObject *, PyObject *const *args, Py_ssize_t n) {
         NoGil unlocked;
         c10::cuda::CUDAGuard guard(q.device());
         out = empty_like_on(q, {q.size(0) * q.size(1), q.size(2) * q.size(3)}, at::kBFloat16);
-        check(gpuk_prefill_attention(q.data_ptr(), kc.data_ptr(), vc.data_ptr(), pos.data_ptr<int64_t>(), out.data_ptr(), static_cast<int>(q.size(0)),
-                                     static_cast<int>(q.size(1)), static_cast<int>(q.size(2)), static_cast<int>(kc.size(1)), static_cast<int>(q.size(3)),
-                                     static_cast<int>(len), static_cast<int>(kc.size(2)), stream_of(q)), "prefill_attention");
+        check(gpuk_prefill_attention(q.data_ptr(), kc.data_ptr(), vc.data_ptr(), pos.data_ptr<int64_t>(), out.data_ptr(), int_size(q.size(0)),
+                                     int_size(q.size(1)), int_size(q.size(2)), int_size(kc.size(1)), int_size(q.size(3)),
+                                     int_size(len), int_size(kc.size(2)), stream_of(q)), "prefill_attention");
     }
     return THPVariable_Wrap(std::move(out));
     END_HANDLE_TH_ERRORS
@@ -284,7 +288,8 @@ PyObject *fp8_linear(PyObject *, PyObject *const *args, Py_ssize_t n) {
     TORCH_CHECK(w.size(1) == k && xs.numel() == m && ws.numel() == channels, "gpuk: fp8_linear operand shapes do not match");
     TORCH_CHECK(xs.scalar_type() == at::kFloat && ws.scalar_type() == at::kFloat && xs.is_contiguous() && ws.is_contiguous(), "gpuk: fp8_linear takes contiguous fp32 scales");
     TORCH_CHECK(xs.is_cuda() && ws.is_cuda(), "gpuk: fp8_linear takes CUDA scales");
-    const bool packed = PyObject_IsTrue(args[5]) == 1;
+    const int packed = PyObject_IsTrue(args[5]);
+    if (packed < 0) throw python_error();
     const int64_t split = int_arg(args[6]);
     Tensor out;
     if (args[4] != Py_None) {

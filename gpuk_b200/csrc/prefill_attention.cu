@@ -304,6 +304,7 @@ extern "C" int gpuk_prefill_attention(const void *q, const void *k_cache, const 
     if (batch < 0 || t < 0 || heads <= 0 || kv_heads <= 0 || len <= 0 || max_seq < len) return set_last_error(GPUK_ERR_INVALID_ARGUMENT, "prefill_attention: bad sizes");
     if (head_dim != kHeadDim || heads % kv_heads)
         return set_last_error(GPUK_ERR_UNSUPPORTED, "prefill_attention: built for heads of %d, a whole number of them per kv head (got %d, %d / %d)", kHeadDim, head_dim, heads, kv_heads);
+    if (static_cast<int64_t>(batch) * heads > 0x7fffffffll) return set_last_error(GPUK_ERR_UNSUPPORTED, "prefill_attention: too many sequences");
     if (batch == 0 || t == 0) return GPUK_OK;
     if (!q || !k_cache || !v_cache || !pos || !out) return set_last_error(GPUK_ERR_INVALID_ARGUMENT, "prefill_attention: null pointer");
     if (!aligned16(q) || !aligned16(k_cache) || !aligned16(v_cache) || !aligned16(out)) return set_last_error(GPUK_ERR_INVALID_ARGUMENT, "prefill_attention: pointers must be 16-byte aligned");

@@ -267,6 +267,13 @@ def test_refused_shapes():
     assert b(16, 16, 16, 16, 16, 1, 4, 8, 2, 64, 4, 8, None) == cabi.ERR_UNSUPPORTED and b(16, 16, 16, 16, 16, 1, 4, 8, 3, 128, 4, 8, None) == cabi.ERR_UNSUPPORTED
     assert b(16, 16, 16, 16, 16, 1, 4, 8, 2, 128, 9, 8, None) == cabi.ERR_INVALID_ARGUMENT and b(16, 16, 8, 16, 16, 1, 4, 8, 2, 128, 4, 8, None) == cabi.ERR_INVALID_ARGUMENT
     assert b(16, 16, 16, 16, 16, 1, 0, 8, 2, 128, 4, 8, None) == cabi.OK
+    # sizes whose products leave 32 or 64 bits
+    big = (1 << 31) - 1
+    assert b(16, 16, 16, 16, 16, big, big, big, 1, 128, 4, 8, None) == cabi.ERR_UNSUPPORTED
+    r = cabi.lib.gpuk_rope_append
+    assert r(16, 16, 16, 16, 16, 16, 16, 1, 1, 1 << 30, 1 << 30, 128, 80, 40, None) == cabi.ERR_UNSUPPORTED
+    assert r(16, 16, 16, 16, 16, 16, 16, big, big, 8, 1, 128, 80, 40, None) == cabi.ERR_UNSUPPORTED
+    assert cabi.lib.gpuk_silu_mul(16, 16, 1 << 62, 1 << 30, None) == cabi.ERR_UNSUPPORTED
     c = cabi.lib.gpuk_swiglu_skinny
     assert c(16, 16, 16, None, 16, 8, 128, 64, 0, None) == cabi.ERR_INVALID_ARGUMENT and c(16, None, 16, None, 12, 8, 128, 64, 0, None) == cabi.ERR_INVALID_ARGUMENT
     assert c(16, None, 16, None, 16, 33, 128, 64, 0, None) == cabi.ERR_UNSUPPORTED and c(16, None, 16, None, 16, 8, 64, 64, 0, None) == cabi.ERR_UNSUPPORTED
