@@ -283,18 +283,20 @@ PyObject *fp8_linear(PyObject *, PyObject *const *args, Py_ssize_t n) {
     expect_args(n, 7, "fp8_linear");
     const Tensor &x = tensor_arg(args[0], "x_fp8"), &xs = tensor_arg(args[1], "x_scale"), &w = tensor_arg(args[2], "w_fp8"), &ws = tensor_arg(args[3], "w_scale");
     TORCH_CHECK(x.scalar_type() == at::kFloat8_e4m3fn && w.scalar_type() == at::kFloat8_e4m3fn, "gpuk: fp8_linear takes float8_e4m3fn operands");
-    TORCH_CHECK(x.is_cuda() && w.is_cuda() && x.is_contiguous() && w.is_contiguous() && x.dim() == 2 && w.dim() == 2, "gpuk: fp8_linear takes contiguous 2-d CUDA tensors");
+    // scales, results and (copied for the call) weights may also be pinned host memory, which the GPU reads
+    auto reachable = [](const Tensor &t) { return t.is_cuda() || t.is_pinned(); };
+    TORCH_CHECK(x.is_cuda() && reachable(w) && x.is_contiguous() && w.is_contiguous() && x.dim() == 2 && w.dim() == 2, "gpuk: fp8_linear takes contiguous 2-d CUDA tensors");
     const int64_t m = x.size(0), k = x.size(1), channels = w.size(0);
     TORCH_CHECK(w.size(1) == k && xs.numel() == m && ws.numel() == channels, "gpuk: fp8_linear operand shapes do not match");
     TORCH_CHECK(xs.scalar_type() == at::kFloat && ws.scalar_type() == at::kFloat && xs.is_contiguous() && ws.is_contiguous(), "gpuk: fp8_linear takes contiguous fp32 scales");
-    TORCH_CHECK(xs.is_cuda() && ws.is_cuda(), "gpuk: fp8_linear takes CUDA scales");
+    TORCH_CHECK(reachable(xs) && reachable(ws), "gpuk: fp8_linear takes CUDA scales");
     const int packed = PyObject_IsTrue(args[5]);
     if (packed < 0) throw python_error();
     const int64_t split = int_arg(args[6]);
     Tensor out;
     if (args[4] != Py_None) {
         out = tensor_arg(args[4], "out");
-        TORCH_CHECK(out.is_cuda() && out.scalar_type() == at::kBFloat16 && out.dim() == 2 && out.size(0) == m && out.size(1) == channels && out.is_contiguous(),
+        TORCH_CHECK(reachable(out) && out.scalar_type() == at::kBFloat16 && out.dim() == 2 && out.size(0) == m && out.size(1) == channels && out.is_contiguous(),
                     "gpuk: fp8_linear writes a contiguous bf16 [tokens, n] tensor");
     }
     TORCH_CHECK(m <= INT_MAX && channels <= INT_MAX && k <= INT_MAX && split >= 0 && split <= INT_MAX, "gpuk: fp8_linear sizes out of range");
@@ -302,7 +304,8 @@ PyObject *fp8_linear(PyObject *, PyObject *const *args, Py_ssize_t n) {
         NoGil unlocked;
         c10::cuda::CUDAGuard guard(x.device());
         if (!out.defined()) out = empty_like_on(x, {m, channels}, at::kBFloat16);
-        TORCH_CHECK(gpuk_fp8_linear_skinny(x.data_ptr(), xs.data_ptr<float>(), w.data_ptr(), ws.data_ptr<float>(), out.data_ptr(), static_cast<int>(m),
+        const Tensor here = w.is_cuda() ? w : w.to(x.device());
+        TORCH_CHECK(gpuk_fp8_linear_skinny(x.data_ptr(), xs.data_ptr<float>(), here.data_ptr(), ws.data_ptr<float>(), out.data_ptr(), static_cast<int>(m),
                                            static_cast<int>(channels), static_cast<int>(k), packed, static_cast<int>(split), stream_of(x)) == GPUK_OK,
                     gpuk_last_error());
     }

@@ -85,3 +85,17 @@ def test_fp8_linear_refuses_before_any_launch():
             gpuk.fp8_linear(x, s, w, c, out)
     with pytest.raises(RuntimeError, match="k_split"):
         gpuk.fp8_linear(x, s, w, c, k_split=3)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m", [8, 20])
+def test_fp8_linear_takes_pinned_host_memory(m):
+    """Scales, weights and results that the GPU reaches over the link."""
+    g = torch.Generator().manual_seed(m)
+    x, w = (torch.randn(m, 256, generator=g) * 50).to(torch.float8_e4m3fn).cuda(), (torch.randn(128, 256, generator=g) * 50).to(torch.float8_e4m3fn)
+    s, c = torch.rand(m, generator=g), torch.rand(128, generator=g)
+    want = gpuk.fp8_linear(x, s.cuda(), w.cuda(), c.cuda())
+    out = torch.zeros(m, 128, dtype=torch.bfloat16).pin_memory()
+    assert gpuk.fp8_linear(x, s.pin_memory(), w.pin_memory(), c.pin_memory(), out) is not None
+    torch.cuda.synchronize()
+    assert torch.equal(out, want.cpu())
