@@ -106,8 +106,10 @@ def test_swiglu(m, f, k, fp8):
     a, b = y.bfloat16().double().split(f, -1)
     want = (a / (1 + torch.exp(-a))).bfloat16().double() * b
     assert bool(((got.double() - want).abs() <= 4 * 2.0 ** -8 * want.abs() + 1e-5).all())
-    if m > 8 or not fp8:      # the projection's parts of k may be cut elsewhere: a step apart in a few places, no more
-        same = _native.silu_mul(_streamed(*ops))
+    same = _native.silu_mul(_streamed(*ops))
+    if m > 8 or not fp8:      # the same parts of k
+        assert torch.equal(got.view(torch.int16), same.view(torch.int16))
+    else:                     # cut elsewhere: a step apart in a few places, no more
         assert float((got.view(torch.int16) == same.view(torch.int16)).float().mean()) > 0.99
 
 
@@ -122,14 +124,53 @@ def test_qkv_rope(batch, t, heads, kv, k, positions, fp8):
     freqs = torch.outer(torch.arange(80).float(), 1.0 / (10000.0 ** (torch.arange(0, 128, 2).float() / 128)))
     cos, sin, pos = freqs.cos().cuda(), freqs.sin().cuda(), torch.tensor(positions).cuda()
     caches = [torch.randn(batch + 1, kv, 40, 128, generator=g).bfloat16().cuda() for _ in range(2)]
-    mine = [c.clone() for c in caches]
+    start, mine = [c.clone() for c in caches], [c.clone() for c in caches]
     q = _native.qkv_rope(*ops, cos, sin, pos, *mine, heads)
     _status_ok()
     want = _native.rope_append(_streamed(*ops), cos, sin, pos, *caches, heads)
-    for a, b in zip((q, *mine), (want, *caches)):
-        # sums in another order of k: a projection may fall one bf16 step aside, and a rotated pair with it by the larger of the two
-        scale = float(b.float().abs().max())
-        assert float((a.float() - b.float()).abs().max()) <= 2.0 ** -7 * scale and float((a == b).float().mean()) > 0.99
+    written = pos % 40
+    for c, s in zip(mine, start):      # nothing but the sequences' own positions
+        left = c.clone()
+        left[:batch, :, written] = s[:batch, :, written]
+        assert torch.equal(left, s)
+    for a, b in zip((q, *(c[:batch, :, written] for c in mine)), (want, *(c[:batch, :, written] for c in caches))):
+        if batch * t > 8 or not fp8:      # the same parts of k
+            assert torch.equal(a, b)
+        else:      # sums in another order of k: a projection may fall one bf16 step aside, and a rotated pair with it by the larger of the two
+            assert float((a.float() - b.float()).abs().max()) <= 2.0 ** -7 * float(b.float().abs().max()) and float((a == b).float().mean()) > 0.99
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("fp8", [False, True])
+@pytest.mark.parametrize("k_split", [1, 2, 8])
+@pytest.mark.parametrize("m", [3, 16, 27])
+def test_epilogues_round_as_the_separate_calls(m, k_split, fp8):
+    """The same parts of k on both sides: the same bits."""
+    k, heads, kv = 2048 + 64, 4, 2
+    g = torch.Generator().manual_seed(m)
+    n = (heads + 2 * kv) * 128
+    x, xs, w, ws = _fused_operands(m, n, k, fp8, g)
+    scales = (_ptr(xs), _ptr(ws)) if fp8 else (None, None)
+
+    def projection():
+        out = torch.empty(m, n, dtype=torch.bfloat16, device="cuda")
+        if fp8:      # so many channels that few tokens go to this kernel too
+            reps = -(-((12 << 20) + 1) // w.numel()) if m <= 8 else 1
+            return gpuk.fp8_linear(x, xs, w.repeat(reps, 1), ws.repeat(1, reps), k_split=k_split)[:, :n].contiguous()
+        cabi.check(cabi.lib.gpuk_linear_skinny(_ptr(x), _ptr(w), _ptr(out), m, n, k, k_split, _stream()))
+        return out
+    y = projection()
+    act = torch.empty(m, n // 2, dtype=torch.bfloat16, device="cuda")
+    cabi.check(cabi.lib.gpuk_swiglu_skinny(_ptr(x), scales[0], _ptr(w), scales[1], _ptr(act), m, n, k, k_split, _stream()))
+    assert torch.equal(act, _native.silu_mul(y))
+    cos, sin, pos = torch.randn(80, 64, generator=g).cuda(), torch.randn(80, 64, generator=g).cuda(), torch.tensor([17], device="cuda")
+    caches = [torch.zeros(m, kv, 40, 128, dtype=torch.bfloat16, device="cuda") for _ in range(4)]
+    q = torch.empty(m, heads * 128, dtype=torch.bfloat16, device="cuda")
+    cabi.check(cabi.lib.gpuk_qkv_rope_skinny(_ptr(x), scales[0], _ptr(w), scales[1], _ptr(cos), _ptr(sin), _ptr(pos), _ptr(q), _ptr(caches[0]), _ptr(caches[1]), m, 1, heads, kv, k,
+                                             80, 40, k_split, _stream()))
+    _status_ok()
+    assert torch.equal(q, _native.rope_append(y, cos, sin, pos, caches[2], caches[3], heads))
+    assert torch.equal(caches[0], caches[2]) and torch.equal(caches[1], caches[3])
 
 
 def _position_reported_once():

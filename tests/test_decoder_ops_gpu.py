@@ -80,3 +80,11 @@ def test_silu_mul_at_the_ends_of_a_chunk_and_of_the_range(rows, f):
     want, got = F.silu(a) * b, _native.silu_mul(x)
     nan = want.isnan()
     assert torch.equal(got.isnan(), nan) and torch.equal(got[~nan].view(torch.int16), want[~nan].view(torch.int16))
+
+
+def test_silu_of_every_bf16():
+    """All 65536 inputs times one: the bits of the operator, NaN where it is."""
+    a = torch.arange(-32768, 32768, dtype=torch.int32).to(torch.int16).view(torch.bfloat16).cuda()
+    got, want = _native.silu_mul(torch.cat([a, torch.ones_like(a)]).view(1, -1))[0], F.silu(a) * torch.ones_like(a)
+    nan = want.isnan()
+    assert torch.equal(got.isnan(), nan) and torch.equal(got[~nan].view(torch.int16), want[~nan].view(torch.int16))
