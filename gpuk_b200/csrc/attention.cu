@@ -334,21 +334,21 @@ extern "C" int gpuk_decode_attention(const void *q, const void *k_cache, const v
     if (batch == 0) return GPUK_OK;
     if (!q || !k_cache || !v_cache || !out) return set_last_error(GPUK_ERR_INVALID_ARGUMENT, "decode_attention: null pointer");
     if (!aligned16(q) || !aligned16(k_cache) || !aligned16(v_cache) || (reinterpret_cast<uintptr_t>(out) & 7u)) return set_last_error(GPUK_ERR_INVALID_ARGUMENT, "decode_attention: pointers must be 16-byte aligned (out: 8)");
-    int sms = 0, *status = nullptr;
-    const int rc = decode_device(&sms, &status);
+    const DecodeDevice *d = nullptr;
+    const int rc = decode_device(&d);
     if (rc != GPUK_OK) return rc;
     const int64_t pairs = static_cast<int64_t>(batch) * kv_heads;
     // up to two CTAs per SM, at least 64 keys each: 1 x 2049 keys, 8 kv heads: 1 part 19.0 us, 2 12.4, 4 8.8, 8 7.0; 4 x 129, 4 kv heads: 3.4, 3.8, 3.4, 4.3;
     // more CTAs than fit at once cost more than they give (16 x 513, 4 kv heads: 4 parts 8.0 us, 8 13.3)
     if (splits == 0) {
         splits = 1;
-        while (splits < 8 && pairs * splits * 2 <= 2 * sms && len > 64 * splits) splits *= 2;
+        while (splits < 8 && pairs * splits * 2 <= 2 * d->sms && len > 64 * splits) splits *= 2;
     }
     if (pairs * splits > 0x7fffffffll) return set_last_error(GPUK_ERR_UNSUPPORTED, "decode_attention: too many sequences");
     DecodeAttentionParams p = {static_cast<const bf16 *>(q), static_cast<const bf16 *>(k_cache), static_cast<const bf16 *>(v_cache), static_cast<bf16 *>(out),
-                               kv_heads, heads / kv_heads, len, max_seq, splits, 1.4426950408889634f / std::sqrt(static_cast<float>(kHeadDim)), status};
+                               kv_heads, heads / kv_heads, len, max_seq, splits, 1.4426950408889634f / std::sqrt(static_cast<float>(kHeadDim)), d->status};
     void *args[] = {&p};
-    const bool deep = pairs * splits <= sms && len > splits * kWarps * kBlockKeys * 2;
+    const bool deep = pairs * splits <= d->sms && len > splits * kWarps * kBlockKeys * 2;
     const void *fn = deep ? reinterpret_cast<const void *>(&decode_attention_kernel<kDeepStages>) : reinterpret_cast<const void *>(&decode_attention_kernel<kStages>);
     const cudaError_t e = launch_kernel(fn, static_cast<int>(pairs) * splits, kThreads, splits, false, args, static_cast<cudaStream_t>(stream),
                                         ring_bytes(deep ? kDeepStages : kStages));

@@ -92,16 +92,17 @@ cudaError_t gpuk::launch_kernel(const void *fn, int grid, int threads, int clust
     return cudaLaunchKernelExC(&cfg, fn, args);
 }
 
-cudaError_t gpuk::resident_ctas(const void *fn, int threads, int cluster, int sm_count, int64_t *ctas) {
+cudaError_t gpuk::resident_ctas(const void *fn, int threads, int cluster, int sm_count, int64_t *ctas, size_t dynamic_smem) {
     if (cluster <= 1) {
         int per_sm = 0;
-        cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, 0);
+        cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, dynamic_smem);
         *ctas = static_cast<int64_t>(per_sm) * sm_count;
         return e;
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(cluster * sm_count);
     cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = dynamic_smem;
     cudaLaunchAttribute attr;
     attr.id = cudaLaunchAttributeClusterDimension;
     attr.val.clusterDim.x = cluster;

@@ -131,11 +131,11 @@ extern "C" int gpuk_rope_append(const void *qkv, const float *cos, const float *
     if (!qkv || !cos || !sin || !pos || !q_out || !k_cache || !v_cache) return set_last_error(GPUK_ERR_INVALID_ARGUMENT, "rope_append: null pointer");
     if (!aligned16(qkv) || !aligned16(cos) || !aligned16(sin) || !aligned16(q_out) || !aligned16(k_cache) || !aligned16(v_cache))
         return set_last_error(GPUK_ERR_INVALID_ARGUMENT, "rope_append: pointers must be 16-byte aligned");
-    int sms = 0, *status = nullptr;
-    const int rc = decode_device(&sms, &status);
+    const DecodeDevice *d = nullptr;
+    const int rc = decode_device(&d);
     if (rc != GPUK_OK) return rc;
     RopeParams p = {static_cast<const bf16 *>(qkv), cos, sin, pos, static_cast<bf16 *>(q_out), static_cast<bf16 *>(k_cache), static_cast<bf16 *>(v_cache),
-                    static_cast<int64_t>(batch) * t * (heads + 2 * kv_heads) * (head_dim / kRopeVec), status + kStatusPosition, t, heads, kv_heads, head_dim, table_rows, max_seq};
+                    static_cast<int64_t>(batch) * t * (heads + 2 * kv_heads) * (head_dim / kRopeVec), d->status + kStatusPosition, t, heads, kv_heads, head_dim, table_rows, max_seq};
     const int64_t grid = (p.total + kThreads - 1) / kThreads;
     if (grid > 0x7fffffffll) return set_last_error(GPUK_ERR_UNSUPPORTED, "rope_append: too many rows");
     void *args[] = {&p};

@@ -256,35 +256,34 @@ __global__ void pack_weight_kernel(const uint4 *w, uint4 *packed, int n, int k) 
     }
 }
 
-int *g_status_by_device[64] = {};   // the address of decode_status on each GPU, set by the first call on it
-int g_sms_by_device[64] = {};
+DecodeDevice g_devices[64] = {};      // `status`: set by the first call on a device, last
 
 }  // namespace
 }  // namespace gpuk
 
 int gpuk::fp8_frags_per_warp_tuning = 0;
 
-int gpuk::decode_device(int *sms, int **status) {
+int gpuk::decode_device(const DecodeDevice **out) {
     int device = 0;
     if (cudaGetDevice(&device) != cudaSuccess) return set_last_error(GPUK_ERR_CUDA, "no current device");
     if (device < 0 || device >= 64) return set_last_error(GPUK_ERR_UNSUPPORTED, "device index %d", device);
     // guarded for concurrent callers
     static std::mutex init_mutex;
     std::lock_guard<std::mutex> lock(init_mutex);
-    if (!g_status_by_device[device]) {
+    DecodeDevice &d = g_devices[device];
+    if (!d.status) {
         void *word = nullptr;
         cudaError_t e = cudaGetSymbolAddress(&word, decode_status);
+        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&d.sms, cudaDevAttrMultiProcessorCount, device);
         for (const void *fn : {reinterpret_cast<const void *>(&fp8_linear_skinny_kernel<1>), reinterpret_cast<const void *>(&fp8_linear_skinny_kernel<2>)})
             if (e == cudaSuccess) e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
-        if (e == cudaSuccess) e = stream_linear_setup();
+        if (e == cudaSuccess) e = stream_linear_setup(&d);
         if (e == cudaSuccess) e = decode_attention_setup();
         if (e == cudaSuccess) e = prefill_attention_setup();
-        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&g_sms_by_device[device], cudaDevAttrMultiProcessorCount, device);
         if (e != cudaSuccess) return set_last_error(GPUK_ERR_CUDA, "cannot prepare the kernels of a decode step: %s", cudaGetErrorString(e));
-        g_status_by_device[device] = static_cast<int *>(word);
+        d.status = static_cast<int *>(word);
     }
-    *sms = g_sms_by_device[device];
-    *status = g_status_by_device[device];
+    *out = &d;
     return GPUK_OK;
 }
 
@@ -303,21 +302,21 @@ extern "C" int gpuk_fp8_linear_skinny(const void *x_fp8, const float *x_scale, c
     if (w_layout != 0 && w_layout != 1) return set_last_error(GPUK_ERR_INVALID_ARGUMENT, "fp8_linear: w_layout must be 0 (row-major) or 1 (blocked)");
     if (k_split != 0 && k_split != 1 && k_split != 2 && k_split != 4 && k_split != 8)
         return set_last_error(GPUK_ERR_INVALID_ARGUMENT, "fp8_linear: k_split must be 0, 1, 2, 4 or 8");
-    int sms = 0, *status = nullptr;
-    const int rc = decode_device(&sms, &status);
+    const DecodeDevice *d = nullptr;
+    const int rc = decode_device(&d);
     if (rc != GPUK_OK) return rc;
     if (m > kTokens || (!fp8_frags_per_warp_tuning && static_cast<int64_t>(n) * k > kWarpMaxBytes)) {
-        StreamLinearCall c = {x_fp8, x_scale, w_scale, w_fp8, out_bf16, m, n, k, w_layout == 1, kPlain, {}, k_split, sms};
-        return stream_linear(c, status, static_cast<cudaStream_t>(stream));
+        StreamLinearCall c = {x_fp8, x_scale, w_scale, w_fp8, out_bf16, m, n, k, w_layout == 1, kPlain, {}, k_split};
+        return stream_linear(c, *d, static_cast<cudaStream_t>(stream));
     }
     // split k as far as the whole grid still runs as one wave (two CTAs per SM) and every part keeps a few steps
     int ks = k_split;
     if (ks == 0) {
         ks = 1;
-        while (ks < 8 && (n / kTileN) * ks * 2 <= 2 * sms && k / kStepBytes >= 8 * ks) ks *= 2;
+        while (ks < 8 && (n / kTileN) * ks * 2 <= 2 * d->sms && k / kStepBytes >= 8 * ks) ks *= 2;
     }
     Fp8LinearParams p = {static_cast<const uint8_t *>(x_fp8), x_scale, static_cast<const uint8_t *>(w_fp8), w_scale,
-                         static_cast<__nv_bfloat16 *>(out_bf16), m, n, k, ks, w_layout, status};
+                         static_cast<__nv_bfloat16 *>(out_bf16), m, n, k, ks, w_layout, d->status};
     const int fr = fp8_frags_per_warp_tuning ? fp8_frags_per_warp_tuning : n >= 2048 ? 2 : 1;
     const void *fn = fr == 2 ? reinterpret_cast<const void *>(&fp8_linear_skinny_kernel<2>) : reinterpret_cast<const void *>(&fp8_linear_skinny_kernel<1>);
     void *args[] = {&p};
@@ -341,12 +340,12 @@ extern "C" int gpuk_fp8_pack_weight(const void *w_fp8, void *packed, int n, int 
 extern "C" int gpuk_fp8_linear_status(void) {
     int device = 0;
     if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64) return set_last_error(GPUK_ERR_CUDA, "fp8_linear: no current device");
-    if (!g_status_by_device[device]) return GPUK_OK;     // no call on this device yet
+    if (!g_devices[device].status) return GPUK_OK;     // no call on this device yet
     int v[kDecodeStatusWords] = {};
     cudaError_t e = cudaDeviceSynchronize();
-    if (e == cudaSuccess) e = cudaMemcpy(v, g_status_by_device[device], sizeof(v), cudaMemcpyDeviceToHost);
+    if (e == cudaSuccess) e = cudaMemcpy(v, g_devices[device].status, sizeof(v), cudaMemcpyDeviceToHost);
     // a position is the caller's mistake and is reported once; a launch that went wrong stays on record
-    if (e == cudaSuccess && v[kStatusPosition]) e = cudaMemset(g_status_by_device[device] + kStatusPosition, 0, sizeof(int));
+    if (e == cudaSuccess && v[kStatusPosition]) e = cudaMemset(g_devices[device].status + kStatusPosition, 0, sizeof(int));
     if (e != cudaSuccess) return set_last_error(GPUK_ERR_CUDA, "fp8_linear: cannot read the status words: %s", cudaGetErrorString(e));
     if (v[0]) return set_last_error(GPUK_ERR_BAD_LAUNCH, "fp8_linear: a launch ran without its planned thread-block cluster and wrote nothing, or gave up a wait");
     if (v[kStatusPosition]) return set_last_error(GPUK_ERR_INVALID_ARGUMENT, "decoder: a position outside the KV cache or the table of angles; its keys and values were not written, its queries are NaN");

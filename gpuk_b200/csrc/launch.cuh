@@ -29,7 +29,7 @@ struct ArShape {
 cudaError_t launch_kernel(const void *fn, int grid, int threads, int cluster, bool all_resident, void **args, cudaStream_t stream,
                           size_t dynamic_smem = 0);
 // CTAs of `fn` that can be resident on the whole GPU at once, counting whole clusters only.
-cudaError_t resident_ctas(const void *fn, int threads, int cluster, int sm_count, int64_t *ctas);
+cudaError_t resident_ctas(const void *fn, int threads, int cluster, int sm_count, int64_t *ctas, size_t dynamic_smem = 0);
 
 template <typename T>
 cudaError_t launch_norm_quant(const NormQuantParams &p, int vpt, int threads, int grid, cudaStream_t stream);

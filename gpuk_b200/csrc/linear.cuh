@@ -26,16 +26,22 @@ struct StreamLinearCall {
     LinearEpilogue epilogue;                // kSwiGlu: out [m, n / 2] = silu(first half) * second half; kRopeAppend: out [m, heads * 128], keys and values to the caches
     RopeCall rope;
     int ks;                                 // CTAs that share a tile (0: chosen from the shape)
-    int sms;
 };
-cudaError_t stream_linear_setup();          // once per device
+// A device as the kernels of a decode step plan for it.
+struct DecodeDevice {
+    int sms;
+    // The status words that the kernels set (gpuk_fp8_linear_status): the first where a launch went wrong, the one at kStatusPosition where a position pointed
+    // outside the cache or the table of angles.
+    int *status;
+    // CTAs that run at once in clusters of a given size: fewer than SMs times CTAs per SM, by what does not divide the groups of SMs that clusters stay in
+    int stream_ctas[2][9];                  // streaming linear layer with 16 and 32 columns, k split
+};
+cudaError_t stream_linear_setup(DecodeDevice *d);          // once per device
 cudaError_t decode_attention_setup();
 cudaError_t prefill_attention_setup();
-// The current device's SMs and the status words that kernels of a decode step set (gpuk_fp8_linear_status): the first where a launch went wrong, the
-// one at kStatusPosition where a position pointed outside the cache or the table of angles.  The first call on a device
-// opts the kernels in to their shared memory, so that no later call has set-up left to do.
 constexpr int kStatusPosition = 1, kDecodeStatusWords = 2;
-int decode_device(int *sms, int **status);
-int stream_linear(const StreamLinearCall &c, int *status, cudaStream_t stream);
+// The current device; the first call on it opts the kernels in to their shared memory, so that no later call has set-up left to do.
+int decode_device(const DecodeDevice **device);
+int stream_linear(const StreamLinearCall &c, const DecodeDevice &d, cudaStream_t stream);
 
 }  // namespace gpuk

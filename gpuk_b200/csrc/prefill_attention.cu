@@ -308,8 +308,8 @@ extern "C" int gpuk_prefill_attention(const void *q, const void *k_cache, const 
     if (batch == 0 || t == 0) return GPUK_OK;
     if (!q || !k_cache || !v_cache || !pos || !out) return set_last_error(GPUK_ERR_INVALID_ARGUMENT, "prefill_attention: null pointer");
     if (!aligned16(q) || !aligned16(k_cache) || !aligned16(v_cache) || !aligned16(out)) return set_last_error(GPUK_ERR_INVALID_ARGUMENT, "prefill_attention: pointers must be 16-byte aligned");
-    int sms = 0, *status = nullptr;
-    const int rc = decode_device(&sms, &status);
+    const DecodeDevice *d = nullptr;
+    const int rc = decode_device(&d);
     if (rc != GPUK_OK) return rc;
     const int tiles = (t + kTiles * kTile - 1) / (kTiles * kTile);
     const int64_t rows = static_cast<int64_t>(batch) * t, ctas = static_cast<int64_t>(batch) * heads * tiles;
@@ -323,7 +323,7 @@ extern "C" int gpuk_prefill_attention(const void *q, const void *k_cache, const 
     if (!e) e = encode_map(&kmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, k_cache, 3, kv_sizes, kv_strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
     if (!e) e = encode_map(&vmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, v_cache, 3, kv_sizes, kv_strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
     if (e) return set_last_error(GPUK_ERR_CUDA, "prefill_attention: the driver refused a tensor map (%d)", e);
-    PrefillAttentionParams p = {pos, static_cast<const bf16 *>(q), static_cast<bf16 *>(out), t, heads, kv_heads, len, tiles, batch * heads, 1.4426950408889634f / std::sqrt(static_cast<float>(kHeadDim)), status};
+    PrefillAttentionParams p = {pos, static_cast<const bf16 *>(q), static_cast<bf16 *>(out), t, heads, kv_heads, len, tiles, batch * heads, 1.4426950408889634f / std::sqrt(static_cast<float>(kHeadDim)), d->status};
     void *args[] = {&qmap, &kmap, &vmap, &p};
     const cudaError_t err = launch_kernel(reinterpret_cast<const void *>(&prefill_attention_kernel), static_cast<int>(ctas), kThreads, 1, false, args,
                                           static_cast<cudaStream_t>(stream), kSmemBytes);

@@ -51,11 +51,9 @@ constexpr int kThreads = 128;            // warp 0 issues copies, warp 1 multipl
 constexpr int kStep = 128;               // bytes of k per pipeline step
 constexpr int kWBytes = kTileRows * kStep;
 constexpr int kAcc = 4;                  // accumulators the steps take turns with: shorter chains of rounded sums
-constexpr int kRingMax = 11;
+constexpr int kRingMax = 6;              // steps of the deepest ring
 constexpr int kPitch = kTileRows + 4;    // floats per token in the partial tile
 constexpr int kMaxTokens = 32;
-
-constexpr int kMaxSmem = 220 * 1024;     // of the ring
 
 enum Weights { kFp8Blocked, kFp8Rows, kBf16Rows };
 
@@ -278,6 +276,13 @@ __global__ void __launch_bounds__(kThreads, 2) stream_linear_kernel(const __grid
 }
 
 
+// Never launched: asked how many CTAs of the streaming kernel's size run at once, since the answer for a kernel with tensor memory is one per SM.
+__global__ void __launch_bounds__(kThreads) yardstick_kernel() {}
+
+// Steps in the ring of a CTA.  Where k is not split six keep more in flight; four leave room for a third CTA and for the next kernel's (1280 x 8192: 6.8 / 7.3 us with
+// 4 / 8, and 22528 x 4096 in two parts of k, 16 tokens: 30.1 us, where rings of six, for which there is no third CTA, took 36.5).
+int ring_stages(int columns, bool split, int tiles, int sms) { return columns == 32 ? 5 : split || tiles <= sms ? 4 : kRingMax; }
+
 template <int W, int EPI>
 const void *kernel_for(int columns) {
     return columns == 16 ? reinterpret_cast<const void *>(&stream_linear_kernel<W, 16, EPI>) : reinterpret_cast<const void *>(&stream_linear_kernel<W, 32, EPI>);
@@ -292,18 +297,29 @@ const void *kernel_of(int w, int epilogue, int columns) {
 
 }  // namespace
 
-cudaError_t stream_linear_setup() {
+cudaError_t stream_linear_setup(DecodeDevice *d) {
+    for (int columns = 16; columns <= kMaxTokens; columns += 16) {
+        const int smem = smem_bytes(columns, ring_stages(columns, true, 0, d->sms)) + 256;      // barriers and such
+        const void *fn = reinterpret_cast<const void *>(&yardstick_kernel);
+        cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        for (int ks = 1; ks <= 8 && e == cudaSuccess; ++ks) {
+            int64_t ctas = 0;
+            e = resident_ctas(fn, kThreads, ks, d->sms, &ctas, smem);
+            d->stream_ctas[columns / 32][ks] = static_cast<int>(ctas);
+        }
+        if (e != cudaSuccess) return e;
+    }
     for (int columns = 16; columns <= kMaxTokens; columns += 16)
         for (int w : {kFp8Blocked, kFp8Rows, kBf16Rows})
             for (int epilogue : {kPlain, kSwiGlu, kRopeAppend}) {
                 const cudaError_t e = cudaFuncSetAttribute(kernel_of(w, epilogue, columns), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                           smem_bytes(columns, kMaxSmem / (kWBytes + columns * kStep)));
+                                                           smem_bytes(columns, kRingMax));
                 if (e != cudaSuccess) return e;
             }
     return cudaSuccess;
 }
 
-int stream_linear(const StreamLinearCall &c, int *status, cudaStream_t stream) {
+int stream_linear(const StreamLinearCall &c, const DecodeDevice &d, cudaStream_t stream) {
     const int columns = c.m <= 16 ? 16 : 32, es = c.x_scale ? 1 : 2;
     CUtensorMap wmap, xmap;
     const CUtensorMapDataType type = es == 1 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
@@ -325,21 +341,19 @@ int stream_linear(const StreamLinearCall &c, int *status, cudaStream_t stream) {
     }
     if (rc) return set_last_error(GPUK_ERR_CUDA, "linear: the driver refused the tensor map (%d)", rc);
     const int tiles = c.n / kTileRows, steps = static_cast<int>((row + kStep - 1) / kStep);
-    // Parts of k: as many as give one wave of CTAs (three per SM with 16 columns, two with 32), 1 or an even number or 3 (5 and 7 leave clusters
-    // badly packed), as long as a part keeps enough steps to pay for its start: 8 tokens, 2048 x 2048 in 16 steps: 1 part 6.9 us, 2 5.3,
-    // 4 4.2, 8 4.7; 64 steps: 1280 x 8192 1 20.9, 4 8.2, 8 6.6, 10240 x 8192 with 32 tokens 1 24.0, 2 18.5, 3 17.2, 4 24.2.
+    // Parts of k: as many as run at once in clusters of that size (6144 x 8192, 24 tokens: 6 parts, whose 48 clusters do not all fit, 26.6 us, 5 18.7, 4 19.7), 5 and 7 only
+    // where they leave a tenth of the places free (7168 x 4096: 5 14.4, 4 13.5), as long as a part keeps enough steps to pay for its start: 8 tokens, 2048 x 2048 in 16
+    // steps: 1 part 6.9 us, 2 5.3, 4 4.2, 8 4.7; 64 steps: 1280 x 8192 1 20.9, 4 8.2, 8 6.6, 10240 x 8192 with 32 tokens 1 24.0, 2 18.5, 3 17.2, 4 24.2.
     int ks = c.ks;
     if (ks == 0) {
-        const int most = steps >= 32 ? 8 : steps < 8 ? 1 : tiles * 4 <= c.sms * 7 / 5 ? 4 : 2, slots = (columns == 16 ? 3 : 2) * c.sms;
-        for (ks = most; ks > 1 && (tiles * ks > slots || ks == 5 || ks == 7); --ks) {}
+        const int most = steps >= 32 ? 8 : steps < 8 ? 1 : tiles * 4 <= d.sms * 7 / 5 ? 4 : 2, *fit = d.stream_ctas[columns / 32];
+        for (ks = most; ks > 1 && tiles * ks > (ks == 5 || ks == 7 ? fit[ks] * 9 / 10 : fit[ks]); --ks) {}
     }
     const int part_steps = (steps + ks - 1) / ks;
-    // six stages keep more in flight where k is not split; four leave room for the next kernel's CTAs (1280 x 8192: 6.8 / 7.3 us with 4 / 8)
-    int stages = columns == 16 ? (tiles <= c.sms ? 4 : 6) : 5;
-    stages = std::max(1, std::min({stages, part_steps, kRingMax}));
+    const int stages = std::max(1, std::min(ring_stages(columns, ks > 1, tiles, d.sms), part_steps));
     const int smem = std::max(smem_bytes(columns, stages), 1024 + columns * kPitch * 4);
     const bool vec = ((reinterpret_cast<uintptr_t>(c.out) & 7u) | (reinterpret_cast<uintptr_t>(c.w_scale) & 15u)) == 0;
-    StreamParams p = {c.x_scale, c.w_scale, static_cast<bf16 *>(c.out), c.m, c.n, steps, stages, ks, vec, c.rope, status};
+    StreamParams p = {c.x_scale, c.w_scale, static_cast<bf16 *>(c.out), c.m, c.n, steps, stages, ks, vec, c.rope, d.status};
     const void *fn = kernel_of(es == 2 ? kBf16Rows : c.blocked ? kFp8Blocked : kFp8Rows, c.epilogue, columns);
     void *args[] = {&wmap, &xmap, &p};
     const cudaError_t e = launch_kernel(fn, tiles * ks, kThreads, ks, false, args, stream, smem);
@@ -362,19 +376,19 @@ static int run_skinny(const char *what, StreamLinearCall c, void *stream) {
     if (c.m == 0) return GPUK_OK;
     if (!c.x || !c.w || !c.out || !c.x_scale != !c.w_scale) return set_last_error(GPUK_ERR_INVALID_ARGUMENT, "%s: null pointer", what);
     if ((reinterpret_cast<uintptr_t>(c.x) | reinterpret_cast<uintptr_t>(c.w)) & 15u) return set_last_error(GPUK_ERR_INVALID_ARGUMENT, "%s: operands must be 16-byte aligned", what);
-    int *status = nullptr;
-    const int rc = decode_device(&c.sms, &status);
-    return rc != GPUK_OK ? rc : stream_linear(c, status, static_cast<cudaStream_t>(stream));
+    const DecodeDevice *d = nullptr;
+    const int rc = decode_device(&d);
+    return rc != GPUK_OK ? rc : stream_linear(c, *d, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int gpuk_linear_skinny(const void *x_bf16, const void *w_bf16, void *out_bf16, int m, int n, int k, int k_split, void *stream) {
-    return run_skinny("linear", {x_bf16, nullptr, nullptr, w_bf16, out_bf16, m, n, k, false, kPlain, {}, k_split, 0}, stream);
+    return run_skinny("linear", {x_bf16, nullptr, nullptr, w_bf16, out_bf16, m, n, k, false, kPlain, {}, k_split}, stream);
 }
 
 extern "C" int gpuk_swiglu_skinny(const void *x, const float *x_scale, const void *w, const float *w_scale, void *out_bf16, int m, int n, int k, int k_split, void *stream) {
     if ((reinterpret_cast<uintptr_t>(out_bf16) & 7u) | (reinterpret_cast<uintptr_t>(w_scale) & 15u))
         return set_last_error(GPUK_ERR_INVALID_ARGUMENT, "swiglu: scales must be 16-byte aligned, results 8-byte");
-    return run_skinny("swiglu", {x, x_scale, w_scale, w, out_bf16, m, n, k, false, kSwiGlu, {}, k_split, 0}, stream);
+    return run_skinny("swiglu", {x, x_scale, w_scale, w, out_bf16, m, n, k, false, kSwiGlu, {}, k_split}, stream);
 }
 
 extern "C" int gpuk_qkv_rope_skinny(const void *x, const float *x_scale, const void *w, const float *w_scale, const float *cos, const float *sin, const int64_t *pos,
@@ -387,5 +401,5 @@ extern "C" int gpuk_qkv_rope_skinny(const void *x, const float *x_scale, const v
          reinterpret_cast<uintptr_t>(sin) | reinterpret_cast<uintptr_t>(w_scale)) & 15u)
         return set_last_error(GPUK_ERR_INVALID_ARGUMENT, "qkv_rope: pointers must be 16-byte aligned");
     return run_skinny("qkv_rope", {x, x_scale, w_scale, w, q_out, batch * t, (heads + 2 * kv_heads) * kTileRows, k, false, kRopeAppend,
-                                   {cos, sin, pos, k_cache, v_cache, t, heads, kv_heads, table_rows, max_seq}, k_split, 0}, stream);
+                                   {cos, sin, pos, k_cache, v_cache, t, heads, kv_heads, table_rows, max_seq}, k_split}, stream);
 }

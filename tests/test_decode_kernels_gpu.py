@@ -23,10 +23,11 @@ def _status_ok():
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("k_split", [0, 1, 3, 8])
-@pytest.mark.parametrize("m,n,k", [(1, 128, 8), (16, 256, 64), (17, 128, 72), (32, 384, 1000), (31, 1280, 4096), (9, 16384, 2048)])
+@pytest.mark.parametrize("m,n,k", [(1, 128, 8), (16, 256, 64), (17, 128, 72), (32, 384, 1000), (31, 1280, 4096), (9, 16384, 2048), (24, 6144, 2048),
+                                   (32, 4352, 4096), (4, 19072, 1024), (17, 18944, 1024)])
 def test_bf16_linear(m, n, k, k_split):
     """Tokens on both sides of the 16-column tile, k that ends inside a step (8, 72, 1000), fewer steps than parts, tiles below and above
-    the number of SMs.  fp32 sums of exact products, one rounding: one bf16 step."""
+    the number of SMs, and numbers of them that clusters of six or eight would not fit.  fp32 sums of exact products, one rounding: one bf16 step."""
     g = torch.Generator().manual_seed(m + n + k)
     x, w = torch.randn(m, k, generator=g).bfloat16(), torch.randn(n, k, generator=g).bfloat16()
     dx, dw = x.cuda(), w.cuda()
