@@ -9,7 +9,7 @@
 //     no second kernel.
 //   * a warp owns every fourth block of 16 keys of the range and fetches it by cp.async into a ring of its own
 //     (4 KiB of keys and 4 KiB of values per block), so no warp waits for another before the end.  Three blocks deep, two CTAs per SM; six deep
-//     where there are not more CTAs than SMs, so that an SM keeps 128 to 160 KiB in flight either way.  The first blocks are brought into L2
+//     where all CTAs run at once with one per SM, so that an SM keeps 128 to 160 KiB in flight either way.  The first blocks are brought into L2
 //     before griddepcontrol.wait.
 //   * scores and outputs are mma.sync.m16n8k16 with the group's heads as the 16 rows (padded), keys / head dimension as columns:
 //     the score fragment of a warp is, register for register, the operand of the second product.  A KV block of 16 keys
@@ -39,7 +39,7 @@ constexpr int kMaxGroup = 16;              // query heads per kv head: the rows 
 constexpr int kWarps = 4;
 constexpr int kThreads = kWarps * 32;
 constexpr int kBlockKeys = 16;             // keys a warp takes at a time
-constexpr int kStages = 3, kDeepStages = 6;    // ... and blocks of them in its ring: two CTAs per SM, or one where there are not more CTAs than SMs
+constexpr int kStages = 3, kDeepStages = 6;    // ... and blocks of them in its ring: two CTAs per SM, or one
 constexpr int kRowBytes = kHeadDim * 2;
 constexpr int kTileBytes = kBlockKeys * kRowBytes;           // keys or values of one block
 constexpr int ring_bytes(int stages) { return kWarps * stages * 2 * kTileBytes; }      // 96 or 192 KiB
@@ -310,14 +310,26 @@ __global__ void __launch_bounds__(kThreads, STAGES == kStages ? 2 : 1) decode_at
     cluster_barrier();      // nobody leaves while its partial results may still be read
 }
 
+const void *kernel_of(bool deep) {
+    return deep ? reinterpret_cast<const void *>(&decode_attention_kernel<kDeepStages>) : reinterpret_cast<const void *>(&decode_attention_kernel<kStages>);
+}
+int stages_of(bool deep) { return deep ? kDeepStages : kStages; }
+
 bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
 }  // namespace
 
-cudaError_t decode_attention_setup() {
-    const cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void *>(&decode_attention_kernel<kStages>), cudaFuncAttributeMaxDynamicSharedMemorySize, ring_bytes(kStages));
-    return e != cudaSuccess ? e : cudaFuncSetAttribute(reinterpret_cast<const void *>(&decode_attention_kernel<kDeepStages>), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                       ring_bytes(kDeepStages));
+cudaError_t decode_attention_setup(DecodeDevice *d) {
+    cudaError_t e = cudaSuccess;
+    for (int deep = 0; deep < 2 && e == cudaSuccess; ++deep) {
+        e = cudaFuncSetAttribute(kernel_of(deep), cudaFuncAttributeMaxDynamicSharedMemorySize, ring_bytes(stages_of(deep)));
+        for (int splits = 1; splits <= 8 && e == cudaSuccess; ++splits) {
+            int64_t ctas = 0;
+            e = resident_ctas(kernel_of(deep), kThreads, splits, d->sms, &ctas, ring_bytes(stages_of(deep)));
+            d->attention_ctas[deep][splits] = static_cast<int>(ctas);
+        }
+    }
+    return e;
 }
 
 }  // namespace gpuk
@@ -338,20 +350,21 @@ extern "C" int gpuk_decode_attention(const void *q, const void *k_cache, const v
     const int rc = decode_device(&d);
     if (rc != GPUK_OK) return rc;
     const int64_t pairs = static_cast<int64_t>(batch) * kv_heads;
-    // up to two CTAs per SM, at least 64 keys each: 1 x 2049 keys, 8 kv heads: 1 part 19.0 us, 2 12.4, 4 8.8, 8 7.0; 4 x 129, 4 kv heads: 3.4, 3.8, 3.4, 4.3;
-    // more CTAs than fit at once cost more than they give (16 x 513, 4 kv heads: 4 parts 8.0 us, 8 13.3)
+    // A cluster of parts costs about a microsecond and, from the second CTA an SM on, the overlap with the launch in front, so a part needs its keys: more than 160 in each half while
+    // every CTA has an SM to itself (4 x 129 keys, 4 kv heads: 1 part 3.2 us, 2 3.6; 32 x 300, 1: 2 parts 4.8, 8 5.8), 384 beyond (7 x 300, 8: 1 part 5.0, 4 6.3; 7 x 1000: 2 parts
+    // 10.2, 4 9.3), and all clusters have to run at once (2 x 2049, 8 kv heads, 8 parts: with the long ring, for which the
+    // 16 clusters do not fit, 13.6 us, with the short one 8.4).
     if (splits == 0) {
         splits = 1;
-        while (splits < 8 && pairs * splits * 2 <= 2 * d->sms && len > 64 * splits) splits *= 2;
+        while (splits < 8 && len > (pairs * splits * 2 <= d->sms ? 160 : 384) * splits && pairs * splits * 2 <= d->attention_ctas[0][splits * 2]) splits *= 2;
     }
     if (pairs * splits > 0x7fffffffll) return set_last_error(GPUK_ERR_UNSUPPORTED, "decode_attention: too many sequences");
     DecodeAttentionParams p = {static_cast<const bf16 *>(q), static_cast<const bf16 *>(k_cache), static_cast<const bf16 *>(v_cache), static_cast<bf16 *>(out),
                                kv_heads, heads / kv_heads, len, max_seq, splits, 1.4426950408889634f / std::sqrt(static_cast<float>(kHeadDim)), d->status};
     void *args[] = {&p};
-    const bool deep = pairs * splits <= d->sms && len > splits * kWarps * kBlockKeys * 2;
-    const void *fn = deep ? reinterpret_cast<const void *>(&decode_attention_kernel<kDeepStages>) : reinterpret_cast<const void *>(&decode_attention_kernel<kStages>);
-    const cudaError_t e = launch_kernel(fn, static_cast<int>(pairs) * splits, kThreads, splits, false, args, static_cast<cudaStream_t>(stream),
-                                        ring_bytes(deep ? kDeepStages : kStages));
+    const bool deep = pairs * splits <= d->attention_ctas[1][splits] && len > splits * kWarps * kBlockKeys * 2;
+    const cudaError_t e = launch_kernel(kernel_of(deep), static_cast<int>(pairs) * splits, kThreads, splits, false, args, static_cast<cudaStream_t>(stream),
+                                        ring_bytes(stages_of(deep)));
     if (e != cudaSuccess) return set_last_error(GPUK_ERR_CUDA, "decode_attention: launch failed: %s", cudaGetErrorString(e));
     return GPUK_OK;
 }

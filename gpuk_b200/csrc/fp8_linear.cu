@@ -278,7 +278,7 @@ int gpuk::decode_device(const DecodeDevice **out) {
         for (const void *fn : {reinterpret_cast<const void *>(&fp8_linear_skinny_kernel<1>), reinterpret_cast<const void *>(&fp8_linear_skinny_kernel<2>)})
             if (e == cudaSuccess) e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
         if (e == cudaSuccess) e = stream_linear_setup(&d);
-        if (e == cudaSuccess) e = decode_attention_setup();
+        if (e == cudaSuccess) e = decode_attention_setup(&d);
         if (e == cudaSuccess) e = prefill_attention_setup();
         if (e != cudaSuccess) return set_last_error(GPUK_ERR_CUDA, "cannot prepare the kernels of a decode step: %s", cudaGetErrorString(e));
         d.status = static_cast<int *>(word);

@@ -35,9 +35,10 @@ struct DecodeDevice {
     int *status;
     // CTAs that run at once in clusters of a given size: fewer than SMs times CTAs per SM, by what does not divide the groups of SMs that clusters stay in
     int stream_ctas[2][9];                  // streaming linear layer with 16 and 32 columns, k split
+    int attention_ctas[2][9];               // decode attention with the short and the long ring
 };
 cudaError_t stream_linear_setup(DecodeDevice *d);          // once per device
-cudaError_t decode_attention_setup();
+cudaError_t decode_attention_setup(DecodeDevice *d);
 cudaError_t prefill_attention_setup();
 constexpr int kStatusPosition = 1, kDecodeStatusWords = 2;
 // The current device; the first call on it opts the kernels in to their shared memory, so that no later call has set-up left to do.

@@ -216,7 +216,7 @@ def test_positions_outside_the_cache_or_the_table(table_rows, bad, fused, fp8):
 @pytest.mark.gpu
 @pytest.mark.parametrize("splits", [0, 1, 3, 8])
 @pytest.mark.parametrize("batch,heads,kv_heads,length,max_seq", [(1, 8, 2, 1, 1), (3, 16, 1, 17, 32), (2, 4, 4, 64, 64), (4, 16, 4, 129, 256), (5, 8, 1, 1000, 1024),
-                                                                (40, 64, 8, 80, 256)])
+                                                                (40, 64, 8, 80, 256), (16, 4, 1, 700, 704), (2, 128, 8, 1300, 1300), (9, 64, 8, 1600, 1600)])
 def test_decode_attention(batch, heads, kv_heads, length, max_seq, splits):
     """One key, ends inside a block of 16, parts of the cluster without keys, 1 to 16 query heads per kv head, both ring depths.  What lies behind
     the keys is NaN.  Probabilities are rounded to bf16 before the second product (a relative 2^-8 each, half of the last of eight bits) and
@@ -452,6 +452,20 @@ def test_native_calls_hand_back_what_the_kernels_do_not_read():
                 call(fine, bad)
     wide = flat[:2 * 4 * 136].view(2, 1, 4, 136)[..., :128]
     assert _native.decode_attention(q, wide, wide, 4) is None
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("length", [32767, 32768, 32769, 32900])
+def test_decoder_on_both_sides_of_the_library_s_attention(decoder, length):
+    """Few sequences and long contexts: the same step by the operators, up to the roundings of bf16 between them."""
+    m = decoder(max_seq_len=33024)
+    m.fill_kv_cache(length)
+    one, pos = torch.ones(2, 1, dtype=torch.long, device="cuda"), torch.tensor([length - 1], device="cuda")
+    got = m.forward(one, pos, cache_len=length)
+    _status_ok()
+    m.own_elementwise = False
+    want = m.forward(one, pos, cache_len=length)
+    assert float((got.float() - want.float()).norm()) <= 0.03 * float(want.float().norm())
 
 
 @pytest.mark.gpu
