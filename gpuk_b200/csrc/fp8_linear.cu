@@ -3,10 +3,10 @@
 // block (F.linear in model/tensor_parallel.py:66 of the reference, which has no FP8 path of its own).
 //
 // The product is a weight-streaming problem: every weight byte is read once and used for at most 32 multiply-adds.  Two kernels share
-// the work.  This one, on warp-level mma, takes at most 8 tokens on weights of up to 12 MiB: it has no tensor map, tensor memory or
+// the work.  This one, on warp-level mma, takes at most 8 tokens on weights of up to 32 MiB: it has no tensor map, tensor memory or
 // ring to set up and ends a microsecond sooner.  Beyond, its conversions (below) bound it, and the tcgen05 kernel of stream_linear.cu is the
-// faster one.  Measured, here / there, 8 tokens: 1024 x 1024 2.8 / 3.5 us, 1280 x 8192 5.4 / 6.6, 5120 x 2048 5.1 / 5.3, 4096 x 8192
-// 9.4 / 9.5 (row-major 10.9 / 9.5), 7168 x 8192 14.7 / 12.4, 57344 x 8192 82 / 73; with 16 and 32 tokens, 7168 x 8192: 15.4 / 12.6 and
+// faster one.  Measured, here / there, 8 tokens: 1024 x 1024 2.8 / 3.5 us, 1280 x 8192 5.5 / 6.6, 5120 x 2048 5.1 / 5.3, 5120 x 4096 7.6 / 7.7 (row-major 8.0 /
+// 7.7), 4096 x 8192 8.1 / 9.9 (row-major 8.5 / 9.8), 5120 x 8192 11.3 / 10.3, 57344 x 8192 82 / 73; with 16 and 32 tokens, 7168 x 8192: 15.4 / 12.6 and
 // 21.7 / 13.2.
 //
 //   * weights [n, k] (k contiguous, e4m3) are the 16-row operand of the warp-level mma and the
@@ -53,8 +53,11 @@ constexpr int kXRow = kXSteps * kStepBytes + 64;   // shared-memory row pitch; 6
 constexpr int kXBuf = kTokens * kXRow;              // one activation buffer
 constexpr int kWSlot = 2 * kThreads * 16;           // one k step of the CTA's weights: two 16-byte vectors per thread
 constexpr int kPartPitch = kTileN + 4;              // floats per token row of the partial tile (128 channels + padding)
-constexpr int kSmemBytes = kDepth * kWSlot + 2 * kXBuf;   // 64 KiB + 9 KiB: three CTAs per SM
-constexpr int64_t kWarpMaxBytes = 12 << 20;      // weights up to which this kernel is the faster one (see the entry point)
+// What a CTA uses is 73 KiB.  It asks for 100, so that two fit an SM: three leave some SMs with three CTAs and some with one (8 tokens, 4096 x 8192
+// row-major: 10.9 -> 8.6 us).
+constexpr int kSmemBytes = 100 * 1024;
+static_assert(kDepth * kWSlot + 2 * kXBuf <= kSmemBytes, "ring and activations");
+constexpr int64_t kWarpMaxBytes = 32 << 20;      // weights up to which this kernel is the faster one (see the entry point)
 constexpr int kMaxTokens = 32;     // ... of the entry point
 static_assert(kTokens * kPartPitch * 4 <= kDepth * kWSlot, "the partial tile reuses the weight ring");
 static_assert((kDepth & (kDepth - 1)) == 0 && kXSteps == kDepth, "slot and buffer arithmetic below");

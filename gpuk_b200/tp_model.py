@@ -84,7 +84,8 @@ class _Linear:
 
     def streamed(self, x: torch.Tensor):
         """The weight and its scales (None in bf16) as the streaming kernels with a fused epilogue take them, or None where the projection runs
-        elsewhere: on the CPU, in a library, or -- 8 tokens at most on small FP8 weights -- on the warp-level kernel (csrc/fp8_linear.cu)."""
+        elsewhere: on the CPU, in a library, or -- 8 tokens at most on small FP8 weights, up to where the epilogue repays the time by which the
+        streaming kernel is behind -- on the warp-level kernel (csrc/fp8_linear.cu)."""
         w = self.w_q if self.fp8 else self.weight
         if not (self.own_gemm and x.is_cuda and 0 < x.shape[0] <= 32 and self.weight.dtype == torch.bfloat16 and x.dtype == w.dtype):
             return None

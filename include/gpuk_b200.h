@@ -283,7 +283,7 @@ int gpuk_ws_set_option(gpuk_ws *ws, const char *name, int64_t value);
  * resident CTAs per SM, 0 = as many as fit).  One more name belongs to gpuk_fp8_linear_skinny:
  * "fp8_frags_per_warp" (16-row fragments a warp of its warp-level kernel multiplies per k step: 1 = eight warps per CTA, 2 = four
  * warps that convert each activation vector once for two fragments, either for all calls of at most 8 tokens; 0 = default: that kernel for
- * at most 8 tokens on weights of up to 12 MiB, with 2 fragments from 2048 output channels; the tcgen05 kernel beyond).
+ * at most 8 tokens on weights of up to 32 MiB, with 2 fragments from 2048 output channels; the tcgen05 kernel beyond).
  * Not thread-safe against concurrent calls.
  */
 int gpuk_set_tuning(const char *name, int64_t value);

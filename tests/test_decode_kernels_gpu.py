@@ -58,7 +58,7 @@ def test_more_clusters_than_tensor_memory_holds(m, k_split, fp8):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("packed", [False, True])
-@pytest.mark.parametrize("m,n,k", [(8, 1536, 8192), (8, 1664, 8192), (9, 128, 64), (16, 256, 192), (17, 256, 4160), (32, 10240, 1024)])
+@pytest.mark.parametrize("m,n,k", [(8, 1536, 8192), (8, 1664, 8192), (8, 4096, 8192), (7, 4224, 8192), (9, 128, 64), (16, 256, 192), (17, 256, 4160), (32, 10240, 1024)])
 def test_fp8_linear_around_the_dispatch(m, n, k, packed):
     """The weight size and the token count at which the entry point changes kernels, k with an odd number of 64-byte blocks, and an
     output and channel scales that are aligned for single elements only."""
@@ -90,7 +90,7 @@ def _streamed(x, xs, w, ws):
     """The projection alone, by the same kernel: `w` repeated until the entry point leaves the warp-level kernel out."""
     if xs is None:
         return _native.linear(x, w)
-    reps = 1 if x.shape[0] > 8 else -(-((12 << 20) + 1) // w.numel())
+    reps = 1 if x.shape[0] > 8 else -(-((32 << 20) + 1) // w.numel())
     return gpuk.fp8_linear(x, xs, w.repeat(reps, 1), ws.repeat(1, reps))[:, :w.shape[0]].contiguous()
 
 
@@ -156,7 +156,7 @@ def test_epilogues_round_as_the_separate_calls(m, k_split, fp8):
     def projection():
         out = torch.empty(m, n, dtype=torch.bfloat16, device="cuda")
         if fp8:      # so many channels that few tokens go to this kernel too
-            reps = -(-((12 << 20) + 1) // w.numel()) if m <= 8 else 1
+            reps = -(-((32 << 20) + 1) // w.numel()) if m <= 8 else 1
             return gpuk.fp8_linear(x, xs, w.repeat(reps, 1), ws.repeat(1, reps), k_split=k_split)[:, :n].contiguous()
         cabi.check(cabi.lib.gpuk_linear_skinny(_ptr(x), _ptr(w), _ptr(out), m, n, k, k_split, _stream()))
         return out
