@@ -96,10 +96,13 @@ __device__ __forceinline__ void norm_quant_rows(const NormQuantParams &p, Epilog
 }
 
 // The residual of a CTA's first row into L2 while the kernel in front of this one ends: a hint, it is read only after the wait.  Not the input, which
-// that kernel has usually still to write, and only where CTAs can be there that early (1024 x 8192 bf16, calls back to back: 11.4 -> 10.1 us).
-constexpr unsigned kEarlyCtas = 1184;
+// that kernel has usually still to write, and only where CTAs can be there that early (1024 x 8192 bf16, calls back to back: 11.4 -> 10.1 us).  Rows of more than 1024
+// vectors leave an SM room for a CTA or two, so that most of these would only read twice: with many rows it costs (fp32, with / without: 2500 x 6144 33.5 / 33.5 us, 7200 x
+// 6144 91.2 / 89.3, 7200 x 7680 114.5 / 111.5; few rows gain, 300 x 6144 6.7 / 7.6).
+constexpr unsigned kEarlyCtas = 1184;      // eight for each of 148 SMs
+template <int VPT>
 __device__ __forceinline__ void prefetch_residual(const NormQuantParams &p) {
-    if (blockIdx.x >= kEarlyCtas || blockIdx.x >= p.rows) return;
+    if (blockIdx.x >= kEarlyCtas || blockIdx.x >= p.rows || (VPT == 8 && p.rows > 2 * kEarlyCtas)) return;
     const char *row = static_cast<const char *>(p.ep.residual) + static_cast<int64_t>(blockIdx.x) * p.ep.row_vecs * 16;
     for (int at = threadIdx.x * 128; at < p.ep.row_vecs * 16; at += blockDim.x * 128) asm volatile("prefetch.global.L2 [%0];" ::"l"(row + at));
 }
@@ -108,7 +111,7 @@ template <typename T, int VPT>
 __global__ void __launch_bounds__(tile_max_threads<VPT>(), tile_min_blocks<VPT>())
     fused_norm_quant_kernel(const __grid_constant__ NormQuantParams p) {
     __shared__ EpilogueSmem sm;
-    prefetch_residual(p);
+    prefetch_residual<VPT>(p);
     grid_dependency_sync();
     if (p.full) norm_quant_rows<T, VPT, true>(p, sm);
     else norm_quant_rows<T, VPT, false>(p, sm);
@@ -203,7 +206,7 @@ __global__ void __launch_bounds__(tile_max_threads<VPT>(), staged_min_blocks<VPT
     fused_norm_quant_staged_kernel(const __grid_constant__ NormQuantParams p) {
     extern __shared__ __align__(128) unsigned char stage_mem[];
     __shared__ StagedSmem sm;
-    prefetch_residual(p);
+    prefetch_residual<VPT>(p);
     grid_dependency_sync();
     if (p.full) norm_quant_staged_rows<T, VPT, true>(p, stage_mem, sm);
     else norm_quant_staged_rows<T, VPT, false>(p, stage_mem, sm);
