@@ -390,10 +390,10 @@ class GPUKDistEnv:
             cabi.check(cabi.lib.gpuk_ws_set_ready_words(ctypes.c_void_p(self.fptr), ctypes.c_void_p(words.data_ptr()),
                                                         int(rows_per_word), int(value)))
         if self._o is _TorchOps and not torch.compiler.is_compiling():
+            # FP8 asked for with the policy for none (-1 here) is an error of the operator
             qt = (QUANT_STATIC_E4M3FN_448 if static_scale is not None else
-                  QUANT_NONE if not fp8_out else fp8_policy_id if quant_type is None else quant_type)
-            # FP8 asked for with a policy that is none is an error of the operator
-            if (static_scale is None or isinstance(static_scale, torch.Tensor)) and not (fp8_out and qt == QUANT_NONE):
+                  QUANT_NONE if not fp8_out else fp8_policy_id if quant_type is None else quant_type or -1)
+            if static_scale is None or isinstance(static_scale, torch.Tensor):
                 results = _native.add_rms(self.fptr or 0, allreduce_in, residual_in, rms_weight, eps, qt,
                                           None if static_scale is None else static_scale.reshape(-1))
                 if results is not None:

@@ -35,6 +35,9 @@ import torch
 import torch.distributed as dist
 import torch.nn.functional as F
 
+import gpuk_b200 as gpuk
+from gpuk_b200 import _native
+
 
 @dataclass
 class DecoderArgs:
@@ -96,11 +99,8 @@ class _Linear:
     def __call__(self, x: torch.Tensor, x_scale: Optional[torch.Tensor] = None) -> torch.Tensor:
         # measured on B200: at up to 32 tokens the streaming kernels are the faster ones at the decoder's shapes (fp8_linear.cu, stream_linear.cu)
         own = self.own_gemm and x.is_cuda and 0 < x.shape[0] <= 32 and self.weight.dtype == torch.bfloat16
-        if own:
-            from gpuk_b200 import _native
         if self.fp8 and x.dtype == torch.float8_e4m3fn:
             if own and _native.no_modes() and (x.shape[0] <= 8 or self.w_q.is_contiguous()):
-                import gpuk_b200 as gpuk
                 if gpuk.fp8_linear_supported(x.shape[0], *self.w_q.shape):
                     if x.shape[0] > 8:
                         return gpuk.fp8_linear(x, x_scale, self.w_q, self.w_scale)
@@ -197,8 +197,7 @@ class TPDecoder:
             z = self._zeros.get(h.shape)
             if z is None:
                 z = self._zeros[h.shape] = torch.zeros_like(h)
-            import gpuk_b200 as gpuk
-            results = gpuk._native.add_rms(0, h, z, weight, self.args.norm_eps, 3 if self.fp8 else 0, None)
+            results = _native.add_rms(0, h, z, weight, self.args.norm_eps, 3 if self.fp8 else 0, None)
             if results is not None:
                 return results[1], results[2] if self.fp8 else None
             residual_out = torch.empty_like(h)
@@ -245,21 +244,21 @@ class TPDecoder:
         hd = a.head_dim
         h = F.embedding(tokens, self.tok_embeddings).view(b * t, a.dim)
         # positions in any other form that indexes a tensor go to the operators, as do caches, tables and weights that the kernels cannot read as they are
-        own = self.own_elementwise and isinstance(input_pos, torch.Tensor) and input_pos.shape == (t,) and input_pos.dtype in (torch.int64, torch.int32) and \
-            (not input_pos.is_cuda or input_pos.device == self.cos.device)
+        own = self.own_elementwise and isinstance(input_pos, torch.Tensor) and input_pos.shape == (t,)
+        if own:
+            pos = input_pos.to(device=self.device, dtype=torch.int64).contiguous()
+            own = pos is input_pos or (input_pos.dtype in (torch.int64, torch.int32) and (not input_pos.is_cuda or input_pos.device == self.cos.device))
         here = input_pos
         if own and input_pos.is_cuda:
             here = input_pos.cpu() if cache_len is None else None
         last = int(here[-1]) + 1 if cache_len is None else cache_len
         if own:
-            from gpuk_b200 import _native
             if last > a.max_seq_len and t == 1 and cache_len is not None:
                 last = a.max_seq_len      # as a slice of the cache takes it
             if last > a.max_seq_len:
                 raise RuntimeError(f"position {last - 1} is beyond the KV cache ({a.max_seq_len} positions)")
             if here is not None and here.numel() and not -a.max_seq_len <= int(here.min()) <= int(here.max()) < a.max_seq_len:
                 raise RuntimeError(f"a position in [{int(here.min())}, {int(here.max())}] is beyond the KV cache ({a.max_seq_len} positions)")
-            pos = input_pos.to(device=self.device, dtype=torch.int64).contiguous()
         tables = mask = None      # what the operators need, once one of them is called
         normed, scale = self._norm_only(h, self.layers[0]["attention_norm"])
         for li, layer in enumerate(self.layers):
