@@ -116,7 +116,7 @@ def fp8_linear(x_fp8: torch.Tensor, x_scale: torch.Tensor, w_fp8: torch.Tensor, 
     the reference has no FP8 path).  ``x_fp8`` [tokens, k] and ``w_fp8`` [n, k] are ``float8_e4m3fn``, ``x_scale``
     holds one fp32 scale per token (any shape with ``tokens`` elements), ``w_scale`` one per output channel;
     ``packed=True`` says ``w_fp8`` came from ``fp8_pack_weight``.
-    Hand-written weight-streaming kernel (``csrc/fp8_linear.cu``); raises for shapes it is not built for --
+    Hand-written weight-streaming kernels (``csrc/fp8_linear.cu`` and ``csrc/stream_linear.cu``); raises for shapes they are not built for --
     ``fp8_linear_supported`` tells, and larger batches belong to a library GEMM."""
     return _native.fp8_linear(x_fp8, x_scale, w_fp8, w_scale, out, packed, k_split)
 

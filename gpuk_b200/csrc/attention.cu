@@ -18,8 +18,9 @@
 //
 // fp32 scores, running maximum and sums; probabilities are rounded to bf16 for the second product.
 //
-// Measured, 64 / 8 heads, the library's attention in brackets: 32 sequences x 2049 keys 42.8 us (51.0), 6.3 TB/s; 32 x 300 8.7 (11.0); 8 x 2049 of
-// 32 / 8 heads 13.9 (14.5); 4 x 129 of 16 / 4 heads 3.4 (5.4); 7 x 1000 9.4 (8.6).  Error against float64 1.65e-3 to 1.79e-3 (1.73e-3 to 1.89e-3).
+// Measured, 64 / 8 heads, the library's attention in brackets: 32 sequences x 2049 keys 42.5 us (49.7), 6.3 TB/s; 32 x 300 8.5 (10.7); 7 x 2049 of
+// 32 / 8 heads 12.7 (13.4); 4 x 129 of 16 / 4 heads 3.2 (5.3).  Behind it: 7 x 1000 9.2 (8.6), 12 x 1000 12.2 (11.0), 1 x 8192 14.0 (12.0), 1 x 8192 of 8 / 1 heads 12.2 (8.6); its
+// call takes 25 us more on the host.  Error against float64 1.65e-3 to 1.79e-3 (1.73e-3 to 1.89e-3).
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 

@@ -391,10 +391,13 @@ __device__ __forceinline__ float block_max(float v, float *sm, const Group &g) {
 }
 
 // ---------------------------------------------------------------------------------------
-// programmatic dependent launch: the first statement of every kernel that is launched with
-// the programmatic-serialization attribute.  Waits until the preceding grid of the stream has
-// completed and its writes are visible (a no-op in an ordinary launch), then lets the grid
-// that follows begin to place its CTAs, which will wait here in their turn.
+// programmatic dependent launch: every thread of a kernel that is launched with the
+// programmatic-serialization attribute comes through here before it reads or writes global memory.
+// In front of it stand only what the CTA keeps to itself (barriers, tensor memory) and prefetches
+// into L2, which are hints.  Waits until the preceding grid of the stream has completed and its writes
+// are visible (a no-op in an ordinary launch), then lets the grid that follows begin to place
+// its CTAs, which will wait here in their turn.  Tensor memory is allocated in front: a CTA of the grid
+// that follows must not take columns for which one of this grid still waits.
 // ---------------------------------------------------------------------------------------
 __device__ __forceinline__ void grid_dependency_sync() {
     asm volatile("griddepcontrol.wait;" ::: "memory");

@@ -5,11 +5,11 @@
 // native path on sm_100 (its conversions and HMMAs bound the kernel at 3 TB/s with 32 tokens), so the weights go straight
 // from shared memory into tcgen05.mma, which one thread issues:
 //
-//   * a tile is 128 output channels = the 128 rows of one tcgen05.mma; the tokens are its 16 or 32 columns.  The accumulator
-//     takes 32 columns of tensor memory.
+//   * a tile is 128 output channels = the 128 rows of one tcgen05.mma; the tokens are its 16 or 32 columns.  The accumulators
+//     (below) take four times as many columns of tensor memory.
 //   * a pipeline step is 128 bytes of k: 16 KiB of weights and 2 or 4 KiB of activations, fetched by one TMA copy each into a ring.
-//     Two CTAs per SM keep up to 2 * kStages * 16 KiB of weights in flight per SM, about four times what latency times
-//     bandwidth asks for, so that one CTA's start and end hide behind the other's stream.
+//     Two or three CTAs per SM with rings of four to six steps keep 160 to 192 KiB of weights in flight per SM, several times what latency
+//     times bandwidth asks for, so that one CTA's start and end hide behind the other's stream.
 //   * where there are fewer tiles than CTAs fit, k is split over a thread-block cluster whose CTAs sum their partial tiles through
 //     distributed shared memory in CTA order (deterministic, no atomics, no workspace).
 //   * the weights the ring takes first are brought into L2 before griddepcontrol.wait, while the kernel in front still runs (32 tokens,
@@ -27,8 +27,10 @@
 // us; of two small layers, 4 sequences, 121 -> 112 us.
 //
 // Measured, 32 tokens, FP8: 57344 x 8192 75 us (6.3 TB/s; the warp-level kernel 136, the library GEMM 89), 10240 x 8192 16.6 (39, 20.7), 7168 x 8192 13.2
-// (21.7, 17.3), 4096 x 8192 10.1 (13.5, 15.8).  bf16: 8192 x 8192 23.8 us (library 25.3), 8192 x 28672 71.8 (71.2); 4 tokens: 3072 x 2048
-// 5.9 (7.5), 2048 x 4096 7.0 (12.4), 8192 x 2048 9.0 (8.0).  Below 30 MB what is left is a fixed 3 us of start and end.
+// (21.7, 17.3), 4096 x 8192 10.1 (13.5, 15.8).  bf16, the library in brackets: 32 tokens, 8192 x 8192 22.7 us (24.8), 8192 x 28672 71.8 (71.2), 22528 x 4096 33.7
+// (32.4), 1024 x 8192 9.3 (15.2), 3072 x 2048 7.1 (5.9); 4 tokens, 2048 x 4096 7.3 (12.9), 3072 x 2048 6.0 (7.5), 8192 x 2048 9.0 (8.2), 8192 x 3584 12.1 (11.4).  Below 30 MB
+// what is left is a fixed 3 us of start and end; there the library is ahead by up to a microsecond and a half for 8192 channels, and for 17 tokens and more.  A
+// call of it takes 4 us more on the host, and an epilogue here saves a launch.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
