@@ -3,7 +3,7 @@
 // current stream of the tensors' device, with the interpreter lock released as a dispatcher operator or ctypes would.  Why
 // neither of those: a call through them costs several microseconds of host time, which is what bounds a step of a few sequences
 // (fused epilogue, 8 rows: 11.0 -> 6.6 us a call; FP8 linear layer, 8 tokens, 1280 x 8192: 14.8 -> 5.7 us).  All but fp8_linear return None for a
-// call that belongs to the operators: see direct() and add_rms.
+// call that belongs to the operators: see NotDirect and add_rms.
 #include <ATen/cuda/CUDAContext.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <ATen/PythonTorchFunctionTLS.h>
@@ -28,13 +28,6 @@ void check(int status, const char *what) {
 const Tensor &tensor_arg(PyObject *o, const char *what) {
     TORCH_CHECK(THPVariable_Check(o), "gpuk: ", what, " must be a tensor");
     return THPVariable_Unpack(o);
-}
-// A contiguous CUDA tensor of the given type on the given device (-1: any).
-const Tensor &cuda_arg(PyObject *o, const char *what, at::ScalarType type, int device = -1) {
-    const Tensor &t = tensor_arg(o, what);
-    TORCH_CHECK(t.is_cuda() && t.is_contiguous() && t.scalar_type() == type, "gpuk: ", what, " must be a contiguous CUDA tensor of ", type);
-    TORCH_CHECK(device < 0 || t.get_device() == device, "gpuk: ", what, " is on another device");
-    return t;
 }
 int64_t int_arg(PyObject *o) {
     const int64_t v = PyLong_AsLongLong(o);
@@ -75,39 +68,55 @@ bool no_modes() {
                                             c10::DispatchKey::Tracer, c10::DispatchKey::Python, c10::DispatchKey::PreDispatch});
     return !tls.included_.has_any(front) && !c10::impl::TorchDispatchModeTLS::any_modes_set() && at::impl::PythonTorchFunctionTLS::stack_len() == 0;
 }
-// Whether the decode calls below read this tensor as it is.  Where one of theirs does not, or a mode wants to see operators, they return None and the caller takes
-// the operators, which accept any strides and types that go together.  What is no CUDA tensor is an error of the call.
-bool direct(PyObject *o, at::ScalarType type, uintptr_t align = 16) {
-    if (!THPVariable_Check(o) || !THPVariable_Unpack(o).is_cuda()) return true;
-    if (!plain(o, -1)) return false;
+// Thrown for a tensor that a decode call below does not read as it is: it returns None, and the caller takes the operators, which accept any strides and types that go
+// together.
+struct NotDirect {};
+// A plain contiguous CUDA tensor of the given type and alignment on the given device (-1: any).
+bool direct(PyObject *o, at::ScalarType type, int device, uintptr_t align) {
+    if (!plain(o, device)) return false;
     const Tensor &t = THPVariable_Unpack(o);
     return t.scalar_type() == type && reinterpret_cast<uintptr_t>(t.const_data_ptr()) % align == 0;
 }
-
-// The same of a KV cache.  The library's attention reads it in vectors of 16 bytes and faults on one whose rows are not aligned for them: such a cache is refused.
-bool direct_cache(PyObject *o) {
-    if (direct(o, at::kBFloat16)) return true;
-    const Tensor &t = THPVariable_Unpack(o);
-    if (plain_class(o) && t.layout() == at::kStrided && t.dim() == 4 && t.stride(3) == 1) {
-        bool aligned = reinterpret_cast<uintptr_t>(t.const_data_ptr()) % 16 == 0;
-        for (int i = 0; i < 3; ++i) aligned = aligned && t.stride(i) * t.element_size() % 16 == 0;
-        TORCH_CHECK(aligned, "gpuk: rows of a KV cache must be 16-byte aligned");
-    }
-    return false;
+// What is no CUDA tensor, or on another device, is an error.
+const Tensor &cuda_arg(PyObject *o, const char *what, at::ScalarType type, int device = -1, uintptr_t align = 16) {
+    if (direct(o, type, device, align)) return THPVariable_Unpack(o);
+    const Tensor &t = tensor_arg(o, what);
+    TORCH_CHECK(t.is_cuda(), "gpuk: ", what, " must be a contiguous CUDA tensor of ", type);
+    TORCH_CHECK(device < 0 || t.get_device() == device, "gpuk: ", what, " is on another device");
+    throw NotDirect();
 }
+// The same of a KV cache.  The library's attention reads it in vectors of 16 bytes and faults on one whose rows are not aligned for them: such a cache is refused.
+const Tensor &cache_arg(PyObject *o, const char *what, int device) {
+    if (direct(o, at::kBFloat16, device, 16)) return THPVariable_Unpack(o);
+    if (plain_class(o)) {
+        const Tensor &t = THPVariable_Unpack(o);
+        if (t.is_cuda() && t.layout() == at::kStrided && t.dim() == 4 && t.stride(3) == 1) {
+            bool aligned = reinterpret_cast<uintptr_t>(t.const_data_ptr()) % 16 == 0;
+            for (int i = 0; i < 3; ++i) aligned = aligned && t.stride(i) * t.element_size() % 16 == 0;
+            TORCH_CHECK(aligned, "gpuk: rows of a KV cache must be 16-byte aligned");
+        }
+    }
+    return cuda_arg(o, what, at::kBFloat16, device);
+}
+// Around such a call: None while a mode wants to see operators, and for tensors that are not direct.
+#define DIRECT_CALL(name, count)     \
+    HANDLE_TH_ERRORS                 \
+    expect_args(n, count, name);     \
+    if (!no_modes()) Py_RETURN_NONE; \
+    try {
+#define END_DIRECT_CALL                                  \
+    }                                                    \
+    catch (const NotDirect &) { Py_RETURN_NONE; }        \
+    END_HANDLE_TH_ERRORS
 
 // rope_append(qkv [rows, (heads + 2 kv_heads) * head_dim], cos, sin, pos [t], k_cache, v_cache, heads) -> q [rows, heads * head_dim]
 PyObject *rope_append(PyObject *, PyObject *const *args, Py_ssize_t n) {
-    HANDLE_TH_ERRORS
-    expect_args(n, 7, "rope_append");
-    if (!no_modes() || !direct(args[0], at::kBFloat16) || !direct(args[1], at::kFloat) || !direct(args[2], at::kFloat) || !direct(args[3], at::kLong, 8) ||
-        !direct_cache(args[4]) || !direct_cache(args[5]))
-        Py_RETURN_NONE;
+    DIRECT_CALL("rope_append", 7)
     const Tensor &qkv = cuda_arg(args[0], "qkv", at::kBFloat16);
     const int dev = qkv.get_device();
     const Tensor &cos = cuda_arg(args[1], "cos", at::kFloat, dev), &sin = cuda_arg(args[2], "sin", at::kFloat, dev);
-    const Tensor &pos = cuda_arg(args[3], "positions", at::kLong, dev);
-    const Tensor &kc = cuda_arg(args[4], "k_cache", at::kBFloat16, dev), &vc = cuda_arg(args[5], "v_cache", at::kBFloat16, dev);
+    const Tensor &pos = cuda_arg(args[3], "positions", at::kLong, dev, 8);
+    const Tensor &kc = cache_arg(args[4], "k_cache", dev), &vc = cache_arg(args[5], "v_cache", dev);
     const int64_t heads = int_arg(args[6]);
     TORCH_CHECK(kc.dim() == 4 && vc.sizes() == kc.sizes() && qkv.dim() == 2 && cos.dim() == 2 && sin.sizes() == cos.sizes(), "gpuk: rope_append shapes do not match");
     const int64_t kv = kc.size(1), max_seq = kc.size(2), hd = kc.size(3), t = pos.numel(), rows = qkv.size(0);
@@ -123,14 +132,12 @@ PyObject *rope_append(PyObject *, PyObject *const *args, Py_ssize_t n) {
                                int_size(cos.size(0)), int_size(max_seq), stream_of(qkv)), "rope_append");
     }
     return THPVariable_Wrap(std::move(q));
-    END_HANDLE_TH_ERRORS
+    END_DIRECT_CALL
 }
 
 // silu_mul(x [rows, 2 f]) -> [rows, f]
 PyObject *silu_mul(PyObject *, PyObject *const *args, Py_ssize_t n) {
-    HANDLE_TH_ERRORS
-    expect_args(n, 1, "silu_mul");
-    if (!no_modes() || !direct(args[0], at::kBFloat16)) Py_RETURN_NONE;
+    DIRECT_CALL("silu_mul", 1)
     const Tensor &x = cuda_arg(args[0], "x", at::kBFloat16);
     TORCH_CHECK(x.dim() == 2 && x.size(1) % 2 == 0, "gpuk: silu_mul takes [rows, 2 f]");
     Tensor out;
@@ -141,14 +148,12 @@ PyObject *silu_mul(PyObject *, PyObject *const *args, Py_ssize_t n) {
         check(gpuk_silu_mul(x.data_ptr(), out.data_ptr(), x.size(0), int_size(x.size(1) / 2), stream_of(x)), "silu_mul");
     }
     return THPVariable_Wrap(std::move(out));
-    END_HANDLE_TH_ERRORS
+    END_DIRECT_CALL
 }
 
 // linear(x [m, k], w [n, k]) -> [m, n], bf16, m <= 32
 PyObject *linear(PyObject *, PyObject *const *args, Py_ssize_t n) {
-    HANDLE_TH_ERRORS
-    expect_args(n, 2, "linear");
-    if (!no_modes() || !direct(args[0], at::kBFloat16) || !direct(args[1], at::kBFloat16)) Py_RETURN_NONE;
+    DIRECT_CALL("linear", 2)
     const Tensor &x = cuda_arg(args[0], "x", at::kBFloat16);
     const Tensor &w = cuda_arg(args[1], "w", at::kBFloat16, x.get_device());
     TORCH_CHECK(x.dim() == 2 && w.dim() == 2 && x.size(1) == w.size(1), "gpuk: linear operand shapes do not match");
@@ -161,7 +166,7 @@ PyObject *linear(PyObject *, PyObject *const *args, Py_ssize_t n) {
                                  stream_of(x)), "linear");
     }
     return THPVariable_Wrap(std::move(out));
-    END_HANDLE_TH_ERRORS
+    END_DIRECT_CALL
 }
 
 // x [m, k] and w [n, k] in FP8 with their scales, or in bf16 with None for both: checked, and as the C ABI takes them.
@@ -169,15 +174,11 @@ struct Operands {
     const Tensor &x, &w;
     const float *x_scale = nullptr, *w_scale = nullptr;
     int m, n, k;
-    static bool are_direct(PyObject *const *args) {
-        const at::ScalarType type = args[1] == Py_None ? at::kBFloat16 : at::kFloat8_e4m3fn;
-        return direct(args[0], type) && direct(args[2], type) && direct(args[1], at::kFloat, 4) && direct(args[3], at::kFloat);
-    }
     Operands(PyObject *const *args) : x(cuda_arg(args[0], "x", args[1] == Py_None ? at::kBFloat16 : at::kFloat8_e4m3fn)), w(cuda_arg(args[2], "w", x.scalar_type(), x.get_device())) {
         TORCH_CHECK(x.dim() == 2 && w.dim() == 2 && x.size(1) == w.size(1) && (args[1] == Py_None) == (args[3] == Py_None), "gpuk: linear operand shapes do not match");
         m = int_size(x.size(0)), n = int_size(w.size(0)), k = int_size(w.size(1));
         if (args[1] == Py_None) return;
-        const Tensor &xs = cuda_arg(args[1], "x_scale", at::kFloat, x.get_device()), &ws = cuda_arg(args[3], "w_scale", at::kFloat, x.get_device());
+        const Tensor &xs = cuda_arg(args[1], "x_scale", at::kFloat, x.get_device(), 4), &ws = cuda_arg(args[3], "w_scale", at::kFloat, x.get_device());
         TORCH_CHECK(xs.numel() == m && ws.numel() == n, "gpuk: linear takes a scale per token and per channel");
         x_scale = xs.data_ptr<float>(), w_scale = ws.data_ptr<float>();
     }
@@ -185,9 +186,7 @@ struct Operands {
 
 // swiglu(x, x_scale, w [2 f, k], w_scale) -> [m, f]: silu of the first f channels times the others
 PyObject *swiglu(PyObject *, PyObject *const *args, Py_ssize_t n) {
-    HANDLE_TH_ERRORS
-    expect_args(n, 4, "swiglu");
-    if (!no_modes() || !Operands::are_direct(args)) Py_RETURN_NONE;
+    DIRECT_CALL("swiglu", 4)
     const Operands o(args);
     Tensor out;
     {
@@ -197,20 +196,16 @@ PyObject *swiglu(PyObject *, PyObject *const *args, Py_ssize_t n) {
         check(gpuk_swiglu_skinny(o.x.data_ptr(), o.x_scale, o.w.data_ptr(), o.w_scale, out.data_ptr(), o.m, o.n, o.k, 0, stream_of(o.x)), "swiglu");
     }
     return THPVariable_Wrap(std::move(out));
-    END_HANDLE_TH_ERRORS
+    END_DIRECT_CALL
 }
 
 // qkv_rope(x, x_scale, w, w_scale, cos, sin, pos [t], k_cache, v_cache, heads) -> q [m, heads * 128]; keys and values go to the caches
 PyObject *qkv_rope(PyObject *, PyObject *const *args, Py_ssize_t n) {
-    HANDLE_TH_ERRORS
-    expect_args(n, 10, "qkv_rope");
-    if (!no_modes() || !Operands::are_direct(args) || !direct(args[4], at::kFloat) || !direct(args[5], at::kFloat) || !direct(args[6], at::kLong, 8) ||
-        !direct_cache(args[7]) || !direct_cache(args[8]))
-        Py_RETURN_NONE;
+    DIRECT_CALL("qkv_rope", 10)
     const Operands o(args);
     const int dev = o.x.get_device();
-    const Tensor &cos = cuda_arg(args[4], "cos", at::kFloat, dev), &sin = cuda_arg(args[5], "sin", at::kFloat, dev), &pos = cuda_arg(args[6], "positions", at::kLong, dev);
-    const Tensor &kc = cuda_arg(args[7], "k_cache", at::kBFloat16, dev), &vc = cuda_arg(args[8], "v_cache", at::kBFloat16, dev);
+    const Tensor &cos = cuda_arg(args[4], "cos", at::kFloat, dev), &sin = cuda_arg(args[5], "sin", at::kFloat, dev), &pos = cuda_arg(args[6], "positions", at::kLong, dev, 8);
+    const Tensor &kc = cache_arg(args[7], "k_cache", dev), &vc = cache_arg(args[8], "v_cache", dev);
     const int64_t heads = int_arg(args[9]), t = pos.numel();
     TORCH_CHECK(kc.dim() == 4 && vc.sizes() == kc.sizes() && cos.dim() == 2 && sin.sizes() == cos.sizes() && kc.size(3) == 128 && cos.size(1) == 64 && heads > 0 &&
                     o.n == (heads + 2 * kc.size(1)) * 128 && t > 0 && o.m % t == 0 && o.m / t <= kc.size(0), "gpuk: qkv_rope shapes do not match");
@@ -224,17 +219,15 @@ PyObject *qkv_rope(PyObject *, PyObject *const *args, Py_ssize_t n) {
                                    int_size(cos.size(0)), int_size(kc.size(2)), 0, stream_of(o.x)), "qkv_rope");
     }
     return THPVariable_Wrap(std::move(q));
-    END_HANDLE_TH_ERRORS
+    END_DIRECT_CALL
 }
 
 // decode_attention(q [batch, heads, 128], k_cache, v_cache [>= batch, kv_heads, max_seq, 128], len) -> [batch, heads * 128]
 PyObject *decode_attention(PyObject *, PyObject *const *args, Py_ssize_t n) {
-    HANDLE_TH_ERRORS
-    expect_args(n, 4, "decode_attention");
-    if (!no_modes() || !direct(args[0], at::kBFloat16) || !direct_cache(args[1]) || !direct_cache(args[2])) Py_RETURN_NONE;
+    DIRECT_CALL("decode_attention", 4)
     const Tensor &q = cuda_arg(args[0], "q", at::kBFloat16);
     const int dev = q.get_device();
-    const Tensor &kc = cuda_arg(args[1], "k_cache", at::kBFloat16, dev), &vc = cuda_arg(args[2], "v_cache", at::kBFloat16, dev);
+    const Tensor &kc = cache_arg(args[1], "k_cache", dev), &vc = cache_arg(args[2], "v_cache", dev);
     const int64_t len = int_arg(args[3]);
     TORCH_CHECK(q.dim() == 3 && kc.dim() == 4 && vc.sizes() == kc.sizes() && q.size(0) <= kc.size(0) && q.size(2) == kc.size(3) && len <= kc.size(2),
                 "gpuk: decode_attention shapes do not match");
@@ -248,19 +241,16 @@ PyObject *decode_attention(PyObject *, PyObject *const *args, Py_ssize_t n) {
               "decode_attention");
     }
     return THPVariable_Wrap(std::move(out));
-    END_HANDLE_TH_ERRORS
+    END_DIRECT_CALL
 }
 
 // prefill_attention(q [batch, t, heads, 128], k_cache, v_cache, pos [t], len) -> [batch * t, heads * 128]
 PyObject *prefill_attention(PyObject *, PyObject *const *args, Py_ssize_t n) {
-    HANDLE_TH_ERRORS
-    expect_args(n, 5, "prefill_attention");
-    if (!no_modes() || !direct(args[0], at::kBFloat16) || !direct_cache(args[1]) || !direct_cache(args[2]) || !direct(args[3], at::kLong, 8))
-        Py_RETURN_NONE;
+    DIRECT_CALL("prefill_attention", 5)
     const Tensor &q = cuda_arg(args[0], "q", at::kBFloat16);
     const int dev = q.get_device();
-    const Tensor &kc = cuda_arg(args[1], "k_cache", at::kBFloat16, dev), &vc = cuda_arg(args[2], "v_cache", at::kBFloat16, dev);
-    const Tensor &pos = cuda_arg(args[3], "positions", at::kLong, dev);
+    const Tensor &kc = cache_arg(args[1], "k_cache", dev), &vc = cache_arg(args[2], "v_cache", dev);
+    const Tensor &pos = cuda_arg(args[3], "positions", at::kLong, dev, 8);
     const int64_t len = int_arg(args[4]);
     TORCH_CHECK(q.dim() == 4 && kc.dim() == 4 && vc.sizes() == kc.sizes() && q.size(0) <= kc.size(0) && q.size(3) == kc.size(3) && pos.numel() == q.size(1) && len <= kc.size(2),
                 "gpuk: prefill_attention shapes do not match");
@@ -274,7 +264,7 @@ PyObject *prefill_attention(PyObject *, PyObject *const *args, Py_ssize_t n) {
                                      int_size(len), int_size(kc.size(2)), stream_of(q)), "prefill_attention");
     }
     return THPVariable_Wrap(std::move(out));
-    END_HANDLE_TH_ERRORS
+    END_DIRECT_CALL
 }
 
 // fp8_linear(x [m, k], x_scale, w [n, k], w_scale, out or None, packed, k_split) -> [m, n]

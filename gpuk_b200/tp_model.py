@@ -287,7 +287,7 @@ class TPDecoder:
                     # Up to 16 pairs of sequence and kv head, the eight parts that a pair's keys are cut into leave SMs idle, and the library's attention, which cuts further, is
                     # ahead on the device for long contexts (one pair: 4096 keys 8.1 / 7.3 us, 16384 20.3 / 9.5, 32768 35.9 / 11.5; eight: 32768 37.8 / 25.5).  Its call costs
                     # 25 us more on the host, so it is taken where that is made good.
-                    att = _native.decode_attention(q.reshape(b, self.h_local, hd), layer["k_cache"], layer["v_cache"], last)
+                    att = _native.decode_attention(q.view(b, self.h_local, hd), layer["k_cache"], layer["v_cache"], last)
             if att is None:
                 if t > 1 and mask is None:
                     mask = (torch.arange(last, device=self.device)[None, :] <= input_pos[:, None])[None, None]
