@@ -962,12 +962,13 @@ int gpuk_ws_selftest_wait(gpuk_ws *ws, void *stream) {
     return GPUK_OK;
 }
 
-// Which of the one-GPU kernels takes a call.  Measured in us, calls back to back, bf16 with dynamic scales:
+// Which of the one-GPU kernels takes a call.  Measured in us, calls back to back, bf16 with dynamic scales (the lines hold for fp16; in fp32 a CTA per row is the faster one for
+// 768 vectors too: 7200 x 3072 50.7 persistent, 46.0):
 //   a warp per row: rows of at most 256 vectors, 2 MiB of input and more.  16384 x 2048 37.3 (persistent CTAs 47.7, a CTA per row 52.9), 1500 x 1024 3.4
 //     (4.1, 4.1); 600 x 1024, 1.2 MiB, 2.7 (2.4 with a CTA per row).
 //   persistent CTAs, 2 stages of 512 threads: rows of at least 640 vectors, 32 rows per SM and more: 16384 x 6144 108 (a CTA per row 116), 6000 x 8192 56.1 (57.3);
-//     fewer rows 3500 x 6144 25.8 (23.1), shorter ones 6000 x 4096 38.2 (30.6).  At 1024 vectors a CTA per row comes ahead again from 48
-//     rows per SM: 16384 x 8192 151 (160).
+//     fewer rows 3500 x 6144 25.8 (23.1), shorter ones 6000 x 4096 38.2 (30.6).  Towards 1024 vectors a CTA per row is taken from 48 rows per SM on: it is steady (12000 x
+//     8192 111, 16384 x 8192 150), where the persistent kernel varies from run to run (107 to 114, 145 to 160); in fp32 it is ahead (16384 x 4096 138, 148).
 //   ... 4 stages of 256 threads: rows of up to 640 vectors from 64 rows per SM: 16384 x 3072 61 (a CTA per row 66.6), 16384 x 5120 94 (106).
 //   a CTA per row otherwise.
 struct K1Choice {

@@ -258,8 +258,10 @@ class TPDecoder:
                 last = a.max_seq_len      # as a slice of the cache takes it
             if last > a.max_seq_len:
                 raise RuntimeError(f"position {last - 1} is beyond the KV cache ({a.max_seq_len} positions)")
-            if here is not None and here.numel() and not -a.max_seq_len <= int(here.min()) <= int(here.max()) < a.max_seq_len:
-                raise RuntimeError(f"a position in [{int(here.min())}, {int(here.max())}] is beyond the KV cache ({a.max_seq_len} positions)")
+            if here is not None and t:
+                lo, hi = map(int, here.aminmax())
+                if lo < -a.max_seq_len or hi >= a.max_seq_len:
+                    raise RuntimeError(f"a position in [{lo}, {hi}] is beyond the KV cache ({a.max_seq_len} positions)")
         tables = mask = None      # what the operators need, once one of them is called
         normed, scale = self._norm_only(h, self.layers[0]["attention_norm"])
         for li, layer in enumerate(self.layers):
