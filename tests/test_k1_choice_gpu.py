@@ -27,3 +27,38 @@ def test_persistent_ctas(tokens, vecs, quant):
     parts, res, w = util.random_case(1, tokens, vecs * 8, torch.bfloat16, seed=tokens + vecs + quant)
     got = util.k1(parts[0].cuda(), res.cuda(), w.cuda(), 1e-6, quant)
     util.check_against_oracle(got, eo.add_rms_quant(parts[0], res, w, 1e-6, quant), quant, exact_residual=True)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("quant", [0, 3])
+@pytest.mark.parametrize("tokens,vecs", [(1100, 120), (520, 256), (9475, 300), (4740, 768)])
+def test_rows_that_are_not_finite(tokens, vecs, quant, dtype):
+    """NaN, infinities, sums of squares that overflow and rows of zeros: a warp per row and persistent CTAs give what a CTA per row gives, and the rows beside them are
+    as without."""
+    from gpuk_b200 import cabi
+    hidden = vecs * (16 // dtype.itemsize)
+    parts, res, w = util.random_case(1, tokens, hidden, dtype, seed=tokens + vecs)
+    x, big = parts[0], torch.finfo(dtype).max
+    x[0], res[0] = 0, 0
+    x[1, 3], x[2, 5], x[3, 7], x[tokens - 1, hidden - 1] = float("nan"), float("inf"), float("-inf"), float("nan")
+    x[4], res[4] = big, 0
+    x[5], res[5] = float("inf"), float("-inf")
+    got = util.k1(x.cuda(), res.cuda(), w.cuda(), 1e-6, quant)
+    cabi.check(cabi.lib.gpuk_set_tuning(b"k1_staged_min_rows", 1 << 40))
+    try:
+        want = util.k1(x.cuda(), res.cuda(), w.cuda(), 1e-6, quant)
+    finally:
+        cabi.check(cabi.lib.gpuk_set_tuning(b"k1_staged_min_rows", -1))
+    special = [0, 1, 2, 3, 4, 5, tokens - 1]
+    rest = torch.ones(tokens, dtype=torch.bool)
+    rest[special] = False
+    for name, a, b in zip(("residual", "norm", "scale"), got[:2 if quant == 0 else 3], want):
+        a, b = a.float(), b.float()
+        assert torch.equal(a[special].isnan(), b[special].isnan()), name
+        # the root of a sum in another order: a few units of fp32 in it, and so in what is not rounded further; a step of FP8 (1/8); in 16 bits two roundings, of the normalised
+        # value and of its product with the weight, each of which can fall the other way by a step (bf16: 1/128)
+        step = 0.0 if name == "residual" else 2.0 ** -20 if name == "scale" or dtype == torch.float32 and quant == 0 else 2.0 ** -3 if quant else 2.0 ** -6
+        for rows in (special, rest):
+            c, d = a[rows].nan_to_num(7.0), b[rows].nan_to_num(7.0)
+            assert bool(((c - d).abs() <= d.abs() * step).all()), name
+        assert bool(a[rest].isfinite().all())
