@@ -207,15 +207,19 @@ __global__ void __launch_bounds__(kThreads, 2) stream_linear_kernel(const __grid
     for (int j = 0; j < N; ++j) asm volatile("st.shared.f32 [%0], %1;" ::"r"(partial + (j * kPitch + channel) * 4), "f"(r[j]) : "memory");
     tc_fence_before();
     if (ks > 1) cluster_arrive();
-    __syncthreads();
     // Before the wait for the cluster: a CTA that waits for its peers holds no tensor memory, for which a peer may still be waiting on another SM, behind
     // CTAs that in their turn wait for theirs.  Allocation has no time limit, and neither shared memory nor registers keep short parts of k at four CTAs an SM.
+    // Only the warp that frees waits for the others' reads of it.
     if (warp == 1) {
+        asm volatile("barrier.cta.sync 1, %0;" ::"n"(kThreads) : "memory");
         tc_fence_after();
         tmem_free<kTmemCols>(acc);
         __syncwarp();
+    } else {
+        asm volatile("barrier.cta.arrive 1, %0;" ::"n"(kThreads) : "memory");
     }
     if (ks > 1) cluster_wait();
+    else __syncthreads();
     // the tile's outputs, four channels at a time, dealt out over the cluster; the sum over the cluster in CTA order
     auto sum = [&](int tok, int ch, int n) {      // channels ch.. of the tile, n.. of the weights
         const uint32_t at = partial + (tok * kPitch + ch) * 4;
